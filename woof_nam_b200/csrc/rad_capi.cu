@@ -31,6 +31,12 @@
 namespace rad {
 __constant__ int c_lw_ns[17] = {0, 10, 22, 38, 52, 68, 76, 88, 96, 108, 114, 122, 130, 134, 136, 138, 140};
 __constant__ int c_sw_ns[15] = {0, 6, 18, 26, 34, 44, 54, 56, 66, 74, 80, 86, 94, 100, 112};
+// band of each SW g-point
+__constant__ unsigned char c_sw_band[112] = {
+    0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2, 2, 2, 3, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4,
+    4, 4, 4, 4, 4, 4, 5, 5, 5, 5, 5, 5, 5, 5, 5, 5, 6, 6, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 8, 8, 8, 8, 8, 8, 8, 8, 9, 9,
+    9, 9, 9, 9, 10, 10, 10, 10, 10, 10, 11, 11, 11, 11, 11, 11, 11, 11, 12, 12, 12, 12, 12, 12, 13, 13, 13, 13, 13,
+    13, 13, 13, 13, 13, 13, 13};
 }  // namespace rad
 
 #include "rad_lw.cuh"
@@ -73,6 +79,7 @@ struct RadHandle {
     int64_t lwpg_cap = 0, swpg_cap = 0;            // columns they hold
     int4* d_sw4img = nullptr;                      // chunked SW: set-up and gas-optics images of one chunk's columns
     unsigned char* d_sw4 = nullptr;                // chunked SW: header and layer R/T of one chunk's columns
+    int* d_sw4item = nullptr;                      // chunked SW: work items of the float64 fix-up
     int64_t sw4_cap = 0;                           // columns d_sw4 and d_sw4img hold
     float* d_aerf = nullptr;                       // aerosol band tables of the loaded month (AF_* offsets)
     int* d_aeri = nullptr;                         // their integer part (AI_* offsets)
@@ -367,12 +374,15 @@ int ensure_launch_scratch(RadHandle* h, int64_t ntot, int64_t ncmin)
     if (swc > 0 && (h->cfg.parts & RAD_PART_SW) && std::min(swc, ntot) > h->sw4_cap) {
         if (h->d_sw4) cudaFree(h->d_sw4);
         if (h->d_sw4img) cudaFree(h->d_sw4img);
+        if (h->d_sw4item) cudaFree(h->d_sw4item);
         h->d_sw4 = nullptr;
         h->d_sw4img = nullptr;
+        h->d_sw4item = nullptr;
         h->sw4_cap = 0;
         const int64_t need = std::min(swc, ntot);
         RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4, (size_t)need * sw4_block_bytes(h->cfg.nlay)));
         RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4img, (size_t)need * sw4_image_bytes(true)));
+        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4item, (size_t)sw4_item_bytes(h->cfg.nlay, need)));
         h->sw4_cap = need;
     }
     if (h->cfg.route == RAD_ROUTE_MCICA && ntot * h->cfg.nlay > h->mask_cap) {
@@ -614,18 +624,22 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 // into the chunk scratch, then the adding sweeps one CTA per column
                 const int64_t swc = sw4_chunk(cfg);
                 const size_t smem0 = sw4_gas_smem(any_aer);
-                const size_t smem1 = sw4_gas_smem(any_aer);   // the image without taug (read from the image)
+                const size_t smem1 = sw4_rt_smem(any_aer);    // the image without taug (read from the image)
                 const size_t smem2 = (size_t)(SW2_NSEG - 1) * 4 * SW2_THREADS * sizeof(float);
                 const size_t bb = sw4_block_bytes(nlay);
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_gas_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0));
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_rt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_sweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_sweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
                 for (int64_t d0 = 0; d0 < ntot; d0 += swc) {
                     const int64_t nc = std::min(swc, ntot - d0);
-                    sw4_gas_kernel<<<(unsigned)nc, SW4_GAS_THREADS, smem0, st>>>(bt, any_aer ? 1 : 0, h->d_err, (int)d0, h->d_sw4img);
-                    sw4_rt_kernel<<<(unsigned)nc, SW4_RT_THREADS, smem1, st>>>(bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0,
-                                                                         h->d_sw4img, h->d_sw4, bb);
+                    sw4_gas_kernel<<<(unsigned)nc, SW4_GAS_THREADS, smem0, st>>>(bt, any_aer ? 1 : 0, h->d_err, (int)d0, h->d_sw4img,
+                                                                                 h->d_sw4item);
+                    sw4_rt_kernel<<<(unsigned)nc, SW4_RT_THREADS, smem1, st>>>(bt, any_aer ? 1 : 0, (int)d0, h->d_sw4img, h->d_sw4,
+                                                                               bb, h->d_sw4item);
+                    sw4_fix_kernel<<<(unsigned)(SW4_FIX_MINB * h->nsm), SW4_FIX_THREADS, smem1, st>>>(
+                        bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, h->d_sw4item);
                     if (diag_sw) {
                         sw4_sweep_kernel<true><<<(unsigned)nc, SW2_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
                                                                                         h->d_sw4, bb, h->d_swpg);
@@ -635,7 +649,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                                                                                          h->d_sw4, bb);
                     }
                 }
-                nlaunch = (diag_sw ? 4 : 3) * ((ntot + swc - 1) / swc);
+                nlaunch = (diag_sw ? 5 : 4) * ((ntot + swc - 1) / swc);
             } else {       // SW2_CTAS_PER_SM CTAs per SM walk the day list, each with its R/T store
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw2_column_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 sw2_column_kernel<true><<<(unsigned)(SW2_CTAS_PER_SM * h->nsm), SW2_THREADS, smem, st>>>(
@@ -828,7 +842,8 @@ int64_t rad_workspace_bytes(const RadHandle* h, int64_t ncol)
         const int64_t swc = sw4_chunk(h->cfg);
         if (h->cfg.precision == RAD_PREC_MIXED && (h->cfg.parts & RAD_PART_SW) && swc <= 0) b += sw2_rt_bytes(h->nsm);
         if (swc > 0 && (h->cfg.parts & RAD_PART_SW))
-            b += std::min(swc, ncol) * (int64_t)(sw4_block_bytes(h->cfg.nlay) + sw4_image_bytes(true));
+            b += std::min(swc, ncol) * (int64_t)(sw4_block_bytes(h->cfg.nlay) + sw4_image_bytes(true)) +
+                 sw4_item_bytes(h->cfg.nlay, std::min(swc, ncol));
     }
     return b;
 }
@@ -1505,7 +1520,7 @@ void rad_destroy(RadHandle* h)
     for (void* p : {(void*)h->d_lwf, (void*)h->d_swf, (void*)h->d_lwd, (void*)h->d_swd,
                     (void*)h->d_err, (void*)h->d_flag, (void*)h->d_pos, (void*)h->d_daycol, (void*)h->d_lt,
                     (void*)h->d_k8, (void*)h->d_kw, (void*)h->d_cmin, (void*)h->d_nday, h->d_cub, (void*)h->d_lwm,
-                    (void*)h->d_swm, (void*)h->d_lw3, (void*)h->d_lw3list, (void*)h->d_swrt, (void*)h->d_sw4, (void*)h->d_sw4img, (void*)h->d_lwpg, (void*)h->d_swpg, (void*)h->d_aerf,
+                    (void*)h->d_swm, (void*)h->d_lw3, (void*)h->d_lw3list, (void*)h->d_swrt, (void*)h->d_sw4, (void*)h->d_sw4img, (void*)h->d_sw4item, (void*)h->d_lwpg, (void*)h->d_swpg, (void*)h->d_aerf,
                     (void*)h->d_aeri})
         if (p) cudaFree(p);
     delete h;

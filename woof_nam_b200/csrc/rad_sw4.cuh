@@ -1,5 +1,5 @@
 // rad_sw4.cuh -- the chunked SW of rad_solve (mixed precision): set-up and gas optics, the layer reflectances
-// and transmittances, and the adding sweeps in three kernels per chunk of sunlit columns.
+// and transmittances, their float64 fix-ups, and the adding sweeps in four kernels per chunk of sunlit columns.
 //
 // Same statements as sw2_column (rad_sw2.cuh), split where the work changes shape, and each kernel small enough
 // that the CTAs resident on an SM run out of the instruction cache (one kernel with all three phases spent most
@@ -8,20 +8,26 @@
 //    (sw2_setup), gas and Rayleigh optical depths per (g-point, layer); writes the column image (the part of the
 //    shared-memory layout the later phases read, taug included).
 //  * sw4_rt_kernel, one CTA per column: loads the image, then the layer R/T of the clear pass and, in the
-//    layers with cloud, of the cloudy pass (spcvrtc.cu:112-173, 330-460), lanes on 32 consecutive
-//    (layer, g-point) tasks so that a warp shares the cloudy branch, two tasks per thread side by side, in
-//    float without branches.  A task whose R/T needs a float64 step (the resonance, or an exp-table argument
-//    near an entry bound whose neighbouring entry matters) is queued and formed afterwards by sw2_layer, the
-//    sweep kernels' own function, one per thread.  Output per column: a header (solar source per g-point,
-//    albedos, overlap fractions, heating factors, the cloudy-pass slot of each layer) and the R/T as
-//    [layer][field][g-point] (a warp of the sweep kernel reads 32 consecutive g-points of one field and
-//    layer: one 128-byte line).
+//    layers with cloud, of the cloudy pass (spcvrtc.cu:112-173, 330-460) in float without branches, a task a pair
+//    of neighbouring g-points in packed float2 arithmetic (rad_f32x2.cuh), lanes on 32 consecutive (layer, pair)
+//    tasks so that a warp shares the cloudy branch.  A g-point whose R/T needs a float64 step (the resonance, or an
+//    exp-table argument near an entry bound whose neighbouring entry matters) is queued.  Output per column: a
+//    header (solar source per g-point, albedos, overlap fractions, heating factors, the cloudy-pass slot of each
+//    layer), the R/T as [layer][field][g-point] (a warp of the sweep kernel reads 32 consecutive g-points of one
+//    field and layer: one 128-byte line) and the queue.
+//  * sw4_fix_kernel, over the tile's queues: sw2_layer (the sweep kernels' own function) for the queued g-points.
+//    Bound: issue slots.  Measured per 131,072 columns (65,536 sunlit, 61 layers): 12.76 ms as one kernel with one
+//    g-point per thread and the queue formed by the same CTA; 9.48 ms with pairs; 4.30 + 3.35 ms as two kernels --
+//    the queue's float64 code no longer sets the registers (128, 4 CTAs per SM; now 80, 6 CTAs) nor keeps a CTA's
+//    other warps waiting, and the columns at a resonance (thousands of entries; up to 2,000,000 cycles in one CTA
+//    when a fixed queue of 527 overflowed) spread over the grid.
 //  * sw4_sweep_kernel, one CTA per column: the adding method alone (swflux, spcvrtc.cu:178-215) -- the upward
 //    sweep with segment checkpoints, the downward sweep re-reading each segment's R/T, float64 level sums and
 //    the swrad epilogue.
 // The outputs agree with sw2_column's to float rounding (tests/test_gpu_sw_split.py).
 #pragma once
 #include <type_traits>
+#include "rad_f32x2.cuh"
 #include "rad_sw2.cuh"
 
 namespace rad {
@@ -29,11 +35,9 @@ namespace rad {
 constexpr int SW4_FIELDS = 6;                       // rb, rd, tb, td, e3 (delta-scaled beam), e4 (unscaled beam)
 constexpr int SW4_LAYER = SW4_FIELDS * SW_NGPT;     // floats per layer and pass, [field][g]
 // CTA shapes of the three kernels, swept on the B200 (same bits): the gas-optics kernel at 128 threads x 6 CTAs
-// per SM against 160 x 5, 192 x 4, 256 x 3, 320 x 2, 384 x 2 (SW +0.2 to +9.8 %); the R/T kernel at 128 x 4
-// against 160 x 3, 192 x 3, 224 x 2, 256 x 2 (+1.8 to +8.3 %).
+// per SM against 160 x 5, 192 x 4, 256 x 3, 320 x 2, 384 x 2 (SW +0.2 to +9.8 %).
 constexpr int SW4_RT_THREADS = 128;                 // threads of an R/T CTA
-constexpr int SW4_OPT_MINB = 4;                     // CTAs per SM the R/T kernel is compiled for
-constexpr bool SW4_RT_PAIR = false;                 // two R/T tasks per thread side by side (else one)
+constexpr int SW4_OPT_MINB = 6;                     // CTAs per SM the R/T kernel is compiled for (4: 4.62, 5: 4.41, 6: 4.30 ms)
 constexpr int SW4_SWEEP_MINB = 6;                   // ... and the sweep kernel
 constexpr int SW4_GAS_THREADS = 128;               // threads of a gas-optics CTA
 constexpr int SW4_GAS_MINB = 6;                     // ... and the gas-optics kernel
@@ -51,100 +55,169 @@ struct Sw4Hdr {
 static_assert(sizeof(Sw4Hdr) % 16 == 0, "the header is copied in 16-byte pieces");
 __host__ __device__ constexpr size_t sw4_hdr_bytes() { return (sizeof(Sw4Hdr) + 15) / 16 * 16; }
 // One column's block of the chunk scratch: header, clear R/T [nlay][SW4_LAYER], cloudy R/T [nlay][SW4_LAYER]
-// (the first ncl slots used).
-__host__ __device__ constexpr size_t sw4_block_bytes(int nlay)
+// (the first ncl slots used), and the float64 queue of sw4_rt_kernel (16-bit entries k0 * SW_NGPT + g, the
+// table-entry tests from the front, the resonance from the back).
+__host__ __device__ constexpr size_t sw4_queue_offset(int nlay)
 {
     return sw4_hdr_bytes() + (size_t)2 * nlay * SW4_LAYER * sizeof(float);
 }
-static_assert(sw4_hdr_bytes() % 16 == 0 && (SW4_LAYER * sizeof(float)) % 16 == 0, "16-byte aligned parts");
-
-// ---- branch-free float R/T (the phase-R fast path).  Two tasks per thread run side by side, so the
-// compiler can interleave their long dependency chains; the float64 decisions become flags.
-__device__ __forceinline__ bool sw4_near(float zb)            // sw2_near without branches
+__host__ __device__ constexpr size_t sw4_block_bytes(int nlay)
 {
-    const float ft = zb / ((float)1.0f / (float)0.278f + zb);
-    const float pos = ft * (float)10000 + (float)0.5f;
-    const float fr = pos - floorf(pos);
-    const float m = 10000.0f * ft * (SW2_ZB_EPS * (1.0f - ft) + 3.0e-7f);
-    const bool tbl = fr < m || fr > 1.0f - m;
+    return sw4_queue_offset(nlay) + (size_t)nlay * SW_NGPT * sizeof(uint16_t);
+}
+// Work items of sw4_fix_kernel: at most SW4_FIX_THREADS queue entries of one column, {column of the tile,
+// first entry | entries << 16}; the list's head is the item count.
+constexpr int SW4_FIX_THREADS = 64;
+constexpr int SW4_FIX_MINB = 8;                     // CTAs per SM the fix kernel is compiled for
+__host__ __device__ constexpr int64_t sw4_max_items(int nlay) { return nlay * SW_NGPT / SW4_FIX_THREADS + 2; }
+__host__ __device__ constexpr int64_t sw4_item_bytes(int nlay, int64_t cols) { return 16 + cols * sw4_max_items(nlay) * (int64_t)sizeof(int2); }
+static_assert(sw4_hdr_bytes() % 16 == 0 && (SW4_LAYER * sizeof(float)) % 16 == 0 && SW_NGPT * sizeof(uint16_t) % 16 == 0,
+              "16-byte aligned parts");
+
+// ---- branch-free float R/T of two g-points side by side (the phase-R fast path); the float64 decisions become flags.
+struct SwRT2 {
+    F2 rb, rd, tb, td, e3, e4;
+};
+// Position of zb in the reference's exp table: ft = zb / (bpade + zb), pos = 10^4 ft + 1/2, it = floor(pos) as a float
+// (adding 2^23 rounded down leaves the integer part, so no float <-> integer conversion is needed).
+struct SwPos2 {
+    F2 ft, pos, it;
+};
+__device__ __forceinline__ SwPos2 sw4_pos(F2 zb)
+{
+    SwPos2 p;
+    p.ft = div2(zb, zb + (float)1.0f / (float)0.278f);
+    p.pos = fma2(p.ft, f2(10000.0f), f2(0.5f));
+    p.it = f2_add_rm(p.pos, f2(8388608.0f)) - 8388608.0f;
+    return p;
+}
+__device__ __forceinline__ bool sw4_near1(float zb, float pos, float it, float m)   // sw2_near without branches
+{
+    const bool tbl = fabsf((pos - it) - 0.5f) > 0.5f - m;
     const bool ser = zb > 0.06f * (1.0f - SW2_ZB_EPS);
     return zb <= 0.06f * (1.0f + SW2_ZB_EPS) ? ser : tbl;
 }
-__device__ __forceinline__ float sw4_tblexp(float zb, float& em)   // sw2_tblexp without branches
+__device__ __forceinline__ void sw4_near(F2 zb, const SwPos2& p, bool& n0, bool& n1)
 {
-    const float ftind = zb / ((float)1.0f / (float)0.278f + zb);
-    const int it = min(10000, (int)(ftind * (float)10000 + (float)0.5f));
-    const float et = it >= 10000 ? 1.0e-20f : __expf(-(3.59712230f * (float)it) / (float)(10000 - it));
-    const bool ser = zb <= 0.06f;
-    em = ser ? zb - 0.5f * zb * zb : 1.0f - et;
-    return ser ? 1.0f - zb + 0.5f * zb * zb : et;
+    const F2 m = (p.ft * 10000.0f) * fma2(f2(1.0f) - p.ft, f2(SW2_ZB_EPS), f2(3.0e-7f));
+    n0 = sw4_near1(zb.x, p.pos.x, p.it.x, m.x);
+    n1 = sw4_near1(zb.y, p.pos.y, p.it.y, m.y);
 }
-// sw2_rt_float (prologue of two-stream mode MODE, R/T, direct transmissions) without branches; ok = false where
+// The table entry exp(-bpade it / (10^4 - it)) (1e-20 for the last) and its complement, the series below 0.06
+// (sw2_tblexp without branches; bpade log2(e) folded into one constant).
+__device__ __forceinline__ float sw4_entry(float it)
+{
+    const float e = ex2a(__fdividef(-5.18955054f * it, 10000.0f - it));
+    return it >= 10000.0f ? 1.0e-20f : e;
+}
+__device__ __forceinline__ F2 sw4_tblexp(F2 zb, const SwPos2& p, F2& em)
+{
+    const F2 et{sw4_entry(p.it.x), sw4_entry(p.it.y)};
+    const F2 h = fma2(zb * -0.5f, zb, zb), ec = 1.0f - et, es = 1.0f - h;
+    const bool s0 = zb.x <= 0.06f, s1 = zb.y <= 0.06f;
+    em = F2{s0 ? h.x : ec.x, s1 ? h.y : ec.y};
+    return F2{s0 ? es.x : et.x, s1 ? es.y : et.y};
+}
+// What a float R/T is left with: nothing, a neighbouring table entry to test, or the resonance in float64.
+enum : int { SW4_Q_NONE = 0, SW4_Q_NEAR = 1, SW4_Q_RES = 2 };
+// sw2_rt_float (prologue of two-stream mode MODE, R/T, direct transmissions) without branches; q0 / q1 say where
 // sw2_rt_mixed would take a float64 step or test a neighbouring table entry (the outputs are then not used).
-template <int MODE>
-__device__ __forceinline__ void sw4_rt(float t0, float tabs, float s0, float y0, float cz, float snt, float wk, float wf,
-                                       SwLayerRT& r, bool& ok)
+// ASY = false: the asymmetry is zero (the clear pass without aerosol, 85 % of the work), so delta scaling changes
+// nothing and the three direct-beam exponentials are one.
+template <int MODE, bool ASY>
+__device__ __forceinline__ void sw4_rt(F2 t0, F2 tabs, F2 s0, F2 y0, float cz, float snt, F2 wk, F2 wf, SwRT2& r, int& q0,
+                                       int& q1)
 {
     const float ftiny = 1.0e-12f;
     const float cwmin = (float)(1.0 - ((double)1.0f - (double)1.0e-6f));
-    const float cw = fmaxf(cwmin, tabs / t0);
-    const float zssaw = 1.0f - cw;
-    const float zasyw = y0 / fmaxf(ftiny, s0);
-    const float za2s = zssaw * (zasyw * zasyw);
-    const float om = 1.0f - za2s;
-    SwPro<float> p;
-    p.ztau1 = om * t0;
-    p.zssa1 = (zssaw - za2s) / om;
-    const float cw1 = cw / om;
-    const float zasy1 = zasyw / (1.0f + zasyw), zasy3 = 0.75f * zasy1;
-    float gm, gp;
+    const F2 cw = max2(quot2(tabs, t0, rcp2(t0)), cwmin);
+    const F2 zssaw = 1.0f - cw;
+    F2 ztau1, zssa1, cw1, zasy1, zasy3;
+    if constexpr (ASY) {
+        const F2 sm = max2(s0, ftiny), zasyw = quot2(y0, sm, rcp2(sm));
+        const F2 za2s = zssaw * (zasyw * zasyw);
+        const F2 om = 1.0f - za2s, ro = rcp2(om);
+        ztau1 = om * t0;
+        zssa1 = quot2(zssaw - za2s, om, ro);
+        cw1 = quot2(cw, om, ro);
+        const F2 z1 = zasyw + 1.0f;
+        zasy1 = quot2(zasyw, z1, rcp2(z1));
+        zasy3 = zasy1 * 0.75f;
+    } else {
+        ztau1 = t0; zssa1 = zssaw; cw1 = cw; zasy1 = f2(0.0f); zasy3 = f2(0.0f);
+    }
+    F2 g1, g2, g3, gm, gp;
     if constexpr (MODE == 2) {
-        p.g1 = 2.0f - p.zssa1 * (1.25f + zasy3);
-        p.g2 = 0.75f * p.zssa1 * (1.0f - zasy1);
-        p.g3 = 0.5f - zasy3 * cz;
-        gm = 2.0f * cw1;
-        gp = 2.0f - p.zssa1 * (0.5f + 1.5f * zasy1);
+        g1 = ASY ? nma2(zssa1, zasy3 + 1.25f, f2(2.0f)) : fma2(zssa1, f2(-1.25f), f2(2.0f));
+        g2 = ASY ? (zssa1 * 0.75f) * (1.0f - zasy1) : zssa1 * 0.75f;
+        g3 = ASY ? nma2(zasy3, f2(cz), f2(0.5f)) : f2(0.5f);
+        gm = cw1 + cw1;
+        gp = ASY ? nma2(zssa1, fma2(zasy1, f2(1.5f), f2(0.5f)), f2(2.0f)) : fma2(zssa1, f2(-0.5f), f2(2.0f));
     } else if constexpr (MODE == 1) {
-        p.g1 = 1.75f - p.zssa1 * (1.0f + zasy3);
-        p.g2 = -0.25f - p.zssa1 * (1.0f - zasy3);
-        p.g3 = 0.5f - zasy3 * cz;
-        gm = p.g1 - p.g2;
-        gp = p.g1 + p.g2;
+        g1 = nma2(zssa1, zasy3 + 1.0f, f2(1.75f));
+        g2 = nma2(zssa1, 1.0f - zasy3, f2(-0.25f));
+        g3 = nma2(zasy3, f2(cz), f2(0.5f));
+        gm = g1 - g2;
+        gp = g1 + g2;
     } else {
         const float zsr3 = 1.7320508f;
-        p.g1 = zsr3 * (2.0f - p.zssa1 * (1.0f + zasy1)) * 0.5f;
-        p.g2 = zsr3 * p.zssa1 * (1.0f - zasy1) * 0.5f;
-        p.g3 = (1.0f - zsr3 * zasy1 * cz) * 0.5f;
-        gm = zsr3 * cw1;
-        gp = zsr3 * (1.0f - p.zssa1 * zasy1);
+        g1 = nma2(zssa1, zasy1 + 1.0f, f2(2.0f)) * zsr3 * 0.5f;
+        g2 = (zssa1 * zsr3) * (1.0f - zasy1) * 0.5f;
+        g3 = nma2(zasy1 * zsr3, f2(cz), f2(1.0f)) * 0.5f;
+        gm = cw1 * zsr3;
+        gp = nma2(zssa1, zasy1, f2(1.0f)) * zsr3;
     }
-    p.g4 = 1.0f - p.g3;
-    p.zrk = sqrtf(gm * gp);
-    p.zrp = p.zrk * cz;
-    p.zrpp = (1.0f - p.zrp) * (1.0f + p.zrp);
-    const float zb1 = fminf(p.zrk * p.ztau1, 500.0f), zb2 = fminf(p.ztau1 * snt, 500.0f), zb4 = t0 * snt;
-    ok = !(fabsf(p.zrpp) < SW2_RESONANCE) && !(wk > 0.0f && (sw4_near(zb1) || sw4_near(zb2))) &&
-         !(wf * 4.0e-4f > 1.0f && sw4_near(zb4));
-    float em1, em2, em;
-    const float e1 = sw4_tblexp(zb1, em1), e2 = sw4_tblexp(zb2, em2);
+    const F2 g4 = 1.0f - g3;
+    const F2 zrk = sqrt2(gm * gp);
+    const F2 zrp = zrk * cz;
+    const F2 zrpp0 = (1.0f - zrp) * (zrp + 1.0f);
+    const F2 zbd = ztau1 * snt, zb1 = min2(zrk * ztau1, 500.0f), zb2 = min2(zbd, 500.0f), zb4 = ASY ? t0 * snt : zbd;
+    const SwPos2 p1 = sw4_pos(zb1), p2 = sw4_pos(zb2);
+    F2 em1, em2, em;
+    const F2 e1 = sw4_tblexp(zb1, p1, em1), e2 = sw4_tblexp(zb2, p2, em2);
+    // exp(-ztau1 / mu0): e2's entry; past its clamp at 500 the entries underflow to 0 in float, up to the last one
+    // (10^4 ft + 1/2 >= 10^4 from zb = 71,939 on), which the table sets to 1e-20
+    const F2 eb{zbd.x > 500.0f ? (zbd.x >= 71939.0f ? 1.0e-20f : 0.0f) : e2.x,
+                zbd.y > 500.0f ? (zbd.y >= 71939.0f ? 1.0e-20f : 0.0f) : e2.y};
+    r.e3 = eb;
+    bool n10, n11, n20, n21, n40, n41;
+    sw4_near(zb1, p1, n10, n11);
+    sw4_near(zb2, p2, n20, n21);
+    if constexpr (ASY) {
+        const SwPos2 p4 = sw4_pos(zb4);
+        r.e4 = sw4_tblexp(zb4, p4, em);
+        sw4_near(zb4, p4, n40, n41);
+    } else {
+        r.e4 = eb;
+        n40 = n20 && zbd.x <= 500.0f;
+        n41 = n21 && zbd.y <= 500.0f;
+    }
+    auto code = [](float zrpp, float wk, bool n12, float wf, bool n4) {
+        return fabsf(zrpp) < SW2_RESONANCE ? SW4_Q_RES : (wk > 0.0f && n12) || (wf * 4.0e-4f > 1.0f && n4) ? SW4_Q_NEAR : SW4_Q_NONE;
+    };
+    q0 = code(zrpp0.x, wk.x, n10 || n20, wf.x, n40);
+    q1 = code(zrpp0.y, wk.y, n11 || n21, wf.y, n41);
     // sw2_rt_core with the clamp and the degenerate-denominator case as selects
     const float eps1 = 1.0e-8f;
-    const float zrpp = fabsf(p.zrpp) < eps1 ? (p.zrpp < 0 ? -eps1 : eps1) : p.zrpp;
-    const float g1 = p.g1, g2 = p.g2, g3 = p.g3, g4 = p.g4, zrk = p.zrk, zrp = p.zrp;
-    const float za1 = g1 * g4 + g2 * g3, za2 = g1 * g3 + g2 * g4;
-    const float e11 = e1 * e1, em11 = em1 * (2.0f - em1);
-    const float B = zrk * (1.0f + e11) + g1 * em11;
-    const float D = zrpp * B;
-    const bool degen = D >= -eps1 * e1 && D <= eps1 * e1;
-    const float q = p.zssa1 / D;
-    const float nr = em11 * (za2 - zrk * g3 * zrp) + zrk * (g3 - za2 * cz) * (em1 * em1 + 2.0f * e1 * em2);
-    const float nt = zrk * (g4 + za1 * cz) * (2.0f * e1 * em2 - e2 * em1 * em1) - e2 * em11 * (za1 + zrk * g4 * zrp);
-    r.rb = degen ? eps1 : fmaxf(0.0f, fminf(1.0f, nr * q));
-    r.tb = degen ? e2 : fmaxf(0.0f, fminf(1.0f, e2 + nt * q));
-    r.rd = fmaxf(0.0f, fminf(1.0f, g2 * em11 / B));
-    r.td = fmaxf(0.0f, fminf(1.0f, 2.0f * zrk * e1 / B));
-    r.e3 = sw4_tblexp(p.ztau1 * snt, em);
-    r.e4 = sw4_tblexp(zb4, em);
+    const F2 zrpp{fabsf(zrpp0.x) < eps1 ? copysignf(eps1, zrpp0.x) : zrpp0.x,
+                  fabsf(zrpp0.y) < eps1 ? copysignf(eps1, zrpp0.y) : zrpp0.y};
+    const F2 za1 = fma2(g1, g4, g2 * g3), za2 = fma2(g1, g3, g2 * g4);
+    const F2 e11 = e1 * e1, em11 = em1 * (2.0f - em1);
+    const F2 B = fma2(zrk, e11 + 1.0f, g1 * em11);
+    const F2 D = zrpp * B;
+    const F2 q = quot2(zssa1, D, rcp2(D));
+    const F2 m11 = em1 * em1, e1m2 = (e1 * em2) * 2.0f;
+    const F2 nr = fma2(em11, nma2(zrk * g3, zrp, za2), (zrk * nma2(za2, f2(cz), g3)) * (m11 + e1m2));
+    const F2 nt = nma2(e2 * em11, fma2(zrk * g4, zrp, za1), (zrk * fma2(za1, f2(cz), g4)) * nma2(e2, m11, e1m2));
+    const F2 rb = clamp01(nr * q), tb = clamp01(fma2(nt, q, e2));
+    const bool d0 = fabsf(D.x) <= eps1 * e1.x, d1 = fabsf(D.y) <= eps1 * e1.y;
+    r.rb = F2{d0 ? eps1 : rb.x, d1 ? eps1 : rb.y};
+    r.tb = F2{d0 ? e2.x : tb.x, d1 ? e2.y : tb.y};
+    // td is ~1 in the thin layers, where its rounding acts as absorption that adds up down the column: the Newton step
+    // halves the fluxes' error against float64 (sfcfsw 2.8e-7 -> 1.7e-7 relative)
+    const F2 rB = rcp2(B);
+    r.rd = clamp01(quot2(g2 * em11, B, rB));
+    r.td = clamp01(quot2((zrk + zrk) * e1, B, rB));
 }
 
 // The column image handed from the gas-optics kernel to the R/T kernel: SwSh2 from colmol to its end (taug last)
@@ -171,10 +244,11 @@ __host__ __device__ inline const float* sw4_image_taug(const int4* im)
 
 // Set-up, cloud optics and gas optics of one sunlit column (one CTA, six per SM) into its image.
 __global__ void __launch_bounds__(SW4_GAS_THREADS, SW4_GAS_MINB)
-sw4_gas_kernel(const __grid_constant__ SwBatch bt, int any_aer, int* err, int d0, int4* img)
+sw4_gas_kernel(const __grid_constant__ SwBatch bt, int any_aer, int* err, int d0, int4* img, int* items)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SwSh2& s = *reinterpret_cast<SwSh2*>(smem_raw);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *items = 0;           // the tile's work list, filled by sw4_rt_kernel
     const int d = d0 + (int)blockIdx.x;
     if (d >= *bt.req[0].nday) return;
     const int64_t gcol = bt.req[0].daycol[d];
@@ -205,13 +279,27 @@ sw4_gas_kernel(const __grid_constant__ SwBatch bt, int any_aer, int* err, int d0
     for (int i = tid; i < n1 + n2; i += SW4_GAS_THREADS) im[i < n1 ? i : i + skip] = sm[i];
 }
 
+// The column image (without taug; the aerosol block where taug would be) from global memory into the CTA's shared
+// memory, every 16-byte piece in flight at once (cp.async.cg: L2 to shared).  Returns the SwSh2 the shared memory
+// stands for: only its part from colmol on is there, so the image starts at smem and SwSh2 itself before it.
+__device__ __forceinline__ SwSh2* sw4_load_image(unsigned char* smem, const int4* im, int any_aer, int tid, int nthreads)
+{
+    const uint32_t sb = (uint32_t)__cvta_generic_to_shared(smem);
+    const int n1 = (int)((offsetof(SwSh2, taug) - sw4_image_begin()) / 16);
+    const int n2 = any_aer ? (int)(sizeof(SwAer) / 16) : 0;
+    const int skip = (int)(sizeof(SwSh2::taug) / 16);
+    for (int i = tid; i < n1 + n2; i += nthreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sb + 16u * (uint32_t)i), "l"(im + (i < n1 ? i : i + skip))
+                     : "memory");
+    return reinterpret_cast<SwSh2*>(smem - sw4_image_begin());
+}
+__host__ __device__ constexpr size_t sw4_rt_smem(bool aer) { return sw4_gas_smem(aer) - sw4_image_begin(); }
+
 __global__ void __launch_bounds__(SW4_RT_THREADS, SW4_OPT_MINB)
-sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, const float* ex, const double* exd, int d0,
-              const int4* img, unsigned char* scr, size_t blk_bytes)
+sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int4* img, unsigned char* scr, size_t blk_bytes,
+              int* items)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SwSh2& s = *reinterpret_cast<SwSh2*>(smem_raw);
-    __shared__ signed char slot[NLAY_MAX];
     const int d = d0 + (int)blockIdx.x;
     if (d >= *bt.req[0].nday) return;
     const int64_t gcol = bt.req[0].daycol[d];
@@ -219,233 +307,216 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, const float* ex, 
     const SwIn& a = bt.req[rq];
     const int nlay = a.nlay;
     if (nlay > NLAY_MAX) return;                                   // flagged by the gas-optics kernel
-    SwAer* aer = a.faersw ? reinterpret_cast<SwAer*>(smem_raw + offsetof(SwSh2, taug)) : nullptr;
-    const int64_t col = gcol - bt.off[rq];
     const int tid = threadIdx.x;
     const int4* im = img + (size_t)blockIdx.x * (sw4_image_bytes(any_aer) / 16);
     const float* tgi = sw4_image_taug(im);   // [layer][g], read from the image as the tasks need it
     if (SW4_L2PF && tid == 0) l2_prefetch(tgi, (uint32_t)(nlay * SW_NGPT * sizeof(float)));
-    {   // the rest of the image into shared memory (the aerosol block where taug would be), every 16-byte piece
-        // in flight at once (cp.async.cg: L2 to shared)
-        const uint32_t sb = (uint32_t)__cvta_generic_to_shared(smem_raw + sw4_image_begin());
-        const int n1 = (int)((offsetof(SwSh2, taug) - sw4_image_begin()) / 16);
-        const int n2 = any_aer ? (int)(sizeof(SwAer) / 16) : 0;
-        const int skip = (int)(sizeof(SwSh2::taug) / 16);
-        for (int i = tid; i < n1 + n2; i += SW4_RT_THREADS)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sb + 16u * (uint32_t)i),
-                         "l"(im + (i < n1 ? i : i + skip))
-                         : "memory");
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-    }
+    SwSh2& s = *sw4_load_image(smem_raw, im, any_aer, tid, SW4_RT_THREADS);
+    const SwAer* aer = a.faersw ? reinterpret_cast<const SwAer*>(smem_raw + sw4_rt_smem(false)) : nullptr;
     unsigned char* blk = scr + (size_t)blockIdx.x * blk_bytes;
     Sw4Hdr& H = *reinterpret_cast<Sw4Hdr*>(blk);
     float* rtc = reinterpret_cast<float*>(blk + sw4_hdr_bytes());
     float* rto = rtc + (size_t)nlay * SW4_LAYER;
+    uint16_t* queue = reinterpret_cast<uint16_t*>(blk + sw4_queue_offset(nlay));
     const bool mc = a.mask != nullptr;
+    constexpr int NP = SW_NGPT / 2;
+    __shared__ int qnear, qres;                    // float64 queue: entries from the front, from the back
+    __shared__ unsigned qbit[NLAY_MAX][4];
+    __shared__ signed char slotk[NLAY_MAX];
+    __shared__ unsigned char gband[SW_NGPT];
+    __shared__ __align__(8) float zsol[SW_NGPT];   // solar source of each g-point, H.zsolar
+    __shared__ float rdf[NLAY_MAX];                // heatfac / delp as float
+    for (int j = tid; j < NLAY_MAX * 4; j += SW4_RT_THREADS) qbit[j >> 2][j & 3] = 0u;
+    if (tid == 0) { qnear = 0; qres = 0; }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
     const bool cloudy = mc ? s.zcf1 > 0.0f : s.zcf1 > 1.0e-6f;
-    // the queue of (layer, g-point) tasks whose float64 work is left for the pass after the R/T (the level-sum
-    // scratch fn is not used by this kernel): count, then entries k0 * SW_NGPT + g
-    int* qn = reinterpret_cast<int*>(&s.fn[0][0]);
-    int* qe = qn + 1;
-    constexpr int QCAP = (int)(sizeof(SwSh2::fn) / sizeof(int)) - 1;
+    // layers with a cloudy-pass R/T, counted from the surface (every warp forms the two words of layer bits)
+    unsigned cw[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int k0 = 32 * h + (tid & 31);
+        cw[h] = __ballot_sync(0xffffffffu, cloudy && k0 < nlay && s.cldfrc[k0] > 1.0e-12f);
+    }
+    const int ncl = __popc(cw[0]) + __popc(cw[1]);
+    for (int k0 = tid; k0 < nlay; k0 += SW4_RT_THREADS) {
+        const unsigned below = (1u << (k0 & 31)) - 1u;
+        const int sl = k0 < 32 ? __popc(cw[0] & below) : __popc(cw[0]) + __popc(cw[1] & below);
+        const bool cl = (cw[k0 >> 5] >> (k0 & 31)) & 1u;
+        H.slot[k0] = cl ? (signed char)sl : (signed char)-1;
+        if (cl) slotk[sl] = (signed char)k0;
+        H.rdelp[k0] = s.rdelp[k0];
+        rdf[k0] = (float)s.rdelp[k0];
+    }
+    for (int g = tid; g < SW_NGPT; g += SW4_RT_THREADS) {
+        gband[g] = c_sw_band[g];
+        const float z = s.ssolar * s.sfluxzen[g];
+        zsol[g] = z;
+        H.zsolar[g] = z;
+    }
     if (tid == 0) {
-        int n = 0;
-        for (int k0 = 0; k0 < nlay; ++k0) {
-            const bool cl = cloudy && s.cldfrc[k0] > 1.0e-12f;
-            slot[k0] = cl ? (signed char)n : (signed char)-1;
-            H.slot[k0] = slot[k0];
-            n += cl ? 1 : 0;
-        }
-        H.ncl = n;
+        H.ncl = ncl;
         H.cloudy = cloudy ? 1 : 0;
         H.albbm[0] = s.albbm[0]; H.albbm[1] = s.albbm[1];
         H.albdf[0] = s.albdf[0]; H.albdf[1] = s.albdf[1];
         H.zcf0 = s.zcf0; H.zcf1 = s.zcf1;
-        *qn = 0;
     }
-    for (int k0 = tid; k0 < nlay; k0 += SW4_RT_THREADS) H.rdelp[k0] = s.rdelp[k0];
-    for (int g = tid; g < SW_NGPT; g += SW4_RT_THREADS) H.zsolar[g] = s.ssolar * s.sfluxzen[g];
-    __syncthreads();
     const float cz = s.cosz, snt = s.sntz;
-    const double czd = (double)__ldg(a.coszen + col);
-    __shared__ unsigned char gband[SW_NGPT];
-    for (int g = tid; g < SW_NGPT; g += SW4_RT_THREADS) {
-        int ib = 0;
-        while (g >= c_sw_ns[ib + 1]) ++ib;
-        gband[g] = (unsigned char)ib;
-    }
     __syncthreads();
-    auto store = [&](int k0, int g, const SwLayerRT2& L) {
-        float* pc = rtc + (size_t)k0 * SW4_LAYER + g;
-        pc[0] = L.c.rb; pc[SW_NGPT] = L.c.rd; pc[2 * SW_NGPT] = L.c.tb; pc[3 * SW_NGPT] = L.c.td;
-        pc[4 * SW_NGPT] = L.c.e3; pc[5 * SW_NGPT] = L.c.e4;
-        const int sl = slot[k0];
-        if (sl >= 0) {
-            float* po = rto + (size_t)sl * SW4_LAYER + g;
-            po[0] = L.o.rb; po[SW_NGPT] = L.o.rd; po[2 * SW_NGPT] = L.o.tb; po[3 * SW_NGPT] = L.o.td;
-            po[4 * SW_NGPT] = L.o.e3; po[5 * SW_NGPT] = L.o.e4;
-        }
-    };
-    // the complete layer function (sw2_layer, float64 steps included) for task i = k0 * SW_NGPT + g
-    auto full = [&](int i) {
-        const int k0 = i / SW_NGPT, g = i - k0 * SW_NGPT, ib = gband[g];
-        const float zsolar = s.ssolar * s.sfluxzen[g];
-        const SwExactCtx x{&a, col, s.laytrop, s.kmin8, s.kminw, a.iswmode, czd, 1.0 / czd, exd,
-                           zsolar * (1.5f * 86400.0f / SW2_HEAT_T), zsolar * (1.0f / SW2_FLUX_T)};
-        store(k0, g, sw2_layer(s, aer, x, k0, g, ib, cloudy, mc, cz, snt, ex, __ldg(tgi + i)));
-    };
-    // ---- layer R/T in two passes over the column, each with lanes on 32 consecutive (layer, g-point) tasks and
-    // two tasks per thread side by side; a task whose R/T needs a float64 step or a table-entry test is queued
-    // (qbit marks it) and formed afterwards by sw2_layer, one per thread
-    __shared__ unsigned qbit[NLAY_MAX][4];
-    __shared__ signed char slotk[NLAY_MAX];
-    for (int j = tid; j < NLAY_MAX * 4; j += SW4_RT_THREADS) qbit[j >> 2][j & 3] = 0u;
-    if (tid < nlay && slot[tid] >= 0) slotk[slot[tid]] = (signed char)tid;
-    __syncthreads();
-    const int ncl = H.ncl;
-    auto enqueue = [&](int i) {
-        const int k0 = i / SW_NGPT, g = i - k0 * SW_NGPT;
+    // ---- layer R/T in two passes over the column; a task is a pair of neighbouring g-points of one layer (every
+    // band starts at an even g-point and has an even count, so the pair shares its band's optics), lanes on 32
+    // consecutive pairs of the [layer][g-point pair] order.  A g-point whose R/T needs a float64 step or a
+    // table-entry test is queued once (qbit marks it) for sw4_fix_kernel
+    auto enqueue = [&](int k0, int g, int code) {
         if (atomicOr(&qbit[k0][g >> 5], 1u << (g & 31)) & (1u << (g & 31))) return;   // queued already
-        const int j = atomicAdd(qn, 1);
-        if (j < QCAP) qe[j] = i;
-        else full(i);
+        const int e = code == SW4_Q_NEAR ? atomicAdd(&qnear, 1) : nlay * SW_NGPT - 1 - atomicAdd(&qres, 1);
+        queue[e] = (uint16_t)(k0 * SW_NGPT + g);
     };
-    // clear-pass inputs of task i
-    auto inputs = [&](int i, float& t0, float& ab, float& s0, float& y0, int& ib) {
-        const int k0 = i / SW_NGPT, g = i - k0 * SW_NGPT;
-        ib = gband[g];
-        const float tr = sw2_taur(s, g, k0), tg = __ldg(tgi + i);
-        float ta = 0, tasa = 0, tay = 0, taab = 0;
-        if (aer) { ta = aer->tau[ib][k0]; tasa = aer->tasa[ib][k0]; tay = aer->tay[ib][k0]; taab = aer->tabs[ib][k0]; }
-        t0 = fmaxf(1.0e-12f, tr + tg + ta); s0 = tr + tasa; y0 = tay; ab = tg + taab;
+    auto ld2 = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return F2{v.x, v.y}; };
+    auto st2 = [](float* p, F2 v) { *reinterpret_cast<float2*>(p) = make_float2(v.x, v.y); };
+    // clear-pass inputs of the pair (g, g + 1) of layer k0
+    auto inputs = [&](int k0, int g, int ib, F2& t0, F2& ab, F2& s0, F2& y0) {
+        const float2 tv = __ldg(reinterpret_cast<const float2*>(tgi + k0 * SW_NGPT + g));
+        const F2 tg{tv.x, tv.y};
+        F2 tr;
+        if (g >= 66 && g < 74 && k0 < s.laytrop) tr = F2{s.taur24[g - 66][k0], s.taur24[g - 65][k0]};
+        else tr = ld2(s.raylc + g) * s.colmol[k0];
+        t0 = tr + tg; s0 = tr; y0 = f2(0.0f); ab = tg;
+        if (aer) {
+            t0 = t0 + aer->tau[ib][k0]; s0 = s0 + aer->tasa[ib][k0]; y0 = f2(aer->tay[ib][k0]);
+            ab = ab + aer->tabs[ib][k0];
+        }
+        t0 = max2(t0, 1.0e-12f);
     };
-    auto weights = [&](int i, float& wk, float& wf) {
-        const int k0 = i / SW_NGPT, g = i - k0 * SW_NGPT;
-        const float zsolar = s.ssolar * s.sfluxzen[g];
-        wf = zsolar * (1.0f / SW2_FLUX_T);
-        wk = zsolar * (1.5f * 86400.0f / SW2_HEAT_T) * (float)s.rdelp[k0];
+    auto weights = [&](int k0, int g, F2& wk, F2& wf) {
+        const F2 zs = ld2(zsol + g);
+        wf = zs * (1.0f / SW2_FLUX_T);
+        wk = zs * (1.5f * 86400.0f / SW2_HEAT_T) * rdf[k0];
     };
-    auto put = [&](float* base, int i, const SwLayerRT& r) {
-        float* p = base + i;   // i = k0 * SW_NGPT + g indexes [layer][g]; fields are SW_NGPT apart
-        const int k0 = i / SW_NGPT;
-        p += (size_t)k0 * (SW4_LAYER - SW_NGPT);
-        p[0] = r.rb; p[SW_NGPT] = r.rd; p[2 * SW_NGPT] = r.tb; p[3 * SW_NGPT] = r.td; p[4 * SW_NGPT] = r.e3;
-        p[5 * SW_NGPT] = r.e4;
+    auto put = [&](float* p, const SwRT2& r) {   // p: the pair's place in field 0 of its layer's rows
+        st2(p, r.rb); st2(p + SW_NGPT, r.rd); st2(p + 2 * SW_NGPT, r.tb); st2(p + 3 * SW_NGPT, r.td);
+        st2(p + 4 * SW_NGPT, r.e3); st2(p + 5 * SW_NGPT, r.e4);
     };
     auto run = [&](auto mode_tag) {
         constexpr int MODE = decltype(mode_tag)::value;
-        const int nt = nlay * SW_NGPT;
         // clear pass
-        if constexpr (!SW4_RT_PAIR) {
-            for (int i0 = tid; i0 < nt; i0 += SW4_RT_THREADS) {
-                float t0a, aba, s0a, y0a, wka, wfa;
-                int iba;
-                inputs(i0, t0a, aba, s0a, y0a, iba);
-                weights(i0, wka, wfa);
-                SwLayerRT ra;
-                bool oka;
-                sw4_rt<MODE>(t0a, aba, s0a, y0a, cz, snt, wka, wfa, ra, oka);
-                put(rtc, i0, ra);
-                if (!oka) enqueue(i0);
+        auto clear = [&](auto asy_tag) {
+            for (int i = tid; i < nlay * NP; i += SW4_RT_THREADS) {
+                const int k0 = i / NP, g = 2 * (i - k0 * NP);
+                F2 t0, ab, s0, y0, wk, wf;
+                inputs(k0, g, gband[g], t0, ab, s0, y0);
+                weights(k0, g, wk, wf);
+                SwRT2 r;
+                int q0, q1;
+                sw4_rt<MODE, decltype(asy_tag)::value>(t0, ab, s0, y0, cz, snt, wk, wf, r, q0, q1);
+                put(rtc + (size_t)k0 * SW4_LAYER + g, r);
+                if (q0) enqueue(k0, g, q0);
+                if (q1) enqueue(k0, g + 1, q1);
             }
-        }
-        for (int i0 = tid; SW4_RT_PAIR && i0 < nt; i0 += 2 * SW4_RT_THREADS) {
-            const int i1 = min(i0 + SW4_RT_THREADS, nt - 1);
-            float t0a, aba, s0a, y0a, t0b, abb, s0b, y0b, wka, wfa, wkb, wfb;
-            int iba, ibb;
-            inputs(i0, t0a, aba, s0a, y0a, iba);
-            inputs(i1, t0b, abb, s0b, y0b, ibb);
-            weights(i0, wka, wfa);
-            weights(i1, wkb, wfb);
-            SwLayerRT ra, rb;
-            bool oka, okb;
-            sw4_rt<MODE>(t0a, aba, s0a, y0a, cz, snt, wka, wfa, ra, oka);
-            sw4_rt<MODE>(t0b, abb, s0b, y0b, cz, snt, wkb, wfb, rb, okb);
-            put(rtc, i0, ra);
-            if (!oka) enqueue(i0);
-            if (i0 + SW4_RT_THREADS < nt) {
-                put(rtc, i1, rb);
-                if (!okb) enqueue(i1);
-            }
-        }
+        };
+        if (MODE == 1 || aer) clear(std::true_type{});
+        else clear(std::false_type{});
         __syncthreads();
         // cloudy pass: the layers with a slot, mixture R/T blended with the clear R/T (or, McICA, taken
         // unblended where the g-point's sub-column bit is set)
-        const int nc2 = ncl * SW_NGPT;
-        auto mix = [&](int j, SwLayerRT& o, bool& ok, int& i) {
-            const int sl = j / SW_NGPT, g = j - sl * SW_NGPT, k0 = slotk[sl];
-            i = k0 * SW_NGPT + g;
-            float t0, ab, s0, y0, wk, wf;
-            int ib;
-            inputs(i, t0, ab, s0, y0, ib);
-            weights(i, wk, wf);
+        for (int j = tid; j < ncl * NP; j += SW4_RT_THREADS) {
+            const int sl = j / NP, g = 2 * (j - sl * NP), k0 = slotk[sl], ib = gband[g];
+            F2 t0, ab, s0, y0, wk, wf;
+            inputs(k0, g, ib, t0, ab, s0, y0);
+            weights(k0, g, wk, wf);
+            int q0, q1;
+            SwRT2 m;
+            sw4_rt<MODE, true>(t0 + s.taucw[ib][k0], ab + s.tabsc[ib][k0], s0 + s.ssacw[ib][k0], y0 + s.asycw[ib][k0], cz,
+                               snt, wk, wf, m, q0, q1);
             const float* pc = rtc + (size_t)k0 * SW4_LAYER + g;
-            SwLayerRT c;
-            c.rb = pc[0]; c.rd = pc[SW_NGPT]; c.tb = pc[2 * SW_NGPT]; c.td = pc[3 * SW_NGPT]; c.e3 = pc[4 * SW_NGPT];
-            c.e4 = pc[5 * SW_NGPT];
-            const bool bit = !mc || ((s.mcw[g >> 5][k0] >> (g & 31)) & 1u);
-            SwLayerRT m;
-            sw4_rt<MODE>(t0 + s.taucw[ib][k0], ab + s.tabsc[ib][k0], s0 + s.ssacw[ib][k0], y0 + s.asycw[ib][k0], cz,
-                         snt, wk, wf, m, ok);
-            ok = ok || !bit;
-            if (!bit) {
-                o = c;
-            } else if (mc) {
-                o = m;
+            const SwRT2 c{ld2(pc), ld2(pc + SW_NGPT), ld2(pc + 2 * SW_NGPT), ld2(pc + 3 * SW_NGPT), ld2(pc + 4 * SW_NGPT),
+                          ld2(pc + 5 * SW_NGPT)};
+            if (mc) {
+                const unsigned w = s.mcw[g >> 5][k0] >> (g & 31);
+                const bool b0 = w & 1u, b1 = w & 2u;
+                auto pick = [&](F2 x, F2 y) { return F2{b0 ? x.x : y.x, b1 ? x.y : y.y}; };
+                m.rb = pick(m.rb, c.rb); m.rd = pick(m.rd, c.rd); m.tb = pick(m.tb, c.tb); m.td = pick(m.td, c.td);
+                m.e3 = pick(m.e3, c.e3); m.e4 = pick(m.e4, c.e4);
+                q0 = b0 ? q0 : SW4_Q_NONE;
+                q1 = b1 ? q1 : SW4_Q_NONE;
             } else {
                 const float zc1 = s.cldfrc[k0], zc0 = 1.0f - zc1;
-                o.rb = zc0 * c.rb + zc1 * m.rb;
-                o.rd = zc0 * c.rd + zc1 * m.rd;
-                o.tb = zc0 * c.tb + zc1 * m.tb;
-                o.td = zc0 * c.td + zc1 * m.td;
-                o.e3 = zc0 * c.e3 + zc1 * m.e3;
-                o.e4 = zc0 * c.e4 + zc1 * m.e4;
+                auto mix = [&](F2 x, F2 y) { return fma2(y, f2(zc0), x * zc1); };
+                m.rb = mix(m.rb, c.rb); m.rd = mix(m.rd, c.rd); m.tb = mix(m.tb, c.tb); m.td = mix(m.td, c.td);
+                m.e3 = mix(m.e3, c.e3); m.e4 = mix(m.e4, c.e4);
             }
-        };
-        if constexpr (!SW4_RT_PAIR) {
-            for (int j0 = tid; j0 < nc2; j0 += SW4_RT_THREADS) {
-                SwLayerRT oa;
-                bool oka;
-                int ia;
-                mix(j0, oa, oka, ia);
-                const int k0 = ia / SW_NGPT, g = ia - k0 * SW_NGPT;
-                if (!(qbit[k0][g >> 5] & (1u << (g & 31)))) {
-                    put(rto, (int)(slot[k0]) * SW_NGPT + g, oa);
-                    if (!oka) enqueue(ia);
-                }
-            }
-        }
-        for (int j0 = tid; SW4_RT_PAIR && j0 < nc2; j0 += 2 * SW4_RT_THREADS) {
-            const int j1 = min(j0 + SW4_RT_THREADS, nc2 - 1);
-            SwLayerRT oa, ob;
-            bool oka, okb;
-            int ia, ib_;
-            mix(j0, oa, oka, ia);
-            mix(j1, ob, okb, ib_);
-            {
-                const int k0 = ia / SW_NGPT, g = ia - k0 * SW_NGPT;
-                if (!(qbit[k0][g >> 5] & (1u << (g & 31)))) {
-                    put(rto, (int)(slot[k0]) * SW_NGPT + g, oa);
-                    if (!oka) enqueue(ia);
-                }
-            }
-            if (j0 + SW4_RT_THREADS < nc2) {
-                const int k0 = ib_ / SW_NGPT, g = ib_ - k0 * SW_NGPT;
-                if (!(qbit[k0][g >> 5] & (1u << (g & 31)))) {
-                    put(rto, (int)(slot[k0]) * SW_NGPT + g, ob);
-                    if (!okb) enqueue(ib_);
-                }
-            }
+            put(rto + (size_t)sl * SW4_LAYER + g, m);
+            if (q0) enqueue(k0, g, q0);
+            if (q1) enqueue(k0, g + 1, q1);
         }
     };
     if (a.iswmode == 1) run(std::integral_constant<int, 1>{});
     else if (a.iswmode == 2) run(std::integral_constant<int, 2>{});
     else run(std::integral_constant<int, 3>{});
     __syncthreads();
-    // ---- the queued tasks with their float64 steps, one per thread
-    const int nq = min(*qn, QCAP);
-    for (int j = tid; j < nq; j += SW4_RT_THREADS) full(qe[j]);
+    // ---- the column's queue as work items of the tile
+    if (tid == 0) {
+        const int n1 = (qnear + SW4_FIX_THREADS - 1) / SW4_FIX_THREADS, n2 = (qres + SW4_FIX_THREADS - 1) / SW4_FIX_THREADS;
+        if (n1 + n2 > 0) {
+            int2* it = reinterpret_cast<int2*>(items + 4) + atomicAdd(items, n1 + n2);
+            for (int j = 0; j < n1; ++j) {
+                const int e = j * SW4_FIX_THREADS;
+                it[j] = make_int2((int)blockIdx.x, e | min(SW4_FIX_THREADS, qnear - e) << 16);
+            }
+            for (int j = 0; j < n2; ++j) {
+                const int e = j * SW4_FIX_THREADS;
+                it[n1 + j] = make_int2((int)blockIdx.x, nlay * SW_NGPT - qres + e | min(SW4_FIX_THREADS, qres - e) << 16);
+            }
+        }
+    }
+}
+
+// The queued g-points of a tile: the complete layer function (sw2_layer, float64 steps included) over the float R/T
+// that sw4_rt_kernel wrote.  A column has ~50 near-entry tests and, in the 1 % of columns with mu0 near a two-stream
+// resonance that all strongly absorbing layers share, thousands of float64 R/T; so the tile's queue is cut into items
+// of at most 64 entries of one column, which a grid of resident CTAs walks.
+__global__ void __launch_bounds__(SW4_FIX_THREADS, SW4_FIX_MINB)
+sw4_fix_kernel(const __grid_constant__ SwBatch bt, int any_aer, const float* ex, const double* exd, int d0, const int4* img,
+               unsigned char* scr, size_t blk_bytes, const int* items)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = items[0], tid = threadIdx.x;
+    for (int w = blockIdx.x; w < n; w += gridDim.x) {
+        const int2 it = reinterpret_cast<const int2*>(items + 4)[w];
+        const int64_t gcol = bt.req[0].daycol[d0 + it.x];
+        const int rq = bt.find(gcol);
+        const SwIn& a = bt.req[rq];
+        const int nlay = a.nlay;
+        const int64_t col = gcol - bt.off[rq];
+        const int4* im = img + (size_t)it.x * (sw4_image_bytes(any_aer) / 16);
+        SwSh2& s = *sw4_load_image(smem_raw, im, any_aer, tid, SW4_FIX_THREADS);
+        const SwAer* aer = a.faersw ? reinterpret_cast<const SwAer*>(smem_raw + sw4_rt_smem(false)) : nullptr;
+        unsigned char* blk = scr + (size_t)it.x * blk_bytes;
+        const Sw4Hdr& H = *reinterpret_cast<const Sw4Hdr*>(blk);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const int e0 = it.y & 0xffff, ne = it.y >> 16;
+        if (tid < ne) {
+            const int i = reinterpret_cast<const uint16_t*>(blk + sw4_queue_offset(nlay))[e0 + tid];
+            const int k0 = i / SW_NGPT, g = i - k0 * SW_NGPT;
+            const float zsolar = H.zsolar[g];
+            const double czd = (double)__ldg(a.coszen + col);
+            const SwExactCtx x{&a, col, s.laytrop, s.kmin8, s.kminw, a.iswmode, czd, 1.0 / czd, exd,
+                               zsolar * (1.5f * 86400.0f / SW2_HEAT_T), zsolar * (1.0f / SW2_FLUX_T)};
+            const SwLayerRT2 L = sw2_layer(s, aer, x, k0, g, c_sw_band[g], H.cloudy != 0, a.mask != nullptr, s.cosz, s.sntz,
+                                           ex, __ldg(sw4_image_taug(im) + i));
+            float* pc = reinterpret_cast<float*>(blk + sw4_hdr_bytes()) + (size_t)k0 * SW4_LAYER + g;
+            pc[0] = L.c.rb; pc[SW_NGPT] = L.c.rd; pc[2 * SW_NGPT] = L.c.tb; pc[3 * SW_NGPT] = L.c.td;
+            pc[4 * SW_NGPT] = L.c.e3; pc[5 * SW_NGPT] = L.c.e4;
+            const int sl = H.slot[k0];
+            if (sl >= 0) {
+                float* po = pc + (size_t)(nlay - k0 + sl) * SW4_LAYER;
+                po[0] = L.o.rb; po[SW_NGPT] = L.o.rd; po[2 * SW_NGPT] = L.o.tb; po[3 * SW_NGPT] = L.o.td;
+                po[4 * SW_NGPT] = L.o.e3; po[5 * SW_NGPT] = L.o.e4;
+            }
+        }
+        __syncthreads();                           // shared memory is reused by the next item
+    }
 }
 
 // Per-g-point level fluxes of one sunlit column for swrad's optional outputs (DIAG sweeps):
