@@ -31,7 +31,12 @@
 namespace rad {
 __constant__ int c_lw_ns[17] = {0, 10, 22, 38, 52, 68, 76, 88, 96, 108, 114, 122, 130, 134, 136, 138, 140};
 __constant__ int c_sw_ns[15] = {0, 6, 18, 26, 34, 44, 54, 56, 66, 74, 80, 86, 94, 100, 112};
-// band of each SW g-point
+// band of each LW / SW g-point
+__constant__ unsigned char c_lw_band[140] = {
+    0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2, 2,
+    3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 5, 5, 5, 5, 5, 5, 5, 5,
+    6, 6, 6, 6, 6, 6, 6, 6, 6, 6, 6, 6, 7, 7, 7, 7, 7, 7, 7, 7, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 9, 9, 9, 9, 9, 9,
+    10, 10, 10, 10, 10, 10, 10, 10, 11, 11, 11, 11, 11, 11, 11, 11, 12, 12, 12, 12, 13, 13, 14, 14, 15, 15};
 __constant__ unsigned char c_sw_band[112] = {
     0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2, 2, 2, 3, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4,
     4, 4, 4, 4, 4, 4, 5, 5, 5, 5, 5, 5, 5, 5, 5, 5, 6, 6, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 8, 8, 8, 8, 8, 8, 8, 8, 9, 9,
@@ -217,6 +222,7 @@ void lw_lut(std::vector<R>& v)   // [ex | tfn | tau], 3 x 10001 (phys_rrtm_lw_rt
     }
     ex[n] = expeps; tau[n] = (R)1.0e10f; tfn[n] = 1;
 }
+constexpr int64_t LW_LUT2 = 3 * 10001 + 1;   // the float32 LUT's {exp, tfn} pairs (8-byte aligned) start here
 template <class R>
 void sw_lut(std::vector<R>& v)   // exp_tbl(0:10000) (phys_rrtm_sw_spcvrtc.py:60-73)
 {
@@ -509,8 +515,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
         if (sizeof(R) == 4 && lwc > 0) {
             // per chunk: gas optics into the scratch, one warp per column sweeps, then (NAM route) the flagged
             // columns -- a cloudy layer under 1 hPa -- again by the float64 column kernel
-            LwLut<float> fl;
-            fl.ex = h->d_lwf; fl.tfn = h->d_lwf + 10001; fl.tau = h->d_lwf + 2 * 10001;
+            const float2* fl = reinterpret_cast<const float2*>(h->d_lwf + LW_LUT2);
             LwLut<double> dl;
             dl.ex = h->d_lwd; dl.tfn = h->d_lwd + 10001; dl.tau = h->d_lwd + 2 * 10001;
             const size_t smem1 = sizeof(LwSetupK<float>), smemd = sizeof(LwShared<double>);
@@ -521,22 +526,18 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 const int64_t nc = std::min(lstep, ntot - c0);
                 RAD_CUDA(h, cudaMemsetAsync(h->d_lw3list, 0, sizeof(int), st));
                 lw3_optics_kernel<<<(unsigned)nc, LW3_OPT_THREADS, smem1, st>>>(bt, c0, h->d_lw3, h->d_lw3list, h->d_err);
-                const unsigned g2 = (unsigned)((nc + LW3_SWEEP_WARPS - 1) / LW3_SWEEP_WARPS);
+                const unsigned g2 = (unsigned)std::min<int64_t>(nc, h->nsm);
                 float* pg = h->d_lwpg;
-                if (mc) {
-                    if (diag_lw) lw3_sweep_kernel<LW_OVR_MCICA, true><<<g2, LW3_SWEEP_WARPS * 32, 0, st>>>(bt, c0, nc, h->d_lw3, fl, h->d_err, pg);
-                    else lw3_sweep_kernel<LW_OVR_MCICA><<<g2, LW3_SWEEP_WARPS * 32, 0, st>>>(bt, c0, nc, h->d_lw3, fl, h->d_err);
-                    h->launches += 2;
-                } else {
-                    if (cfg.iovrlw == 0) {
-                        if (diag_lw) lw3_sweep_kernel<LW_OVR_RANDOM, true><<<g2, LW3_SWEEP_WARPS * 32, 0, st>>>(bt, c0, nc, h->d_lw3, fl, h->d_err, pg);
-                        else lw3_sweep_kernel<LW_OVR_RANDOM><<<g2, LW3_SWEEP_WARPS * 32, 0, st>>>(bt, c0, nc, h->d_lw3, fl, h->d_err);
-                    } else {
-                        if (diag_lw) lw3_sweep_kernel<LW_OVR_MAXRAN, true><<<g2, LW3_SWEEP_WARPS * 32, 0, st>>>(bt, c0, nc, h->d_lw3, fl, h->d_err, pg);
-                        else lw3_sweep_kernel<LW_OVR_MAXRAN><<<g2, LW3_SWEEP_WARPS * 32, 0, st>>>(bt, c0, nc, h->d_lw3, fl, h->d_err);
-                    }
+                const auto sweep = mc ? (diag_lw ? lw3_sweep_kernel<LW_OVR_MCICA, true> : lw3_sweep_kernel<LW_OVR_MCICA>)
+                                   : cfg.iovrlw == 0
+                                       ? (diag_lw ? lw3_sweep_kernel<LW_OVR_RANDOM, true> : lw3_sweep_kernel<LW_OVR_RANDOM>)
+                                       : (diag_lw ? lw3_sweep_kernel<LW_OVR_MAXRAN, true> : lw3_sweep_kernel<LW_OVR_MAXRAN>);
+                RAD_CUDA(h, cudaFuncSetAttribute((const void*)sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lw3_sweep_smem()));
+                sweep<<<g2, LW3_SWEEP_WARPS * 32, lw3_sweep_smem(), st>>>(bt, c0, nc, h->d_lw3, fl, pg);
+                h->launches += 2;
+                if (!mc) {
                     lw3_fp64_kernel<<<(unsigned)h->nsm, LW_THREADS, smemd, st>>>(bt, c0, h->d_lw3list, dl, h->d_err);
-                    h->launches += 3;
+                    h->launches += 1;
                 }
                 if (diag_lw) {
                     k_lw_diag<<<(unsigned)((nc + 3) / 4), 128, 0, st>>>(bt, c0, nc, pg, dout);
@@ -791,6 +792,11 @@ int rad_load_tables(RadHandle* h, const void* blob, size_t nbytes)
     std::vector<float> lwf, swf;
     std::vector<double> lwd, swd;
     lw_lut(lwf); lw_lut(lwd); sw_lut(swf); sw_lut(swd);
+    lwf.resize(LW_LUT2, 0.0f);                   // then the sweeps' copy, {exp, tfn} per entry
+    for (int i = 0; i <= 10000; ++i) {
+        lwf.push_back(lwf[i]);
+        lwf.push_back(lwf[10001 + i]);
+    }
     int rc;
     if ((rc = upload(h, &h->d_lwf, lwf)) || (rc = upload(h, &h->d_lwd, lwd)) || (rc = upload(h, &h->d_swf, swf)) ||
         (rc = upload(h, &h->d_swd, swd)))

@@ -62,4 +62,30 @@ __device__ __forceinline__ float ex2a(float x)
     return r;
 }
 
+// The same names on one float, for code that runs a pair or a single g-point (V = F2 or float).
+template <class V> __device__ __forceinline__ V vset(float a);
+template <> __device__ __forceinline__ F2 vset<F2>(float a) { return f2(a); }
+template <> __device__ __forceinline__ float vset<float>(float a) { return a; }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float nma2(float a, float b, float c) { return fmaf(-a, b, c); }
+__device__ __forceinline__ float f2_add_rm(float a, float b) { return __fadd_rd(a, b); }
+__device__ __forceinline__ float max2(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ float div2(float a, float b) { return __fdividef(a, b); }
+__device__ __forceinline__ float rcp2(float a) { return __fdividef(1.0f, a); }
+__device__ __forceinline__ float quot2(float a, float b, float r)
+{
+    const float q = a * r;
+    return fmaf(nma2(q, b, a), r, q);
+}
+// a <= b, a < b per component
+struct B2 {
+    bool x, y;
+};
+__device__ __forceinline__ B2 le2(F2 a, float b) { return B2{a.x <= b, a.y <= b}; }
+__device__ __forceinline__ bool le2(float a, float b) { return a <= b; }
+__device__ __forceinline__ B2 lt2(F2 a, float b) { return B2{a.x < b, a.y < b}; }
+__device__ __forceinline__ bool lt2(float a, float b) { return a < b; }
+__device__ __forceinline__ F2 sel2(B2 c, F2 a, F2 b) { return F2{c.x ? a.x : b.x, c.y ? a.y : b.y}; }
+__device__ __forceinline__ float sel2(bool c, float a, float b) { return c ? a : b; }
+
 }  // namespace rad

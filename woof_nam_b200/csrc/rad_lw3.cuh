@@ -9,13 +9,11 @@
 //                      rtrnmr), with taug / fracs written straight to the chunk's scratch and the sweep inputs
 //                      copied after them.  Shared memory is the set-up data and the species keys of bands 3,
 //                      4, 5, 7 and 9 (LwSetupK, ~50 KB).
-//   lw3_sweep_kernel   one warp per column: lane l carries g-points l, l + 32, ..., l + 128 (five independent
-//                      recurrences interleaved per lane), reading each layer's optical depths as coalesced
-//                      128-byte rows staged through shared memory by asynchronous copies.  Per layer each
-//                      g-point's radiance CHANGE across the layer is formed directly (source minus radiance x
-//                      absorptance) and summed over g-points in float64; the
-//                      heating rates come from those changes, not from differences of ~300 W/m^2 level
-//                      fluxes.
+//   lw3_sweep_kernel   one warp per column, the two sweeps with the g-points in packed pairs (rad_f32x2.cuh), reading
+//                      each layer's row of the scratch staged through shared memory by asynchronous copies.  Per
+//                      layer each g-point's radiance CHANGE across the layer is formed directly (source minus
+//                      radiance x absorptance) and summed over g-points in float64; the heating rates come from
+//                      those changes, not from differences of ~300 W/m^2 level fluxes.
 //   lw3_fp64_kernel    the plain float64 LW column (lw_column_body<double>) for the columns the optics kernel
 //                      flags: a cloudy layer thinner than LW3_THIN hPa.  Such a layer (a cloud in the 0.1 hPa
 //                      top layer of the precision-stress request) cools at thousands of K/day, and 1e-5 of
@@ -23,21 +21,22 @@
 //                      neighbouring entry of the 10,001-entry transmittance table, and float radiances
 //                      carry ~1e-6 through the column.  Other columns exit at once.
 //
-// Scratch block of one column (floats, 128-byte aligned): taug [nlay][160], fracs [nlay][160] (g-points
-// 140..159 unused), then one 80-word record per layer k = 1..nlay holding everything the sweeps read at that
-// layer (so a layer step touches one contiguous record) and a head record (k = 0) for the surface.  The
-// arithmetic of every term and recurrence is that of rad_lw2.cuh (rtrnmr,
-// phys_rrtm_lw_rtrnmr_body.cuh:130-330; rtrnmc, phys_rrtm_lw_rtrnmc.cu:85-310; rtrn,
+// Scratch block of one column (floats, 128-byte aligned): a head record for the surface, then per layer (surface
+// first) one row: the 140 optical depths, the 140 Planck fractions and an 80-word record holding everything else the
+// sweeps read at that layer, so a layer step reads one contiguous run of 1,440 bytes.  The recurrences are those of
+// rad_lw2.cuh (rtrnmr, phys_rrtm_lw_rtrnmr_body.cuh:130-330; rtrnmc, phys_rrtm_lw_rtrnmc.cu:85-310; rtrn,
 // phys_rrtm_lw_rtrn.cu:94-330).
 #pragma once
+#include "rad_f32x2.cuh"
 #include "rad_lw2.cuh"
 
 namespace rad {
 
-constexpr int LW3_GSTRIDE = 160;                         // floats per layer row of taug / fracs
-constexpr int LW3_SLOTS = 5;                             // g-points per lane in the sweeps
-constexpr int LW3_SWEEP_WARPS = 4;                       // columns per sweep CTA
+constexpr int LW3_SWEEP_WARPS = 16;                      // warps of a sweep CTA (one CTA per SM)
 constexpr int LW3_REC = 80;                              // words per layer record
+constexpr int LW3_ROW = 2 * LW_NGPT + LW3_REC;           // words per layer row: depths, fractions, record
+constexpr int LW3_HEAD = 96;                             // words before the first row (the head record)
+static_assert(LW3_ROW % 4 == 0 && LW_NGPT % 4 == 0 && LW3_HEAD % 4 == 0, "16-byte pieces");
 // layer record k (1..nlay)
 constexpr int R_PKLAY = 0;      // [16] pklay[k]
 constexpr int R_PKLEVU = 16;    // [16] pklev[k]
@@ -48,7 +47,7 @@ constexpr int R_LSTU = 65;      // int lstu[k]
 constexpr int R_LSTD = 66;      // int lstd[k]
 constexpr int R_FACD = 67;      // [6] downward factors at k - 1: clr1 cld1 cmb1 cmb2 clr2 cld2
 constexpr int R_FACU = 73;      // [6] upward factors at k + 1, same order
-// head record (k = 0)
+// head record
 constexpr int H_PKLAY0 = 0;     // [16] pklay[0] (surface)
 constexpr int H_SECDIFF = 16;   // [16]
 constexpr int H_SEMISS = 32;    // [16]
@@ -56,11 +55,7 @@ constexpr int H_FP64 = 48;      // int: 1 when the column is to be solved in flo
 
 constexpr float LW3_THIN = LW_THIN;   // hPa: a cloudy layer thinner than this sends the column to float64
 
-__host__ __device__ constexpr int64_t lw3_rec_floats(int nlay) { return ((((int64_t)nlay + 1) * LW3_REC + 31) / 32) * 32; }
-__host__ __device__ constexpr int64_t lw3_block_floats(int nlay)
-{
-    return (int64_t)2 * nlay * LW3_GSTRIDE + lw3_rec_floats(nlay);
-}
+__host__ __device__ constexpr int64_t lw3_block_floats(int nlay) { return (LW3_HEAD + (int64_t)nlay * LW3_ROW + 31) / 32 * 32; }
 
 // Optics CTA: 9 warps, 3 CTAs per SM (27 warps, at most 72 registers a thread, no spills).  The CTAs per SM set
 // how many columns share an SM's L1 for the table gathers, and more than 3 cost more than they gain; more warps
@@ -86,20 +81,18 @@ __global__ void __launch_bounds__(LW3_OPT_THREADS, LW3_OPT_MINB) lw3_optics_kern
         return;
     }
     float* blk = scr + (int64_t)blockIdx.x * lw3_block_floats(nlay);
-    float* tgo = blk;
-    float* fro = blk + (size_t)nlay * LW3_GSTRIDE;
+    float* row = blk + LW3_HEAD;
     lw_setup_core<float, LW3_OPT_THREADS>(s, a, col, tid, [&](int g, int k0, float tg, float fr) {
-        tgo[k0 * LW3_GSTRIDE + g] = tg;
-        fro[k0 * LW3_GSTRIDE + g] = fr;
+        row[k0 * LW3_ROW + g] = tg;
+        row[k0 * LW3_ROW + LW_NGPT + g] = fr;
     });
-    float* aux = blk + (size_t)2 * nlay * LW3_GSTRIDE;
+    float* aux = row + 2 * LW_NGPT;                // layer k's record at aux + (k - 1) LW3_ROW
     for (int i = tid; i < nlay * 64; i += LW3_OPT_THREADS) {
         const int k = 1 + (i >> 6), w = i & 63, b = w & 15;
-        float* r = aux + (size_t)k * LW3_REC;
-        r[w] = w < 16 ? s.pklay[k][b] : w < 32 ? s.pklev[k][b] : w < 48 ? s.pklev[k - 1][b] : s.taucld[b][k - 1];
+        aux[(k - 1) * LW3_ROW + w] = w < 16 ? s.pklay[k][b] : w < 32 ? s.pklev[k][b] : w < 48 ? s.pklev[k - 1][b] : s.taucld[b][k - 1];
     }
     for (int k = 1 + tid; k <= nlay; k += LW3_OPT_THREADS) {
-        float* r = aux + (size_t)k * LW3_REC;
+        float* r = aux + (k - 1) * LW3_ROW;
         r[R_CLDFRC] = s.cldfrc[k];
         r[R_LSTU] = __int_as_float(s.lstu[k]);
         r[R_LSTD] = __int_as_float(s.lstd[k]);
@@ -108,18 +101,17 @@ __global__ void __launch_bounds__(LW3_OPT_THREADS, LW3_OPT_MINB) lw3_optics_kern
         const float fu[6] = {s.facclr1u[k + 1], s.faccld1u[k + 1], s.faccmb1u[k + 1], s.faccmb2u[k + 1],
                              s.facclr2u[k + 1], s.faccld2u[k + 1]};
         for (int f = 0; f < 6; ++f) { r[R_FACD + f] = fd[f]; r[R_FACU + f] = fu[f]; }
-        r[LW3_REC - 1] = 0.0f;
     }
     if (tid < 16) {
-        aux[H_PKLAY0 + tid] = s.pklay[0][tid];
-        aux[H_SECDIFF + tid] = s.secdiff[tid];
-        aux[H_SEMISS + tid] = s.semiss[tid];
+        blk[H_PKLAY0 + tid] = s.pklay[0][tid];
+        blk[H_SECDIFF + tid] = s.secdiff[tid];
+        blk[H_SEMISS + tid] = s.semiss[tid];
     }
     if (tid == 0) {
         int fp64 = 0;
         for (int k0 = 0; k0 < nlay; ++k0)
             fp64 |= s.delp[k0] < LW3_THIN && s.cldfrc[k0 + 1] > 1.0e-6f;
-        aux[H_FP64] = __int_as_float(fp64);
+        blk[H_FP64] = __int_as_float(fp64);
         if (fp64) fp64list[1 + atomicAdd(fp64list, 1)] = blockIdx.x;    // the chunk's list for lw3_fp64_kernel
     }
 }
@@ -137,128 +129,139 @@ __global__ void __launch_bounds__(LW_THREADS) lw3_fp64_kernel(const __grid_const
     }
 }
 
-// Layer k (1-based, surface first) terms of one g-point (lw2_terms arithmetic), in float or float64.
-template <class R>
-__device__ __forceinline__ LwTerms<R> lw3_terms(const LwLut<R>& lut, R taug, R plfrac, R blay, R plev_u, R plev_d,
-                                                R taucld, R sdif, bool cloudy)
+// The entry of rtrnmr's transmittance / Planck-fraction tables for optical depth od: position 10^4 od / (bpade + od) +
+// 1/2, its integer part taken by adding 2^23 rounded down (entry number in the sum's low bits; clamped, so a NaN depth
+// reads the last entry).  lut[i] = {exp, tfn}, one 8-byte load.  The quotient takes a Newton step: a depth's rounding
+// decides which of two entries, 3e-4 apart, it gets.
+constexpr float LW3_TWO23 = 8388608.0f;
+template <class V>
+__device__ __forceinline__ V lw3_pos(V od)
 {
-    const R bpade = (R)1.0f / (R)0.278f, tblint = (R)10000, rec_6 = (R)0.166667f, c06 = (R)0.06f;
-    LwTerms<R> t;
-    R odepth = fmaxR((R)0, sdif * taug);
-    R atrgas, gasfac;
-    if (odepth <= c06) {
-        atrgas = odepth - (R)0.5f * odepth * odepth;
-        t.trng = (R)1 - atrgas;
-        gasfac = rec_6 * odepth;
-    } else {
-        const R tblind = odepth / (bpade + odepth);
-        const int it = (int)(tblint * tblind + (R)0.5f);
-        t.trng = ldt(lut.ex + it); atrgas = (R)1 - t.trng; gasfac = ldt(lut.tfn + it); odepth = ldt(lut.tau + it);
-    }
-    const R dplnku = plev_u - blay;
-    const R dplnkd = plev_d - blay;
-    t.gassrcd = plfrac * (blay + dplnkd * gasfac) * atrgas;
-    t.gassrcu = plfrac * (blay + dplnku * gasfac) * atrgas;
-    t.atrg = atrgas;
-    t.trnt = 1; t.totsrcd = 0; t.totsrcu = 0; t.atrt = 0;
-    if (cloudy) {
-        const R odtot = odepth + sdif * taucld;
-        R totfac, atrtot;
-        if (odtot < c06) {
-            totfac = rec_6 * odtot; atrtot = odtot - (R)0.5f * odtot * odtot; t.trnt = (R)1 - atrtot;
-        } else {
-            const R tblind = odtot / (bpade + odtot);
-            const int it = (int)(tblint * tblind + (R)0.5f);
-            totfac = ldt(lut.tfn + it); t.trnt = ldt(lut.ex + it); atrtot = (R)1 - t.trnt;
-        }
-        t.totsrcd = plfrac * (blay + dplnkd * totfac) * atrtot;
-        t.totsrcu = plfrac * (blay + dplnku * totfac) * atrtot;
-        t.atrt = atrtot;
-    }
-    return t;
+    const V d = od + vset<V>(1.0f / 0.278f);
+    return f2_add_rm(fma2(quot2(od, d, rcp2(d)), vset<V>(10000.0f), vset<V>(0.5f)), vset<V>(LW3_TWO23));
+}
+__device__ __forceinline__ float2 lw3_entry(const float2* lut, float pr)
+{
+    return lut[min(__float_as_uint(pr) - 0x4b000000u, 10000u)];
+}
+__device__ __forceinline__ void lw3_lookup(const float2* lut, F2 pr, F2& ex, F2& tfn)
+{
+    const float2 a = lw3_entry(lut, pr.x), b = lw3_entry(lut, pr.y);
+    ex = F2{a.x, b.x};
+    tfn = F2{a.y, b.y};
+}
+__device__ __forceinline__ void lw3_lookup(const float2* lut, float pr, float& ex, float& tfn)
+{
+    const float2 a = lw3_entry(lut, pr);
+    ex = a.x;
+    tfn = a.y;
+}
+// The optical depth of table entry it (lw_lut's tau: bpade it / (10^4 - it), 1e10 for the last).
+template <class V>
+__device__ __forceinline__ V lw3_entry_tau(V it)
+{
+    const V d = vset<V>(10000.0f) - it, t = quot2(it, d, rcp2(d)) * vset<V>(1.0f / 0.278f);
+    return sel2(le2(d, 0.0f), vset<V>(1.0e10f), t);
 }
 
-// One layer of one g-point's sweep in arithmetic R on the float state (radtot, radclr and, with the
-// max-random overlap, totrad / clrrad / rad): the recurrences of rtrnmr, rtrnmc and rtrn (OVR, the
-// LW_OVR_* transfer).  Returns the total-sky radiance change across the layer formed directly -- source -
-// radiance x absorptance, per overlap part -- so it keeps its relative precision however small it is beside
-// the radiance.  f = the layer's six max-random overlap factors (clr1 cld1 cmb1 cmb2 clr2 cld2), x = sdif x
-// cloud optical depth.  rtrnmc is rtrn with a cloud fraction of 1 in its cloudy sub-columns.
-template <class R, int OVR>
-__device__ __forceinline__ R lw3_step(float& rtot, float& rclr, float& trad, float& crad, float& radv,
-                                      const LwTerms<R>& t, bool down, bool cl, bool lst, R clfr, const float* f, R x)
+// One layer of one g-point, or of a pair of neighbouring ones (V = float, F2; a pair shares its band), in one direction:
+// the terms (phys_rrtm_lw_rtrnmr_body.cuh:130-190; branch-free, so that the g-points' table loads are all in flight
+// together) and the recurrences of rtrnmr, rtrnmc and rtrn (OVR, the LW_OVR_* transfer) on the state.
+// Returns the total-sky radiance change across the layer formed directly -- source - radiance x absorptance, per
+// overlap part -- so it keeps its relative precision however small it is beside the radiance; incc = the clear-sky one.
+template <class V>
+struct Lw3State {
+    V tot, clr, trad, crad, rad;   // radtot, radclr and, with the max-random overlap, totrad, clrrad, rad
+};
+struct Lw3Layer {                  // what a layer's g-points share (uniform over the warp)
+    float clfr;
+    bool lst;
+    float f[6];                    // the six max-random overlap factors clr1 cld1 cmb1 cmb2 clr2 cld2
+};
+template <int OVR, class V, class M>
+__device__ __forceinline__ V lw3_step(Lw3State<V>& s, const float2* lut, V taug, V plfrac, float blay, float plev, float tcb,
+                                      float sdif, bool cl, M bit, const Lw3Layer& L, V& incc)
 {
-    const R src = down ? t.gassrcd : t.gassrcu, tsrc = down ? t.totsrcd : t.totsrcu;
-    const R prev = (R)rtot;
-    R inc;
-    if (OVR != LW_OVR_MAXRAN) {
-        if (cl) {
-            const R cf = OVR == LW_OVR_MCICA ? (R)1 : clfr;
-            const R efclrfr = (R)1 - ((R)1 - rexp(-x)) * cf;
-            const R S = src + cf * (tsrc - src);
-            rtot = (float)(prev * t.trng * efclrfr + S);
-            const R cabs = -expm1(-x) * cf;        // 1 - efclrfr without the cancellation
-            inc = S - prev * (t.atrg + cabs - t.atrg * cabs);
-        } else {
-            rtot = (float)(prev * t.trng + src);
-            inc = src - prev * t.atrg;
-        }
-        rclr = (float)((R)rclr * t.trng + src);
+    const float rec_6 = 0.166667f, c06 = 0.06f;
+    const float dpl = plev - blay;
+    const V od0 = max2(taug * vset<V>(sdif), 0.0f);
+    const V pr = lw3_pos(od0);
+    V ex, tfn;
+    lw3_lookup(lut, pr, ex, tfn);
+    const auto thin = le2(od0, c06);
+    const V one = vset<V>(1.0f);
+    const V a1 = nma2(od0 * vset<V>(0.5f), od0, od0);
+    const V atr = sel2(thin, a1, one - ex), trn = sel2(thin, one - a1, ex);
+    const V gf = sel2(thin, od0 * vset<V>(rec_6), tfn);
+    const V src = (plfrac * fma2(vset<V>(dpl), gf, vset<V>(blay))) * atr;
+    const V prev = s.tot, pclr = s.clr;
+    V inc = nma2(prev, atr, src);
+    incc = nma2(pclr, atr, src);
+    s.clr = fma2(pclr, trn, src);
+    if (OVR == LW_OVR_MAXRAN && L.lst) {
+        s.trad = prev * vset<V>(L.clfr);
+        s.crad = prev - s.trad;
+        s.rad = vset<V>(0.0f);
+    }
+    if (!cl) {                     // no cloud in the layer (McICA: in none of the warp's sub-columns)
+        s.tot = fma2(prev, trn, src);
         return inc;
     }
-    R tt = trad, cc = crad, r = radv;
-    if (lst) { tt = clfr * prev; cc = prev - tt; r = 0; }
-    if (cl) {
-        const R tp = tt, cp = cc;
-        tt = tt * t.trnt + clfr * tsrc;
-        cc = cc * t.trng + ((R)1 - clfr) * src;
-        rtot = (float)(tt + cc);
-        rclr = (float)((R)rclr * t.trng + src);
-        const R radmod = r * ((R)f[0] * t.trng + (R)f[1] * t.trnt) - (R)f[2] * src + (R)f[3] * tsrc;
-        r = -radmod + (R)f[4] * (cc + radmod) - (R)f[5] * (tt - radmod);
-        tt = tt + r;
-        cc = cc - r;
-        inc = (clfr * tsrc + ((R)1 - clfr) * src) - (tp * t.atrt + cp * t.atrg);
+    // the cloudy part: gas (its table entry's depth) plus cloud
+    const float x = sdif * tcb;
+    const V ot = fma2(vset<V>(sdif), vset<V>(tcb), sel2(thin, od0, lw3_entry_tau(pr - vset<V>(LW3_TWO23))));
+    const V pc = lw3_pos(ot);
+    V exc, tfc;
+    lw3_lookup(lut, pc, exc, tfc);
+    const auto thinc = lt2(ot, c06);
+    const V a2 = nma2(ot * vset<V>(0.5f), ot, ot);
+    const V att = sel2(thinc, a2, one - exc), tft = sel2(thinc, ot * vset<V>(rec_6), tfc);
+    const V tsrc = (plfrac * fma2(vset<V>(dpl), tft, vset<V>(blay))) * att;
+    if (OVR == LW_OVR_MAXRAN) {
+        const V trt = sel2(thinc, one - a2, exc);
+        const V cs = tsrc * vset<V>(L.clfr), gs = src * vset<V>(1.0f - L.clfr);
+        inc = (cs + gs) - fma2(s.trad, att, s.crad * atr);
+        const V tt = fma2(s.trad, trt, cs), cc = fma2(s.crad, trn, gs);
+        s.tot = tt + cc;
+        const V rm = fma2(s.rad, fma2(vset<V>(L.f[0]), trn, trt * vset<V>(L.f[1])),
+                          nma2(vset<V>(L.f[2]), src, tsrc * vset<V>(L.f[3])));
+        const V r = fma2(vset<V>(L.f[4]), cc + rm, nma2(vset<V>(L.f[5]), tt - rm, vset<V>(0.0f) - rm));
+        s.rad = r;
+        s.trad = tt + r;
+        s.crad = cc - r;
     } else {
-        rtot = (float)(prev * t.trng + src);
-        rclr = (float)((R)rclr * t.trng + src);
-        inc = src - prev * t.atrg;
+        // rtrnmc is rtrn with a cloud fraction of 1 in its cloudy sub-columns
+        const float cf = OVR == LW_OVR_MCICA ? 1.0f : L.clfr;
+        const V S = fma2(vset<V>(cf), tsrc - src, src);
+        const float ef = 1.0f - (1.0f - rexp(-x)) * cf;
+        const float ca = -expm1(-x) * cf;                     // 1 - ef without the cancellation
+        const V ctot = fma2(prev * trn, vset<V>(ef), S);
+        const V cinc = nma2(prev, nma2(atr, vset<V>(ca), atr + vset<V>(ca)), S);
+        if (OVR == LW_OVR_MCICA) {
+            s.tot = sel2(bit, ctot, fma2(prev, trn, src));
+            inc = sel2(bit, cinc, inc);
+        } else {
+            s.tot = ctot;
+            inc = cinc;
+        }
     }
-    trad = (float)tt;
-    crad = (float)cc;
-    radv = (float)r;
     return inc;
 }
 
-// The sweeps stream each layer's taug row, fracs row and record (400 floats) through a LW3_NSTAGE-stage ring in
-// shared memory with asynchronous 16-byte copies (cp.async.cg: L2 to shared, no L1 allocation), LW3_NSTAGE - 1
-// layers ahead of the one being computed, so the scratch's DRAM latency overlaps the arithmetic.
-constexpr int LW3_STAGE = 2 * LW3_GSTRIDE + LW3_REC;   // floats per stage
+// The sweeps stream each layer's row (1,440 bytes) through a LW3_NSTAGE-stage ring in shared memory with asynchronous
+// 16-byte copies (cp.async.cg: L2 to shared, no L1 allocation), LW3_NSTAGE - 1 layers ahead of the one being computed,
+// so the scratch's DRAM latency overlaps the arithmetic.  (Bulk copies completed on an mbarrier per slot were 2.5 %
+// slower: lane 0 alone issues and waits, where the 16-byte copies spread over the warp.)
 constexpr int LW3_NSTAGE = 3;
-// LW3_TMA fills the ring by bulk copies instead (cp.async.bulk: the layer's taug row, fracs row and record, three
-// contiguous runs) that lane 0 issues and an mbarrier per slot completes.  Same bits; measured 2.5 % slower over
-// the LW on the B200 (lane 0 alone issues and waits, where the 16-byte copies spread over the warp), so off.
-constexpr bool LW3_TMA = false;
-constexpr int LW3_WAIT_LIMIT = 1 << 16;   // mbarrier tests before a wait gives up (flags RAD_DEV_TIMEOUT)
 
-__device__ __forceinline__ void lw3_cp16(float* dst, const float* src)
+__device__ __forceinline__ void lw3_stage_row(float* st, const float* row, int lane)
 {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
-// Layer k's rows and record into stage st: 100 16-byte pieces over the warp's lanes, one commit group.
-// Sources are 16-byte aligned: rows start at multiples of 640 bytes and records at multiples of 320 bytes
-// of a 128-byte aligned block.
-__device__ __forceinline__ void lw3_stage_layer(float* st, const float* tg, const float* fr, const float* aux, int k,
-                                                int lane)
-{
-    for (int c = lane; c < LW3_STAGE / 4; c += 32) {
-        const float* src = c < 40   ? tg + (size_t)(k - 1) * LW3_GSTRIDE + 4 * c
-                           : c < 80 ? fr + (size_t)(k - 1) * LW3_GSTRIDE + 4 * (c - 40)
-                                    : aux + (size_t)k * LW3_REC + 4 * (c - 80);
-        lw3_cp16(st + 4 * c, src);
-    }
+    const unsigned d = (unsigned)__cvta_generic_to_shared(st) + 16u * (unsigned)lane;
+    const float* src = row + 4 * lane;
+#pragma unroll
+    for (int c = 0; c < LW3_ROW / 4; c += 32)
+        if (c + 32 <= LW3_ROW / 4 || c + lane < LW3_ROW / 4)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * c), "l"(src + 4 * c) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
@@ -269,18 +272,20 @@ __device__ __forceinline__ void lw3_stage_layer(float* st, const float* tg, cons
 constexpr int LW3_PGQ = 8;
 __host__ __device__ constexpr int64_t lw3_pg_floats(int nlay) { return (int64_t)(nlay + 1) * LW3_PGQ * LW_NGPT; }
 
-template <int OVR, bool DIAG = false>
-__global__ void __launch_bounds__(LW3_SWEEP_WARPS * 32) lw3_sweep_kernel(const __grid_constant__ LwBatch bt, int64_t c0,
-                                                                         int64_t nc, const float* __restrict__ scr,
-                                                                         LwLut<float> lut, int* err,
-                                                                         float* __restrict__ pg = nullptr)
+// Shared memory of a sweep CTA: the {exp, tfn} table, then per warp its ring and its level sums.
+struct Lw3Warp {
+    float ring[LW3_NSTAGE][LW3_ROW];
+    double fup[NLAY_MAX + 1], fdn[NLAY_MAX + 1];
+};
+constexpr int LW3_LUT_N = 10001;
+constexpr size_t LW3_LUT_BYTES = (LW3_LUT_N * sizeof(float2) + 15) / 16 * 16;
+constexpr size_t lw3_sweep_smem() { return LW3_LUT_BYTES + LW3_SWEEP_WARPS * sizeof(Lw3Warp); }
+
+// The two sweeps of the chunk's column lc by one warp.
+template <int OVR, bool DIAG>
+__device__ __forceinline__ void lw3_sweep_column(Lw3Warp& W, const float2* lut, const LwBatch& bt, int64_t c0, int64_t lc,
+                                                 const float* __restrict__ scr, float* __restrict__ pg, int lane)
 {
-    __shared__ double fup[LW3_SWEEP_WARPS][NLAY_MAX + 1], fdn[LW3_SWEEP_WARPS][NLAY_MAX + 1];
-    __shared__ __align__(16) float ring[LW3_SWEEP_WARPS][LW3_NSTAGE][LW3_STAGE];
-    __shared__ __align__(8) uint64_t rbar[LW3_SWEEP_WARPS][LW3_NSTAGE];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t lc = (int64_t)blockIdx.x * LW3_SWEEP_WARPS + warp;
-    if (lc >= nc) return;
     const int64_t gc = c0 + lc;
     const int rq = bt.find(gc);
     const LwIn& a = bt.req[rq];
@@ -288,165 +293,118 @@ __global__ void __launch_bounds__(LW3_SWEEP_WARPS * 32) lw3_sweep_kernel(const _
     const int64_t col = gc - bt.off[rq];
     const int64_t N = a.ncol;
     if (nlay > NLAY_MAX || col >= N) return;    // the optics kernel has flagged a bad nlay
-    const float* blk = scr + lc * lw3_block_floats(nlay);
-    const float* tg = blk;
-    const float* fr = blk + (size_t)nlay * LW3_GSTRIDE;
-    const float* aux = blk + (size_t)2 * nlay * LW3_GSTRIDE;
+    const float* head = scr + lc * lw3_block_floats(nlay);
+    const float* rows = head + LW3_HEAD;
     if (DIAG) pg += lc * lw3_pg_floats(nlay);
     // sweep steps: s = 0 .. nlay-1 downward (layer nlay - s), s = nlay .. 2 nlay - 1 upward (layer s - nlay + 1)
     const int nstep = 2 * nlay;
     auto layer_of = [&](int st) { return st < nlay ? nlay - st : st - nlay + 1; };
-    if (LW3_TMA) {
-        if (lane == 0) {
-            for (int q = 0; q < LW3_NSTAGE; ++q) mbar_init(&rbar[warp][q], 1);
-            mbar_init_fence();
-        }
-        __syncwarp();
-    }
-    // layer k's rows and record into ring slot q: lane 0 issues three bulk copies completed on the slot's barrier,
-    // after the warp's reads of the slot's previous layer (ordered by the __syncwarp and the proxy fence)
-    auto stage = [&](int q, int k) {
-        if (LW3_TMA) {
-            __syncwarp();
-            if (lane == 0) {
-                async_proxy_fence();
-                uint64_t* b = &rbar[warp][q];
-                float* dst = ring[warp][q];
-                mbar_expect_tx(b, (unsigned)(LW3_STAGE * sizeof(float)));
-                bulk_copy_g2s(dst, tg + (size_t)(k - 1) * LW3_GSTRIDE, LW3_GSTRIDE * sizeof(float), b);
-                bulk_copy_g2s(dst + LW3_GSTRIDE, fr + (size_t)(k - 1) * LW3_GSTRIDE, LW3_GSTRIDE * sizeof(float), b);
-                bulk_copy_g2s(dst + 2 * LW3_GSTRIDE, aux + (size_t)k * LW3_REC, LW3_REC * sizeof(float), b);
-            }
-        } else {
-            lw3_stage_layer(ring[warp][q], tg, fr, aux, k, lane);
-        }
-    };
 #pragma unroll
-    for (int q = 0; q < LW3_NSTAGE - 1; ++q) stage(q, layer_of(q));
+    for (int q = 0; q < LW3_NSTAGE - 1; ++q) lw3_stage_row(W.ring[q], rows + (size_t)(layer_of(q) - 1) * LW3_ROW, lane);
     const float eps = 1.0e-6f;
-    int gi[LW3_SLOTS], band[LW3_SLOTS];
-    float sdif[LW3_SLOTS];
-    bool val[LW3_SLOTS];
-#pragma unroll
-    for (int j = 0; j < LW3_SLOTS; ++j) {
-        const int g = lane + 32 * j;
-        val[j] = g < LW_NGPT;
-        gi[j] = val[j] ? g : LW_NGPT - 1;
-        int b = 0;
-        while (gi[j] >= c_lw_ns[b + 1]) ++b;
-        band[j] = b;
-        sdif[j] = __ldg(aux + H_SECDIFF + b);
-    }
-    auto mask_bit = [&](int j, int k) {   // McICA: word j holds g-points 32 j .. 32 j + 31
-        return ((__ldg(a.mask + ((size_t)j * nlay + (k - 1)) * N + col) >> lane) & 1u) != 0;
-    };
-    float radtot[LW3_SLOTS], radclr[LW3_SLOTS], trad[LW3_SLOTS], crad[LW3_SLOTS], rad[LW3_SLOTS];
-    // One layer of the sweep for the warp's g-points; returns the warp's float64 sum of the radiance changes.
-    auto layer = [&](const float* stg, int k, bool down) -> double {
-        const float* tgr = stg;
-        const float* frr = stg + LW3_GSTRIDE;
-        const float* r = stg + 2 * LW3_GSTRIDE;
-        const float clfr = r[R_CLDFRC];
-        const bool lst = __float_as_int(r[down ? R_LSTD : R_LSTU]) != 0;
-        float f[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) f[i] = r[(down ? R_FACD : R_FACU) + i];
-        double sum = 0.0;
-#pragma unroll
-        for (int j = 0; j < LW3_SLOTS; ++j) {
-            const int g = gi[j], b = band[j];
-            const bool cl = OVR == LW_OVR_MCICA ? mask_bit(j, k) : clfr >= eps;
-            const float tcb = r[R_TAUCLD + b];
-            const LwTerms<float> t = lw3_terms<float>(lut, tgr[g], frr[g], r[R_PKLAY + b], r[R_PKLEVU + b],
-                                                      r[R_PKLEVD + b], tcb, sdif[j], cl);
-            const float pclr = radclr[j];
-            const float inc = lw3_step<float, OVR>(radtot[j], radclr[j], trad[j], crad[j], rad[j], t, down, cl, lst,
-                                                  clfr, f, sdif[j] * tcb);
-            if (val[j]) sum += (double)inc;
-            if (DIAG && val[j]) {
-                // the clear-sky change across the layer, formed directly like inc; the radiances at the level
-                // the step ends on (k - 1 going down, k going up)
-                const float incc = (down ? t.gassrcd : t.gassrcu) - pclr * t.atrg;
-                float* p = pg + (size_t)k * LW3_PGQ * LW_NGPT + g;
-                p[(down ? 5 : 4) * LW_NGPT] = inc;
-                p[(down ? 7 : 6) * LW_NGPT] = incc;
-                float* q = pg + (size_t)(down ? k - 1 : k) * LW3_PGQ * LW_NGPT + g;
-                q[(down ? 1 : 0) * LW_NGPT] = radtot[j];
-                q[(down ? 3 : 2) * LW_NGPT] = radclr[j];
-            }
+    const bool val = lane < LW_NGPT - 128;                          // the single g-point is real
+    const int g0 = 2 * lane, g1 = 64 + 2 * lane, g2 = val ? 128 + lane : LW_NGPT - 1;
+    const int b0 = c_lw_band[g0], b1 = c_lw_band[g1], b2 = c_lw_band[g2];
+    const float sd0 = __ldg(head + H_SECDIFF + b0), sd1 = __ldg(head + H_SECDIFF + b1), sd2 = __ldg(head + H_SECDIFF + b2);
+    Lw3State<F2> s0, s1;
+    Lw3State<float> s2;
+    s0.tot = s0.clr = s0.trad = s0.crad = s0.rad = f2(0.0f);
+    s1 = s0;
+    s2.tot = s2.clr = s2.trad = s2.crad = s2.rad = 0.0f;
+    auto ld2 = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return F2{v.x, v.y}; };
+    auto st2 = [](float* p, F2 v) { *reinterpret_cast<float2*>(p) = make_float2(v.x, v.y); };
+    // One layer of the sweep for the lane's g-points; returns the warp's float64 sum of the radiance changes.
+    auto layer = [&](const float* st, int k, bool down) -> double {
+        const float* r = st + 2 * LW_NGPT;
+        const float* pl = r + (down ? R_PKLEVD : R_PKLEVU);
+        Lw3Layer L;
+        L.clfr = r[R_CLDFRC];
+        L.lst = __float_as_int(r[down ? R_LSTD : R_LSTU]) != 0;
+        bool cl = L.clfr >= eps;
+        B2 m0{false, false}, m1{false, false};
+        bool m2 = false;
+        if (OVR == LW_OVR_MCICA) {   // word j of a layer holds g-points 32 j .. 32 j + 31
+            auto word = [&](int j) { return __ldg(a.mask + ((size_t)j * nlay + (k - 1)) * N + col); };
+            const unsigned w0 = word(g0 >> 5) >> (g0 & 31), w1 = word(g1 >> 5) >> (g1 & 31), w2 = word(g2 >> 5) >> (g2 & 31);
+            m0 = B2{(w0 & 1u) != 0, (w0 & 2u) != 0};
+            m1 = B2{(w1 & 1u) != 0, (w1 & 2u) != 0};
+            m2 = (w2 & 1u) != 0;
+            cl = __any_sync(0xffffffffu, m0.x || m0.y || m1.x || m1.y || m2);
         }
+        if (OVR == LW_OVR_MAXRAN && cl) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) L.f[i] = r[(down ? R_FACD : R_FACU) + i];
+        }
+        F2 c0_, c1_;
+        float c2_;
+        const F2 i0 = lw3_step<OVR>(s0, lut, ld2(st + g0), ld2(st + LW_NGPT + g0), r[R_PKLAY + b0], pl[b0], r[R_TAUCLD + b0],
+                                    sd0, cl, m0, L, c0_);
+        const F2 i1 = lw3_step<OVR>(s1, lut, ld2(st + g1), ld2(st + LW_NGPT + g1), r[R_PKLAY + b1], pl[b1], r[R_TAUCLD + b1],
+                                    sd1, cl, m1, L, c1_);
+        const float i2 = lw3_step<OVR>(s2, lut, st[g2], st[LW_NGPT + g2], r[R_PKLAY + b2], pl[b2], r[R_TAUCLD + b2], sd2, cl,
+                                       m2, L, c2_);
+        if (DIAG) {
+            // the radiance changes across the layer; the radiances at the level the step ends on (k - 1 going down, k
+            // going up)
+            float* p = pg + ((size_t)k * LW3_PGQ + (down ? 5 : 4)) * LW_NGPT;
+            float* q = pg + ((size_t)(down ? k - 1 : k) * LW3_PGQ + (down ? 1 : 0)) * LW_NGPT;
+            st2(p + g0, i0); st2(p + 2 * LW_NGPT + g0, c0_); st2(q + g0, s0.tot); st2(q + 2 * LW_NGPT + g0, s0.clr);
+            st2(p + g1, i1); st2(p + 2 * LW_NGPT + g1, c1_); st2(q + g1, s1.tot); st2(q + 2 * LW_NGPT + g1, s1.clr);
+            if (val) { p[g2] = i2; p[2 * LW_NGPT + g2] = c2_; q[g2] = s2.tot; q[2 * LW_NGPT + g2] = s2.clr; }
+        }
+        const double sum = ((double)i0.x + (double)i0.y) + ((double)i1.x + (double)i1.y) + (val ? (double)i2 : 0.0);
         return warp_sum(sum);
     };
+    // float64 sum over the column's g-points of one field of the states
+    auto total = [&](F2 x, F2 y, float z) {
+        return warp_sum(((double)x.x + (double)x.y) + ((double)y.x + (double)y.y) + (val ? (double)z : 0.0));
+    };
     // ---- the sweeps: downward, the surface, upward; layer s + LW3_NSTAGE - 1 is copied in while layer s computes
-#pragma unroll
-    for (int j = 0; j < LW3_SLOTS; ++j) { radtot[j] = 0; radclr[j] = 0; trad[j] = 0; crad[j] = 0; rad[j] = 0; }
     double s_tu = 0, s_cu = 0, s_td = 0, s_cd = 0;
+    int slot = 0;                                                    // st % LW3_NSTAGE
     for (int st = 0; st < nstep; ++st) {
-        if (st + LW3_NSTAGE - 1 < nstep)
-            stage((st + LW3_NSTAGE - 1) % LW3_NSTAGE, layer_of(st + LW3_NSTAGE - 1));
-        else if (!LW3_TMA)
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        if (LW3_TMA) {
-            // slot st % LW3_NSTAGE completes its (st / LW3_NSTAGE)-th phase when the step's copies have landed
-            // lane 0 waits for the phase; the __syncwarp then orders the landed data for the other lanes
-            bool ok = true;
-            if (lane == 0)
-                ok = mbar_wait_bounded(&rbar[warp][st % LW3_NSTAGE], (unsigned)((st / LW3_NSTAGE) & 1), LW3_WAIT_LIMIT);
-            __syncwarp();
-            if (!__shfl_sync(0xffffffffu, ok, 0)) {
-                // a copy did not land: flag it, wait (bounded) for the copies still in flight, stop this column
-                if (lane == 0) atomicExch(err, RAD_DEV_TIMEOUT);
-                if (lane == 0)
-                    for (int s2 = st + 1; s2 < min(nstep, st + LW3_NSTAGE); ++s2)
-                        mbar_wait_bounded(&rbar[warp][s2 % LW3_NSTAGE], (unsigned)((s2 / LW3_NSTAGE) & 1),
-                                          LW3_WAIT_LIMIT);
-                return;
-            }
-        } else {
-            // this lane's copies of step st have landed (the LW3_NSTAGE - 1 later groups may still be in flight)
-            asm volatile("cp.async.wait_group %0;" ::"n"(LW3_NSTAGE - 1) : "memory");
-            __syncwarp();                                        // ... and every lane's
-        }
+        const int nx = st + LW3_NSTAGE - 1, nslot = slot == 0 ? LW3_NSTAGE - 1 : slot - 1;
+        if (nx < nstep) lw3_stage_row(W.ring[nslot], rows + (size_t)(layer_of(nx) - 1) * LW3_ROW, lane);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        // this lane's copies of step st have landed (the LW3_NSTAGE - 1 later groups may still be in flight)
+        asm volatile("cp.async.wait_group %0;" ::"n"(LW3_NSTAGE - 1) : "memory");
+        __syncwarp();                                            // ... and every lane's
         if (st == nlay) {
             // surface: emission and reflection
-#pragma unroll
-            for (int j = 0; j < LW3_SLOTS; ++j) {
-                const int b = band[j];
-                const float semi = __ldg(aux + H_SEMISS + b);
-                const float reflct = 1.0f - semi;
-                const float rad0 = semi * __ldg(fr + gi[j]) * __ldg(aux + H_PKLAY0 + b);
-                const float rtd = radtot[j], rcd = radclr[j];
-                radtot[j] = rad0 + reflct * rtd;
-                radclr[j] = rad0 + reflct * rcd;
-                if (DIAG && val[j]) {   // the upward radiances leaving the surface; nothing comes down at the top
-                    pg[(size_t)0 * LW_NGPT + gi[j]] = radtot[j];
-                    pg[(size_t)2 * LW_NGPT + gi[j]] = radclr[j];
-                    pg[((size_t)nlay * LW3_PGQ + 1) * LW_NGPT + gi[j]] = 0.0f;
-                    pg[((size_t)nlay * LW3_PGQ + 3) * LW_NGPT + gi[j]] = 0.0f;
-                }
-                if (val[j]) {
-                    s_tu += (double)radtot[j]; s_cu += (double)radclr[j];
-                    s_td += (double)rtd; s_cd += (double)rcd;
-                }
-                trad[j] = 0; crad[j] = 0; rad[j] = 0;
+            s_td = total(s0.tot, s1.tot, s2.tot);
+            s_cd = total(s0.clr, s1.clr, s2.clr);
+            auto surface = [&](auto& s, auto fr, int b) {
+                using V = decltype(s.tot);
+                const float semi = __ldg(head + H_SEMISS + b);
+                const V rad0 = fr * vset<V>(semi) * vset<V>(__ldg(head + H_PKLAY0 + b));
+                s.tot = fma2(vset<V>(1.0f - semi), s.tot, rad0);
+                s.clr = fma2(vset<V>(1.0f - semi), s.clr, rad0);
+                s.trad = s.crad = s.rad = vset<V>(0.0f);
+            };
+            const float* fr = rows + LW_NGPT;
+            surface(s0, F2{__ldg(fr + g0), __ldg(fr + g0 + 1)}, b0);
+            surface(s1, F2{__ldg(fr + g1), __ldg(fr + g1 + 1)}, b1);
+            surface(s2, __ldg(fr + g2), b2);
+            s_tu = total(s0.tot, s1.tot, s2.tot);
+            s_cu = total(s0.clr, s1.clr, s2.clr);
+            if (DIAG) {   // the upward radiances leaving the surface; nothing comes down at the top
+                float* top = pg + ((size_t)nlay * LW3_PGQ + 1) * LW_NGPT;
+                st2(pg + g0, s0.tot); st2(pg + 2 * LW_NGPT + g0, s0.clr); st2(top + g0, f2(0.0f)); st2(top + 2 * LW_NGPT + g0, f2(0.0f));
+                st2(pg + g1, s1.tot); st2(pg + 2 * LW_NGPT + g1, s1.clr); st2(top + g1, f2(0.0f)); st2(top + 2 * LW_NGPT + g1, f2(0.0f));
+                if (val) { pg[g2] = s2.tot; pg[2 * LW_NGPT + g2] = s2.clr; top[g2] = 0.0f; top[2 * LW_NGPT + g2] = 0.0f; }
             }
-            s_tu = warp_sum(s_tu); s_cu = warp_sum(s_cu); s_td = warp_sum(s_td); s_cd = warp_sum(s_cd);
         }
         const bool down = st < nlay;
         const int k = layer_of(st);
-        const double v = layer(ring[warp][st % LW3_NSTAGE], k, down);
+        const double v = layer(W.ring[slot], k, down);
         if (lane == 0) {
-            if (down) fdn[warp][k - 1] = v;           // D(k-1) - D(k), summed over g
-            else fup[warp][k] = v;                    // U(k) - U(k-1), summed over g
+            if (down) W.fdn[k - 1] = v;           // D(k-1) - D(k), summed over g
+            else W.fup[k] = v;                    // U(k) - U(k-1), summed over g
         }
+        slot = slot == LW3_NSTAGE - 1 ? 0 : slot + 1;
         __syncwarp();                                 // the stage is free for the copy two steps on
     }
-    double t_tu = 0, t_cu = 0;
-#pragma unroll
-    for (int j = 0; j < LW3_SLOTS; ++j)
-        if (val[j]) { t_tu += (double)radtot[j]; t_cu += (double)radclr[j]; }
-    t_tu = warp_sum(t_tu);
-    t_cu = warp_sum(t_cu);
+    const double t_tu = total(s0.tot, s1.tot, s2.tot), t_cu = total(s0.clr, s1.clr, s2.clr);
     __syncwarp();
     // ---- outputs: fluxes x flxfac; heating rates from the per-layer net-flux changes (rtrnmr post)
     const double pi = 3.14159265358979323846;
@@ -454,7 +412,7 @@ __global__ void __launch_bounds__(LW3_SWEEP_WARPS * 32) lw3_sweep_kernel(const _
     const double heatfac = 9.80665 * 1.0e-2 / 1.0046e3;
     for (int k = lane; k < nlay; k += 32) {
         // layer k + 1 (surface first): (U(k) - D(k)) - (U(k+1) - D(k+1)) = -(dU + dD)
-        const double du = fup[warp][k + 1], dd = fdn[warp][k];
+        const double du = W.fup[k + 1], dd = W.fdn[k];
         const int kin = nlay - 1 - k;
         const double dl = (double)__ldg(a.plvl + (size_t)(kin + 1) * N + col) - (double)__ldg(a.plvl + (size_t)kin * N + col);
         a.htlw[(size_t)kin * N + col] = (float)(-(du + dd) * flxfac * (heatfac / dl));
@@ -467,6 +425,28 @@ __global__ void __launch_bounds__(LW3_SWEEP_WARPS * 32) lw3_sweep_kernel(const _
         a.sfcflw[2 * N + col] = (float)(s_td * flxfac);
         a.sfcflw[3 * N + col] = (float)(s_cd * flxfac);
     }
+}
+
+// One warp per column, warps striding over the chunk's columns (grid: at most one CTA per SM).  Lane l carries the
+// pairs of g-points 2 l, 2 l + 1 and 64 + 2 l, 65 + 2 l, in packed arithmetic, and lanes 0..11 the single g-points
+// 128..139.  Bound: the random 8-byte table gathers and issue slots.  Measured per 131,072 columns of 61 layers: 12.4 ms
+// with one g-point per slot, branches and three 4-byte gathers per entry; branch-free pairs with the table through L1
+// 9.4 ms at 5 CTAs of 4 warps per SM (10.0 at 6, 7.05 at 4: the more warps, the less L1 is left for the 80 KB table);
+// with the table in shared memory 6.2 ms at 16 warps per SM (12: 6.7, 14: 7.1, 20: 9.4, 24: 9.6 -- from 20 on the
+// registers no longer hold two pairs' chains side by side), 6.5 ms with the Newton step on the entry positions.
+template <int OVR, bool DIAG = false>
+__global__ void __launch_bounds__(LW3_SWEEP_WARPS * 32, 1)
+lw3_sweep_kernel(const __grid_constant__ LwBatch bt, int64_t c0, int64_t nc, const float* __restrict__ scr,
+                 const float2* __restrict__ lutg, float* __restrict__ pg0 = nullptr)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* lut = reinterpret_cast<float2*>(smem_raw);
+    for (int i = threadIdx.x; i < LW3_LUT_N; i += LW3_SWEEP_WARPS * 32) lut[i] = __ldg(lutg + i);
+    __syncthreads();                                // the only barrier: the warps go their own ways from here
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    Lw3Warp& W = reinterpret_cast<Lw3Warp*>(smem_raw + LW3_LUT_BYTES)[warp];
+    for (int64_t lc = blockIdx.x + (int64_t)gridDim.x * warp; lc < nc; lc += (int64_t)gridDim.x * LW3_SWEEP_WARPS)
+        lw3_sweep_column<OVR, DIAG>(W, lut, bt, c0, lc, scr, pg0, lane);
 }
 
 // lwrad's optional outputs of a chunk from the DIAG sweeps' profiles: one warp per column, lane q < 16 band q
