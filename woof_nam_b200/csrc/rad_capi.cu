@@ -163,9 +163,14 @@ __global__ void k_laytrop(const __grid_constant__ DayBatch b, int nlay, const in
     const int r = b.find(g);
     const DayReq& q = b.req[r];
     const int64_t c = g - b.off[r];
-    int l = nlay;
-    for (int k0 = 0; k0 < nlay; ++k0)
-        if (log((double)q.plyr[(size_t)(nlay - 1 - k0) * q.ncol + c]) > (double)4.56f) l = k0 + 1;
+    // the last layer that qualifies is the first from the top; ln is monotone and exp(4.56) = 95.58, so only a pressure
+    // near the bound takes the logarithm
+    int l = 0;
+    for (int k = 0; k < nlay && l == 0; ++k) {
+        const float p = __ldg(q.plyr + (size_t)k * q.ncol + c);
+        if (p > 95.0f && (p > 96.0f || log((double)p) > (double)4.56f)) l = nlay - k;
+    }
+    if (l == 0) l = nlay;
     lt[d] = l;
     const int w = (int)(c / q.wc);
     const int dw0 = pos[b.off[r] + (int64_t)w * q.wc];
@@ -255,10 +260,15 @@ int ensure_scratch(RadHandle* h, int64_t n)
 {
     if (n + 1 > h->cap) {
         const int64_t cap = n + 1 + (n >> 3);
-        for (int** p : {&h->d_flag, &h->d_pos, &h->d_daycol, &h->d_lt, &h->d_k8, &h->d_kw})
-            if (*p) cudaFree(*p);
-        for (int** p : {&h->d_flag, &h->d_pos, &h->d_daycol, &h->d_lt, &h->d_k8, &h->d_kw})
-            RAD_CUDA(h, cudaMalloc((void**)p, (size_t)cap * sizeof(int)));
+        if (h->d_flag) cudaFree(h->d_flag);
+        h->d_flag = nullptr;
+        h->cap = 0;
+        // the six arrays in one allocation (256-byte steps), d_flag its start
+        const size_t step = ((size_t)cap * sizeof(int) + 255) / 256 * 256;
+        char* base = nullptr;
+        RAD_CUDA(h, cudaMalloc((void**)&base, 6 * step));
+        int** const part[6] = {&h->d_flag, &h->d_pos, &h->d_daycol, &h->d_lt, &h->d_k8, &h->d_kw};
+        for (int i = 0; i < 6; ++i) *part[i] = (int*)(base + i * step);
         size_t need = 0;
         RAD_CUDA(h, cub::DeviceScan::ExclusiveSum(nullptr, need, h->d_flag, h->d_pos, (int)cap));
         if (need > h->cub_bytes) {
@@ -365,12 +375,12 @@ int ensure_launch_scratch(RadHandle* h, int64_t ntot, int64_t ncmin)
         const int64_t need = std::min(lwc, ntot);
         if (need > h->lw3_cap) {
             if (h->d_lw3) cudaFree(h->d_lw3);
-            if (h->d_lw3list) cudaFree(h->d_lw3list);
             h->d_lw3 = nullptr;
             h->d_lw3list = nullptr;
             h->lw3_cap = 0;
-            RAD_CUDA(h, cudaMalloc((void**)&h->d_lw3, (size_t)need * lw3_block_floats(h->cfg.nlay) * sizeof(float)));
-            RAD_CUDA(h, cudaMalloc((void**)&h->d_lw3list, (size_t)(need + 1) * sizeof(int)));
+            const size_t blocks = (size_t)need * lw3_block_floats(h->cfg.nlay);   // the list follows in the same allocation
+            RAD_CUDA(h, cudaMalloc((void**)&h->d_lw3, blocks * sizeof(float) + (size_t)(need + 1) * sizeof(int)));
+            h->d_lw3list = (int*)(h->d_lw3 + blocks);
             h->lw3_cap = need;
         }
     }
@@ -379,16 +389,16 @@ int ensure_launch_scratch(RadHandle* h, int64_t ntot, int64_t ncmin)
         RAD_CUDA(h, cudaMalloc((void**)&h->d_swrt, (size_t)sw2_rt_bytes(h->nsm)));
     if (swc > 0 && (h->cfg.parts & RAD_PART_SW) && std::min(swc, ntot) > h->sw4_cap) {
         if (h->d_sw4) cudaFree(h->d_sw4);
-        if (h->d_sw4img) cudaFree(h->d_sw4img);
-        if (h->d_sw4item) cudaFree(h->d_sw4item);
         h->d_sw4 = nullptr;
         h->d_sw4img = nullptr;
         h->d_sw4item = nullptr;
         h->sw4_cap = 0;
         const int64_t need = std::min(swc, ntot);
-        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4, (size_t)need * sw4_block_bytes(h->cfg.nlay)));
-        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4img, (size_t)need * sw4_image_bytes(true)));
-        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4item, (size_t)sw4_item_bytes(h->cfg.nlay, need)));
+        // blocks, images and the work list in one allocation
+        const size_t blocks = (size_t)need * sw4_block_bytes(h->cfg.nlay), images = (size_t)need * sw4_image_bytes(true);
+        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4, blocks + images + (size_t)sw4_item_bytes(h->cfg.nlay, need)));
+        h->d_sw4img = (int4*)(h->d_sw4 + blocks);
+        h->d_sw4item = (int*)(h->d_sw4 + blocks + images);
         h->sw4_cap = need;
     }
     if (h->cfg.route == RAD_ROUTE_MCICA && ntot * h->cfg.nlay > h->mask_cap) {
@@ -718,12 +728,12 @@ int rad_create(const RadConfig* cfg, RadHandle** out)
     h->cfg = *cfg;
     h->device = device;
     h->nsm = nsm;
-    if (cudaMalloc((void**)&h->d_err, sizeof(int)) != cudaSuccess ||
-        cudaMalloc((void**)&h->d_nday, sizeof(int)) != cudaSuccess) {
+    if (cudaMalloc((void**)&h->d_err, 2 * sizeof(int)) != cudaSuccess) {
         delete h;
         return fail(nullptr, RAD_E_NOMEM, "rad_create: device allocation failed");
     }
-    cudaMemset(h->d_err, 0, sizeof(int));
+    h->d_nday = h->d_err + 1;
+    cudaMemset(h->d_err, 0, 2 * sizeof(int));
     *out = h;
     return RAD_OK;
 }
@@ -772,7 +782,9 @@ int rad_load_tables(RadHandle* h, const void* blob, size_t nbytes)
     if (chi64.size() != 59 * 7) return fail(h, RAD_E_TABLES, "rad_load_tables: missing lw05_chi_mls_f64");
     std::vector<int64_t> off(T_COUNT);
     int64_t tot = 0;
-    for (int t = 0; t < T_COUNT; ++t) { off[t] = tot; tot += (int64_t)vals[t].size(); }
+    // each table on a 128-byte line (32 floats), so that a row of 8 or 16 g-points spans no more lines than it must and
+    // a pair of g-points is one aligned 8-byte load
+    for (int t = 0; t < T_COUNT; ++t) { off[t] = tot; tot += ((int64_t)vals[t].size() + 31) / 32 * 32; }
     std::vector<float> hf(tot);
     std::vector<double> hd(tot);
     for (int t = 0; t < T_COUNT; ++t)
@@ -789,18 +801,30 @@ int rad_load_tables(RadHandle* h, const void* blob, size_t nbytes)
     k.b5_rpb = (float)(chi64[42 * 7 + 2] / chi64[42 * 7 + 1]);
     k.b5_rma = (float)(chi64[6 * 7 + 0] / chi64[6 * 7 + 1]);
     k.b15_r = (float)chi[0 * 7 + 3] / (float)chi[0 * 7 + 1];
-    std::vector<float> lwf, swf;
-    std::vector<double> lwd, swd;
-    lw_lut(lwf); lw_lut(lwd); sw_lut(swf); sw_lut(swd);
-    lwf.resize(LW_LUT2, 0.0f);                   // then the sweeps' copy, {exp, tfn} per entry
-    for (int i = 0; i <= 10000; ++i) {
-        lwf.push_back(lwf[i]);
-        lwf.push_back(lwf[10001 + i]);
-    }
     int rc;
-    if ((rc = upload(h, &h->d_lwf, lwf)) || (rc = upload(h, &h->d_lwd, lwd)) || (rc = upload(h, &h->d_swf, swf)) ||
-        (rc = upload(h, &h->d_swd, swd)))
-        return rc;
+    // the float64 LW and SW LUTs, then the float32 ones and the LW sweeps' {exp, tfn} pairs, in one buffer (d_lwd its
+    // start); the same for every handle, formed once
+    static const std::vector<double> lut = [] {
+        std::vector<float> lwf, swf;
+        std::vector<double> v, swd;
+        lw_lut(lwf); lw_lut(v); sw_lut(swf); sw_lut(swd);
+        lwf.resize(LW_LUT2, 0.0f);
+        for (int i = 0; i <= 10000; ++i) {
+            lwf.push_back(lwf[i]);
+            lwf.push_back(lwf[10001 + i]);
+        }
+        v.insert(v.end(), swd.begin(), swd.end());
+        lwf.insert(lwf.end(), swf.begin(), swf.end());
+        if (lwf.size() & 1) lwf.push_back(0.0f);
+        const size_t n = v.size();
+        v.resize(n + lwf.size() / 2);
+        std::memcpy(v.data() + n, lwf.data(), lwf.size() * sizeof(float));
+        return v;
+    }();
+    if ((rc = upload(h, &h->d_lwd, lut))) return rc;
+    h->d_swd = h->d_lwd + 3 * 10001;
+    h->d_lwf = (float*)(h->d_swd + 10001);
+    h->d_swf = h->d_lwf + LW_LUT2 + 2 * 10001;
     // The k-tables are read through __constant__ pointers, which are per device, not per handle: the
     // first load on a device uploads them and sets the constants; they stay until the process exits and
     // every later handle on that device shares them.  A later blob with different content is refused, so a
@@ -819,7 +843,9 @@ int rad_load_tables(RadHandle* h, const void* blob, size_t nbytes)
             return rc;
         }
         RAD_CUDA(h, cudaMemcpyToSymbol(c_toff, off.data(), T_COUNT * sizeof(int64_t)));
-        RAD_CUDA(h, cudaMemcpyToSymbol(c_tf, &tf, sizeof(float*)));
+        std::vector<const float*> tfp(T_COUNT);
+        for (int t = 0; t < T_COUNT; ++t) tfp[t] = tf + off[t];
+        RAD_CUDA(h, cudaMemcpyToSymbol(c_tfp, tfp.data(), T_COUNT * sizeof(float*)));
         RAD_CUDA(h, cudaMemcpyToSymbol(c_td, &td, sizeof(double*)));
         RAD_CUDA(h, cudaMemcpyToSymbol(c_lwk, &k, sizeof(k)));
         uint32_t pw[624];
@@ -1523,11 +1549,11 @@ void rad_destroy(RadHandle* h)
 {
     if (!h) return;
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
-    for (void* p : {(void*)h->d_lwf, (void*)h->d_swf, (void*)h->d_lwd, (void*)h->d_swd,
-                    (void*)h->d_err, (void*)h->d_flag, (void*)h->d_pos, (void*)h->d_daycol, (void*)h->d_lt,
-                    (void*)h->d_k8, (void*)h->d_kw, (void*)h->d_cmin, (void*)h->d_nday, h->d_cub, (void*)h->d_lwm,
-                    (void*)h->d_swm, (void*)h->d_lw3, (void*)h->d_lw3list, (void*)h->d_swrt, (void*)h->d_sw4, (void*)h->d_sw4img, (void*)h->d_sw4item, (void*)h->d_lwpg, (void*)h->d_swpg, (void*)h->d_aerf,
-                    (void*)h->d_aeri})
+    // one pointer per allocation (d_lwd holds all four LUTs, d_flag the day-list arrays, d_lw3 its list, d_sw4 the images
+    // and the work list, d_err the day count)
+    for (void* p : {(void*)h->d_lwd, (void*)h->d_err, (void*)h->d_flag, (void*)h->d_cmin, h->d_cub, (void*)h->d_lwm,
+                    (void*)h->d_swm, (void*)h->d_lw3, (void*)h->d_swrt, (void*)h->d_sw4, (void*)h->d_lwpg, (void*)h->d_swpg,
+                    (void*)h->d_aerf, (void*)h->d_aeri})
         if (p) cudaFree(p);
     delete h;
 }

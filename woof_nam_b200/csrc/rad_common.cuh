@@ -5,6 +5,7 @@
 // float32 copy and one instantiated for double reads the float64 copy, with the same index arithmetic.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 #include "rad_tabids.h"
 
@@ -14,7 +15,7 @@ constexpr int NLAY_MAX = 64;        // per-thread sweep arrays are sized for thi
 constexpr int LW_NGPT = 140, SW_NGPT = 112;
 
 __constant__ int64_t c_toff[T_COUNT];
-__constant__ const float* c_tf;
+__constant__ const float* c_tfp[T_COUNT];     // each float32 table's address
 __constant__ const double* c_td;
 
 // Scalars the reference's wrappers compute on the host (band 4, 5 and 15 reference ratios), float32.
@@ -24,7 +25,7 @@ struct LwHostConsts {
 __constant__ LwHostConsts c_lwk;
 
 template <class R> __device__ __forceinline__ const R* tab(int id);
-template <> __device__ __forceinline__ const float* tab<float>(int id) { return c_tf + c_toff[id]; }
+template <> __device__ __forceinline__ const float* tab<float>(int id) { return c_tfp[id]; }
 template <> __device__ __forceinline__ const double* tab<double>(int id) { return c_td + c_toff[id]; }
 
 template <class R> __device__ __forceinline__ R ldt(const R* p) { return __ldg(p); }
@@ -59,13 +60,51 @@ __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes)
                  : "memory");
 }
 
-// t(ig, ind) + frac * (t(ig, ind+1) - t(ig, ind)) for a [ind][g] table, 1-based ind.
-template <class R>
-__device__ __forceinline__ R interp(const R* t, int ng, int ind, int ig, R frac)
+// Two neighbouring g-points' values under plain scalar arithmetic (a factor they share stays one register, where the
+// packed operations would need it twice): the gas optics of a pair read both from each k-table row with one 8-byte load
+// and share every index, interpolation weight and shared-memory read.  V = P2 runs a pair (first g-point even; every
+// band's first g-point, its g-point count and every table's offset are even), V = R one g-point.
+struct P2 {
+    float x, y;
+};
+__device__ __forceinline__ P2 operator+(P2 a, P2 b) { return P2{a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ P2 operator-(P2 a, P2 b) { return P2{a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ P2 operator*(float a, P2 b) { return P2{a * b.x, a * b.y}; }
+__device__ __forceinline__ P2 operator*(P2 b, float a) { return P2{b.x * a, b.y * a}; }
+__device__ __forceinline__ P2 operator+(P2 a, float b) { return P2{a.x + b, a.y + b}; }
+template <class V, class R>
+__device__ __forceinline__ V ldv(const R* p)
 {
-    const R a = ldt(t + ((ind - 1) * ng + ig)), b = ldt(t + (ind * ng + ig));   // tables < 2^31 entries
+    if constexpr (sizeof(V) == sizeof(R)) {
+        return __ldg(p);
+    } else {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+        return V{v.x, v.y};
+    }
+}
+template <class V, class R>
+__device__ __forceinline__ V vall(R a)
+{
+    if constexpr (std::is_same<V, P2>::value) return P2{a, a};
+    else return (V)a;
+}
+// v scaled by f of its g-point number
+template <class V, class F>
+__device__ __forceinline__ V vscale(V v, int ig, F f)
+{
+    if constexpr (std::is_same<V, P2>::value) return P2{v.x * f(ig), v.y * f(ig + 1)};
+    else return v * (V)f(ig);
+}
+
+// t(ig, ind) + frac * (t(ig, ind+1) - t(ig, ind)) for a [ind][g] table, 1-based ind.
+template <class V, class R>
+__device__ __forceinline__ V interpv(const R* t, int ng, int ind, int ig, R frac)
+{
+    const V a = ldv<V>(t + ((ind - 1) * ng + ig)), b = ldv<V>(t + (ind * ng + ig));   // tables < 2^31 entries
     return a + frac * (b - a);
 }
+template <class R>
+__device__ __forceinline__ R interp(const R* t, int ng, int ind, int ig, R frac) { return interpv<R>(t, ng, ind, ig, frac); }
 
 // Warp sum of a double, lanes 0..31 (result valid in lane 0); a fixed tree, so bit-reproducible.
 __device__ __forceinline__ double warp_sum(double v)
@@ -119,14 +158,15 @@ __device__ __forceinline__ void for_each_band_pair(const int* ns, int nbands, in
 // task (a quarter of them in the 12-g-point bands): 274 tasks instead of 304 for the LW's 140 g-points on 61
 // layers, 222 instead of 245 for the SW's 112 (LW -5 %, SW -2 % on the B200, same bits).  i / ng is
 // (i * ceil(2^16 / ng)) >> 16, exact for ng <= 16 and i < 2^12 (checked exhaustively).
-template <class F>
+// G = 2: a pair counts as one (the lane's first g-point is even).
+template <int G = 1, class F>
 __device__ __forceinline__ void for_each_band_flat(const int* ns, int nbands, int nlay, int* next, int lane, F f)
 {
     int b = 0, t0 = 0;   // band of the current task and the index of its first task
     int g0, ng, np, nt, mg;
     auto shape = [&](int bb) {
         g0 = ns[bb];
-        ng = ns[bb + 1] - g0;
+        ng = (ns[bb + 1] - g0) / G;
         np = ng * nlay;
         nt = (np + 31) >> 5;
         mg = (65536 + ng - 1) / ng;
@@ -146,7 +186,7 @@ __device__ __forceinline__ void for_each_band_flat(const int* ns, int nbands, in
         const int i = ((t - t0) << 5) + lane;
         if (i < np) {
             const int k0 = (i * mg) >> 16;
-            f(g0 + (i - k0 * ng), k0, b);
+            f(g0 + G * (i - k0 * ng), k0, b);
         }
     }
 }

@@ -48,6 +48,8 @@ struct LwSetup {
     R adjc[LW_NADJ][NLAY_MAX];
     R chir[LW_NCHIR];
     static constexpr bool kKeys = false;      // LwSetupK: the species keys of bands 3, 4, 5, 7, 9 are precomputed
+    using Gas = R;                            // the gas optics' g-points per task (LwSetupK: a pair)
+    static constexpr int kGas = 1;
 };
 
 // The species keys of one binary-species band at one layer (the specparm / js / fs statements of taugb03, 04, 05,
@@ -64,6 +66,8 @@ constexpr int LW_NKEYB = 5;
 template <class R>
 struct LwSetupK : LwSetup<R> {
     static constexpr bool kKeys = true;
+    using Gas = P2;
+    static constexpr int kGas = 2;
     LwKey<R> key[LW_NKEYB][NLAY_MAX];
 };
 
@@ -120,18 +124,18 @@ template <class R> __device__ __forceinline__ int br_joint(R a, R b)
     if (a > (R)0.875f && b > (R)0.875f) return 1;
     return 2;
 }
-template <class R>
-__device__ __forceinline__ R major12(const R* absa, int ng, int ig, R sc, const Sel<R>& s0, R f00, R f10, R sc1,
+template <class V, class R>
+__device__ __forceinline__ V major12(const R* absa, int ng, int ig, R sc, const Sel<R>& s0, R f00, R f10, R sc1,
                                      const Sel<R>& s1, R f01, R f11)
 {
-    auto A = [&](int id) { return ldt(absa + ((id - 1) * ng + ig)); };
+    auto A = [&](int id) { return ldv<V>(absa + ((id - 1) * ng + ig)); };
     const R fac000 = s0.fk0 * f00, fac100 = s0.fk1 * f00, fac200 = s0.fk2 * f00;
     const R fac010 = s0.fk0 * f10, fac110 = s0.fk1 * f10, fac210 = s0.fk2 * f10;
     const R fac001 = s1.fk0 * f01, fac101 = s1.fk1 * f01, fac201 = s1.fk2 * f01;
     const R fac011 = s1.fk0 * f11, fac111 = s1.fk1 * f11, fac211 = s1.fk2 * f11;
-    const R t0 = sc * (fac000 * A(s0.id[0]) + fac010 * A(s0.id[1]) + fac100 * A(s0.id[2]) + fac110 * A(s0.id[3]) +
+    const V t0 = sc * (fac000 * A(s0.id[0]) + fac010 * A(s0.id[1]) + fac100 * A(s0.id[2]) + fac110 * A(s0.id[3]) +
                        fac200 * A(s0.id[4]) + fac210 * A(s0.id[5]));
-    const R t1 = sc1 * (fac001 * A(s1.id[0]) + fac011 * A(s1.id[1]) + fac101 * A(s1.id[2]) + fac111 * A(s1.id[3]) +
+    const V t1 = sc1 * (fac001 * A(s1.id[0]) + fac011 * A(s1.id[1]) + fac101 * A(s1.id[2]) + fac111 * A(s1.id[3]) +
                         fac201 * A(s1.id[4]) + fac211 * A(s1.id[5]));
     return t0 + t1;
 }
@@ -141,12 +145,12 @@ __device__ __forceinline__ R adjcol(R col, R temp, R thr, R off, R ex)   // the 
     const R rat = col / temp;
     return rat > thr ? (off + rpow(rat - off, ex)) * temp : col;
 }
-template <class R>
-__device__ __forceinline__ R minor2d(const R* t, int nj, int ng, int j, R fj, int m, R fm, int ig)  // t[m][j][g]
+template <class V, class R>
+__device__ __forceinline__ V minor2d(const R* t, int nj, int ng, int j, R fj, int m, R fm, int ig)  // t[m][j][g]
 {
-    auto K = [&](int jj, int mm) { return ldt(t + (((mm - 1) * nj + (jj - 1)) * ng + ig)); };
-    const R m1 = K(j, m) + fj * (K(j + 1, m) - K(j, m));
-    const R m2 = K(j, m + 1) + fj * (K(j + 1, m + 1) - K(j, m + 1));
+    auto K = [&](int jj, int mm) { return ldv<V>(t + (((mm - 1) * nj + (jj - 1)) * ng + ig)); };
+    const V m1 = K(j, m) + fj * (K(j + 1, m) - K(j, m));
+    const V m2 = K(j, m + 1) + fj * (K(j + 1, m + 1) - K(j, m + 1));
     return m1 + fm * (m2 - m1);
 }
 
@@ -154,8 +158,8 @@ __device__ __forceinline__ R minor2d(const R* t, int nj, int ng, int j, R fj, in
 // Gas optical depth and Planck fraction of LW g-point g (0..139) at layer k0: the band kernels of the
 // reference restated per (g, layer).  Statement order follows each band's reference kernel.  Table offsets
 // are formed in 32-bit integers (every table is far below 2^31 entries), one wide add per address.
-template <class R, class S>
-__device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = -1)
+template <class R, class V, class S>
+__device__ void lw_gas(const S& s, int g, int k0, V& tg, V& fr, int band_of_g = -1)
 {
     const bool low = s.lower[k0];
     const int jpk = s.jp[k0], jtk = s.jt[k0], jt1k = s.jt1[k0];
@@ -164,7 +168,7 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
     const R sfac = s.selffac[k0], sfr = s.selffrac[k0], ffac = s.forfac[k0], ffr = s.forfrac[k0],
             mf = s.minorfrac[k0];
     auto A4 = [&](const R* t, int ng, int ig, int i0, int i1) {
-        auto a = [&](int id) { return ldt(t + ((id - 1) * ng + ig)); };
+        auto a = [&](int id) { return ldv<V>(t + ((id - 1) * ng + ig)); };
         return f00 * a(i0) + f10 * a(i0 + 1) + f01 * a(i1) + f11 * a(i1 + 1);
     };
     // the precomputed species keys of band slot q at this layer (LwSetupK only)
@@ -188,33 +192,33 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
     case 1: {
         const int NG = 10;
         const R pp = s.pavel[k0], scalen2 = s.colbrd[k0] * s.scaleminorn2[k0], col = s.colamt[0][k0];
-        const R taufor = ffac * interp(tab<R>(T_LW01_FORREF), NG, indf, ig, ffr);
+        const V taufor = ffac * interpv<V>(tab<R>(T_LW01_FORREF), NG, indf, ig, ffr);
         if (low) {
             const R corradj = pp < (R)250 ? (R)1 - (R)0.15f * ((R)250 - pp) / (R)154.4f : (R)1;
-            const R tauself = sfac * interp(tab<R>(T_LW01_SELFREF), NG, inds, ig, sfr);
-            const R taun2 = scalen2 * interp(tab<R>(T_LW01_KA_MN2), NG, indm, ig, mf);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW01_SELFREF), NG, inds, ig, sfr);
+            const V taun2 = scalen2 * interpv<V>(tab<R>(T_LW01_KA_MN2), NG, indm, ig, mf);
             tg = corradj * (col * A4(tab<R>(T_LW01_ABSA), NG, ig, ind0l, ind1l) + tauself + taufor + taun2);
-            fr = ldt(tab<R>(T_LW01_FRACREFA) + ig);
+            fr = ldv<V>(tab<R>(T_LW01_FRACREFA) + ig);
         } else {
             const R corradj = (R)1 - (R)0.15f * (pp / (R)95.6f);
-            const R taun2 = scalen2 * interp(tab<R>(T_LW01_KB_MN2), NG, indm, ig, mf);
+            const V taun2 = scalen2 * interpv<V>(tab<R>(T_LW01_KB_MN2), NG, indm, ig, mf);
             tg = corradj * (col * A4(tab<R>(T_LW01_ABSB), NG, ig, ind0u, ind1u) + taufor + taun2);
-            fr = ldt(tab<R>(T_LW01_FRACREFB) + ig);
+            fr = ldv<V>(tab<R>(T_LW01_FRACREFB) + ig);
         }
         break;
     }
     case 2: {
         const int NG = 12;
         const R col = s.colamt[0][k0];
-        const R taufor = ffac * interp(tab<R>(T_LW02_FORREF), NG, indf, ig, ffr);
+        const V taufor = ffac * interpv<V>(tab<R>(T_LW02_FORREF), NG, indf, ig, ffr);
         if (low) {
             const R corradj = (R)1 - (R)0.05f * (s.pavel[k0] - (R)100) / (R)900;
-            const R tauself = sfac * interp(tab<R>(T_LW02_SELFREF), NG, inds, ig, sfr);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW02_SELFREF), NG, inds, ig, sfr);
             tg = corradj * (col * A4(tab<R>(T_LW02_ABSA), NG, ig, ind0l, ind1l) + tauself + taufor);
-            fr = ldt(tab<R>(T_LW02_FRACREFA) + ig);
+            fr = ldv<V>(tab<R>(T_LW02_FRACREFA) + ig);
         } else {
             tg = col * A4(tab<R>(T_LW02_ABSB), NG, ig, ind0u, ind1u) + taufor;
-            fr = ldt(tab<R>(T_LW02_FRACREFB) + ig);
+            fr = ldv<V>(tab<R>(T_LW02_FRACREFB) + ig);
         }
         break;
     }
@@ -246,12 +250,12 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             }
             const Sel<R> s0 = sel_branch(br0, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br1, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(b3 ? T_LW03_SELFREF : T_LW04_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(b3 ? T_LW03_FORREF : T_LW04_FORREF), NG, indf, ig, ffr);
-            const R major = major12(absa, NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11);
-            if (b3) tg = major + tauself + taufor + adjn2o * minor2d(tab<R>(T_LW03_KA_MN2O), 9, NG, jmn, fmn, indm, mf, ig);
+            const V tauself = sfac * interpv<V>(tab<R>(b3 ? T_LW03_SELFREF : T_LW04_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(b3 ? T_LW03_FORREF : T_LW04_FORREF), NG, indf, ig, ffr);
+            const V major = major12<V>(absa, NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11);
+            if (b3) tg = major + tauself + taufor + adjn2o * minor2d<V>(tab<R>(T_LW03_KA_MN2O), 9, NG, jmn, fmn, indm, mf, ig);
             else tg = major + tauself + taufor;
-            fr = interp(fa, NG, jpl, ig, fpl);
+            fr = interpv<V>(fa, NG, jpl, ig, fpl);
         } else {
             R sc, sc1, fs, fs1, fmn = 0, fpl;
             int js, js1, jmn = 1, jpl;
@@ -273,26 +277,24 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             const int ind1 = ((jpk - 12) * 5 + (jt1k - 1)) * 5 + js1;
             const R fac000 = ((R)1 - fs) * f00, fac010 = ((R)1 - fs) * f10, fac100 = fs * f00, fac110 = fs * f10;
             const R fac001 = ((R)1 - fs1) * f01, fac011 = ((R)1 - fs1) * f11, fac101 = fs1 * f01, fac111 = fs1 * f11;
-            auto B = [&](int id) { return ldt(absb + ((id - 1) * NG + ig)); };
-            const R t0 = sc * (fac000 * B(ind0) + fac010 * B(ind0 + 5) + fac100 * B(ind0 + 1) + fac110 * B(ind0 + 6));
-            const R t1 = sc1 * (fac001 * B(ind1) + fac011 * B(ind1 + 5) + fac101 * B(ind1 + 1) + fac111 * B(ind1 + 6));
+            auto B = [&](int id) { return ldv<V>(absb + ((id - 1) * NG + ig)); };
+            const V t0 = sc * (fac000 * B(ind0) + fac010 * B(ind0 + 5) + fac100 * B(ind0 + 1) + fac110 * B(ind0 + 6));
+            const V t1 = sc1 * (fac001 * B(ind1) + fac011 * B(ind1 + 5) + fac101 * B(ind1 + 1) + fac111 * B(ind1 + 6));
             if (b3) {
-                const R taufor = ffac * interp(tab<R>(T_LW03_FORREF), NG, indf, ig, ffr);
-                tg = t0 + t1 + taufor + adjn2o * minor2d(tab<R>(T_LW03_KB_MN2O), 5, NG, jmn, fmn, indm, mf, ig);
+                const V taufor = ffac * interpv<V>(tab<R>(T_LW03_FORREF), NG, indf, ig, ffr);
+                tg = t0 + t1 + taufor + adjn2o * minor2d<V>(tab<R>(T_LW03_KB_MN2O), 5, NG, jmn, fmn, indm, mf, ig);
             } else {
                 tg = t0 + t1;
-                if (ig >= 7) {
-                    const float adj[7] = {0.92f, 0.88f, 1.07f, 1.1f, 0.99f, 0.88f, 0.943f};
-                    tg = tg * (R)adj[ig - 7];
-                }
+                tg = vscale(tg, ig, [](int i) { return i == 7 ? 0.92f : i == 8 ? 0.88f : i == 9 ? 1.07f : i == 10 ? 1.1f : i == 11 ? 0.99f : i == 12 ? 0.88f : i == 13 ? 0.943f : 1.0f; });
             }
-            fr = interp(fb, NG, jpl, ig, fpl);
+            fr = interpv<V>(fb, NG, jpl, ig, fpl);
         }
         break;
     }
     case 5: {
         const int NG = 16;
-        const R wxk = s.wx[0][k0], ccl4 = ldt(tab<R>(T_LW05_CCL4) + ig);
+        const R wxk = s.wx[0][k0];
+        const V ccl4 = ldv<V>(tab<R>(T_LW05_CCL4) + ig);
         if (low) {
             R sc, sc1, fs, fs1, fm, fpl;
             int js, js1, jm, jpl, br, br1;
@@ -309,12 +311,12 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             }
             const Sel<R> s0 = sel_branch(br, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(T_LW05_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW05_FORREF), NG, indf, ig, ffr);
-            const R abso3 = minor2d(tab<R>(T_LW05_KA_MO3), 9, NG, jm, fm, indm, mf, ig);
-            tg = major12(tab<R>(T_LW05_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW05_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW05_FORREF), NG, indf, ig, ffr);
+            const V abso3 = minor2d<V>(tab<R>(T_LW05_KA_MO3), 9, NG, jm, fm, indm, mf, ig);
+            tg = major12<V>(tab<R>(T_LW05_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
                  abso3 * s.colamt[2][k0] + wxk * ccl4;
-            fr = interp(tab<R>(T_LW05_FRACREFA), NG, jpl, ig, fpl);
+            fr = interpv<V>(tab<R>(T_LW05_FRACREFA), NG, jpl, ig, fpl);
         } else {
             R sc, sc1, fs, fs1, fpl;
             int js, js1, jpl;
@@ -334,27 +336,27 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             const R fac000 = ((R)1 - fs) * f00, fac010 = ((R)1 - fs) * f10, fac100 = fs * f00, fac110 = fs * f10;
             const R fac001 = ((R)1 - fs1) * f01, fac011 = ((R)1 - fs1) * f11, fac101 = fs1 * f01, fac111 = fs1 * f11;
             const R* absb = tab<R>(T_LW05_ABSB);
-            auto B = [&](int id) { return ldt(absb + ((id - 1) * NG + ig)); };
+            auto B = [&](int id) { return ldv<V>(absb + ((id - 1) * NG + ig)); };
             tg = sc * (fac000 * B(ind0) + fac010 * B(ind0 + 5) + fac100 * B(ind0 + 1) + fac110 * B(ind0 + 6)) +
                  sc1 * (fac001 * B(ind1) + fac011 * B(ind1 + 5) + fac101 * B(ind1 + 1) + fac111 * B(ind1 + 6)) + wxk * ccl4;
-            fr = interp(tab<R>(T_LW05_FRACREFB), NG, jpl, ig, fpl);
+            fr = interpv<V>(tab<R>(T_LW05_FRACREFB), NG, jpl, ig, fpl);
         }
         break;
     }
     case 6: {
         const int NG = 8;
         const R wx2 = s.wx[1][k0], wx3 = s.wx[2][k0];
-        const R xsec = wx2 * ldt(tab<R>(T_LW06_CFC11ADJ) + ig) + wx3 * ldt(tab<R>(T_LW06_CFC12) + ig);
+        const V xsec = wx2 * ldv<V>(tab<R>(T_LW06_CFC11ADJ) + ig) + wx3 * ldv<V>(tab<R>(T_LW06_CFC12) + ig);
         if (low) {
             const R adj = s.adjc[1][k0];
-            const R tauself = sfac * interp(tab<R>(T_LW06_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW06_FORREF), NG, indf, ig, ffr);
-            const R absco2 = interp(tab<R>(T_LW06_KA_MCO2), NG, indm, ig, mf);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW06_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW06_FORREF), NG, indf, ig, ffr);
+            const V absco2 = interpv<V>(tab<R>(T_LW06_KA_MCO2), NG, indm, ig, mf);
             tg = s.colamt[0][k0] * A4(tab<R>(T_LW06_ABSA), NG, ig, ind0l, ind1l) + tauself + taufor + adj * absco2 + xsec;
         } else {
             tg = xsec;
         }
-        fr = ldt(tab<R>(T_LW06_FRACREFA) + ig);
+        fr = ldv<V>(tab<R>(T_LW06_FRACREFA) + ig);
         break;
     }
     case 7: {
@@ -377,42 +379,39 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             const R adj = s.adjc[2][k0];
             const Sel<R> s0 = sel_branch(br, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(T_LW07_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW07_FORREF), NG, indf, ig, ffr);
-            tg = major12(tab<R>(T_LW07_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
-                 adj * minor2d(tab<R>(T_LW07_KA_MCO2), 9, NG, jm, fm, indm, mf, ig);
-            fr = interp(tab<R>(T_LW07_FRACREFA), NG, jpl, ig, fpl);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW07_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW07_FORREF), NG, indf, ig, ffr);
+            tg = major12<V>(tab<R>(T_LW07_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
+                 adj * minor2d<V>(tab<R>(T_LW07_KA_MCO2), 9, NG, jm, fm, indm, mf, ig);
+            fr = interpv<V>(tab<R>(T_LW07_FRACREFA), NG, jpl, ig, fpl);
         } else {
             const R adj = s.adjc[2][k0];
-            const R absco2 = interp(tab<R>(T_LW07_KB_MCO2), NG, indm, ig, mf);
+            const V absco2 = interpv<V>(tab<R>(T_LW07_KB_MCO2), NG, indm, ig, mf);
             tg = c3 * A4(tab<R>(T_LW07_ABSB), NG, ig, ind0u, ind1u) + adj * absco2;
-            if (ig >= 5 && ig <= 10) {
-                const float scl[6] = {0.92f, 0.88f, 1.07f, 1.1f, 0.99f, 0.855f};
-                tg = tg * (R)scl[ig - 5];
-            }
-            fr = ldt(tab<R>(T_LW07_FRACREFB) + ig);
+            tg = vscale(tg, ig, [](int i) { return i == 5 ? 0.92f : i == 6 ? 0.88f : i == 7 ? 1.07f : i == 8 ? 1.1f : i == 9 ? 0.99f : i == 10 ? 0.855f : 1.0f; });
+            fr = ldv<V>(tab<R>(T_LW07_FRACREFB) + ig);
         }
         break;
     }
     case 8: {
         const int NG = 8;
         const R adj = s.adjc[3][k0];
-        const R xsec = s.wx[2][k0] * ldt(tab<R>(T_LW08_CFC12) + ig) + s.wx[3][k0] * ldt(tab<R>(T_LW08_CFC22ADJ) + ig);
+        const V xsec = s.wx[2][k0] * ldv<V>(tab<R>(T_LW08_CFC12) + ig) + s.wx[3][k0] * ldv<V>(tab<R>(T_LW08_CFC22ADJ) + ig);
         if (low) {
-            const R tauself = sfac * interp(tab<R>(T_LW08_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW08_FORREF), NG, indf, ig, ffr);
-            const R absco2 = interp(tab<R>(T_LW08_KA_MCO2), NG, indm, ig, mf);
-            const R abso3 = interp(tab<R>(T_LW08_KA_MO3), NG, indm, ig, mf);
-            const R absn2o = interp(tab<R>(T_LW08_KA_MN2O), NG, indm, ig, mf);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW08_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW08_FORREF), NG, indf, ig, ffr);
+            const V absco2 = interpv<V>(tab<R>(T_LW08_KA_MCO2), NG, indm, ig, mf);
+            const V abso3 = interpv<V>(tab<R>(T_LW08_KA_MO3), NG, indm, ig, mf);
+            const V absn2o = interpv<V>(tab<R>(T_LW08_KA_MN2O), NG, indm, ig, mf);
             tg = s.colamt[0][k0] * A4(tab<R>(T_LW08_ABSA), NG, ig, ind0l, ind1l) + tauself + taufor + adj * absco2 +
                  s.colamt[2][k0] * abso3 + s.colamt[3][k0] * absn2o + xsec;
-            fr = ldt(tab<R>(T_LW08_FRACREFA) + ig);
+            fr = ldv<V>(tab<R>(T_LW08_FRACREFA) + ig);
         } else {
-            const R absco2 = interp(tab<R>(T_LW08_KB_MCO2), NG, indm, ig, mf);
-            const R absn2o = interp(tab<R>(T_LW08_KB_MN2O), NG, indm, ig, mf);
+            const V absco2 = interpv<V>(tab<R>(T_LW08_KB_MCO2), NG, indm, ig, mf);
+            const V absn2o = interpv<V>(tab<R>(T_LW08_KB_MN2O), NG, indm, ig, mf);
             tg = s.colamt[2][k0] * A4(tab<R>(T_LW08_ABSB), NG, ig, ind0u, ind1u) + adj * absco2 +
                  s.colamt[3][k0] * absn2o + xsec;
-            fr = ldt(tab<R>(T_LW08_FRACREFB) + ig);
+            fr = ldv<V>(tab<R>(T_LW08_FRACREFB) + ig);
         }
         break;
     }
@@ -436,14 +435,14 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             }
             const Sel<R> s0 = sel_branch(br, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(T_LW09_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW09_FORREF), NG, indf, ig, ffr);
-            tg = major12(tab<R>(T_LW09_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
-                 adj * minor2d(tab<R>(T_LW09_KA_MN2O), 9, NG, jm, fm, indm, mf, ig);
-            fr = interp(tab<R>(T_LW09_FRACREFA), NG, jpl, ig, fpl);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW09_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW09_FORREF), NG, indf, ig, ffr);
+            tg = major12<V>(tab<R>(T_LW09_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
+                 adj * minor2d<V>(tab<R>(T_LW09_KA_MN2O), 9, NG, jm, fm, indm, mf, ig);
+            fr = interpv<V>(tab<R>(T_LW09_FRACREFA), NG, jpl, ig, fpl);
         } else {
-            tg = c5 * A4(tab<R>(T_LW09_ABSB), NG, ig, ind0u, ind1u) + adj * interp(tab<R>(T_LW09_KB_MN2O), NG, indm, ig, mf);
-            fr = ldt(tab<R>(T_LW09_FRACREFB) + ig);
+            tg = c5 * A4(tab<R>(T_LW09_ABSB), NG, ig, ind0u, ind1u) + adj * interpv<V>(tab<R>(T_LW09_KB_MN2O), NG, indm, ig, mf);
+            fr = ldv<V>(tab<R>(T_LW09_FRACREFB) + ig);
         }
         break;
     }
@@ -461,16 +460,16 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
         const R col = b == 14 ? s.colamt[1][k0] : s.colamt[0][k0];
         const R scaleo2 = s.colamt[5][k0] * s.scaleminor[k0];
         if (low) {
-            const R tauself = sfac * interp(tab<R>(is), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(iff), NG, indf, ig, ffr);
+            const V tauself = sfac * interpv<V>(tab<R>(is), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(iff), NG, indf, ig, ffr);
             tg = col * A4(tab<R>(ia), NG, ig, ind0l, ind1l) + tauself + taufor;
-            if (b == 11) tg = tg + scaleo2 * interp(tab<R>(T_LW11_KA_MO2), NG, indm, ig, mf);
-            fr = ldt(tab<R>(ifa) + ig);
+            if (b == 11) tg = tg + scaleo2 * interpv<V>(tab<R>(T_LW11_KA_MO2), NG, indm, ig, mf);
+            fr = ldv<V>(tab<R>(ifa) + ig);
         } else {
             tg = col * A4(tab<R>(ib_), NG, ig, ind0u, ind1u);
-            if (b != 14) tg = tg + ffac * interp(tab<R>(iff), NG, indf, ig, ffr);
-            if (b == 11) tg = tg + scaleo2 * interp(tab<R>(T_LW11_KB_MO2), NG, indm, ig, mf);
-            fr = ldt(tab<R>(ifb) + ig);
+            if (b != 14) tg = tg + ffac * interpv<V>(tab<R>(iff), NG, indf, ig, ffr);
+            if (b == 11) tg = tg + scaleo2 * interpv<V>(tab<R>(T_LW11_KB_MO2), NG, indm, ig, mf);
+            fr = ldv<V>(tab<R>(ifb) + ig);
         }
         break;
     }
@@ -496,16 +495,16 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             const int br = br_joint(sp, sp1);
             const Sel<R> s0 = sel_branch(br, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(b12 ? T_LW12_SELFREF : T_LW16_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(b12 ? T_LW12_FORREF : T_LW16_FORREF), NG, indf, ig, ffr);
-            tg = major12(tab<R>(b12 ? T_LW12_ABSA : T_LW16_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor;
-            fr = interp(tab<R>(b12 ? T_LW12_FRACREFA : T_LW16_FRACREFA), NG, jpl, ig, fpl);
+            const V tauself = sfac * interpv<V>(tab<R>(b12 ? T_LW12_SELFREF : T_LW16_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(b12 ? T_LW12_FORREF : T_LW16_FORREF), NG, indf, ig, ffr);
+            tg = major12<V>(tab<R>(b12 ? T_LW12_ABSA : T_LW16_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor;
+            fr = interpv<V>(tab<R>(b12 ? T_LW12_FRACREFA : T_LW16_FRACREFA), NG, jpl, ig, fpl);
         } else if (b12) {
-            tg = 0;
-            fr = 0;
+            tg = vall<V>((R)0);
+            fr = vall<V>((R)0);
         } else {
             tg = s.colamt[4][k0] * A4(tab<R>(T_LW16_ABSB), NG, ig, 1, 1);   // nspb(16) = 0: row 1 always
-            fr = ldt(tab<R>(T_LW16_FRACREFB) + ig);
+            fr = ldv<V>(tab<R>(T_LW16_FRACREFB) + ig);
         }
         break;
     }
@@ -525,15 +524,15 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             const int br = br_joint(sp, sp1);
             const Sel<R> s0 = sel_branch(br, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(T_LW13_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW13_FORREF), NG, indf, ig, ffr);
-            tg = major12(tab<R>(T_LW13_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
-                 adj * minor2d(tab<R>(T_LW13_KA_MCO2), 9, NG, jm, fm, indm, mf, ig) +
-                 c7 * minor2d(tab<R>(T_LW13_KA_MCO), 9, NG, jmc, fmc, indm, mf, ig);
-            fr = interp(tab<R>(T_LW13_FRACREFA), NG, jpl, ig, fpl);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW13_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW13_FORREF), NG, indf, ig, ffr);
+            tg = major12<V>(tab<R>(T_LW13_ABSA), NG, ig, sc, s0, f00, f10, sc1, s1, f01, f11) + tauself + taufor +
+                 adj * minor2d<V>(tab<R>(T_LW13_KA_MCO2), 9, NG, jm, fm, indm, mf, ig) +
+                 c7 * minor2d<V>(tab<R>(T_LW13_KA_MCO), 9, NG, jmc, fmc, indm, mf, ig);
+            fr = interpv<V>(tab<R>(T_LW13_FRACREFA), NG, jpl, ig, fpl);
         } else {
-            tg = s.colamt[2][k0] * interp(tab<R>(T_LW13_KB_MO3), NG, indm, ig, mf);
-            fr = ldt(tab<R>(T_LW13_FRACREFB) + ig);
+            tg = s.colamt[2][k0] * interpv<V>(tab<R>(T_LW13_KB_MO3), NG, indm, ig, mf);
+            fr = ldv<V>(tab<R>(T_LW13_FRACREFB) + ig);
         }
         break;
     }
@@ -552,26 +551,26 @@ __device__ void lw_gas(const S& s, int g, int k0, R& tg, R& fr, int band_of_g = 
             const int br = br_joint(sp, sp1);
             const Sel<R> s0 = sel_branch(br, fs, ((jpk - 1) * 5 + (jtk - 1)) * 9 + js);
             const Sel<R> s1 = sel_branch(br, fs1, (jpk * 5 + (jt1k - 1)) * 9 + js1);
-            const R tauself = sfac * interp(tab<R>(T_LW15_SELFREF), NG, inds, ig, sfr);
-            const R taufor = ffac * interp(tab<R>(T_LW15_FORREF), NG, indf, ig, ffr);
-            const R taun2 = scalen2 * minor2d(tab<R>(T_LW15_KA_MN2), 9, NG, jm, fm, indm, mf, ig);
+            const V tauself = sfac * interpv<V>(tab<R>(T_LW15_SELFREF), NG, inds, ig, sfr);
+            const V taufor = ffac * interpv<V>(tab<R>(T_LW15_FORREF), NG, indf, ig, ffr);
+            const V taun2 = scalen2 * minor2d<V>(tab<R>(T_LW15_KA_MN2), 9, NG, jm, fm, indm, mf, ig);
             const R* absa = tab<R>(T_LW15_ABSA);
-            auto A = [&](int id) { return ldt(absa + ((id - 1) * NG + ig)); };
-            const R sumA = s0.fk0 * f00 * A(s0.id[0]) + s0.fk0 * f10 * A(s0.id[1]) + s0.fk1 * f00 * A(s0.id[2]) +
+            auto A = [&](int id) { return ldv<V>(absa + ((id - 1) * NG + ig)); };
+            const V sumA = s0.fk0 * f00 * A(s0.id[0]) + s0.fk0 * f10 * A(s0.id[1]) + s0.fk1 * f00 * A(s0.id[2]) +
                            s0.fk1 * f10 * A(s0.id[3]) + s0.fk2 * f00 * A(s0.id[4]) + s0.fk2 * f10 * A(s0.id[5]);
-            const R sumB = s1.fk0 * f01 * A(s1.id[0]) + s1.fk0 * f11 * A(s1.id[1]) + s1.fk1 * f01 * A(s1.id[2]) +
+            const V sumB = s1.fk0 * f01 * A(s1.id[0]) + s1.fk0 * f11 * A(s1.id[1]) + s1.fk1 * f01 * A(s1.id[2]) +
                            s1.fk1 * f11 * A(s1.id[3]) + s1.fk2 * f01 * A(s1.id[4]) + s1.fk2 * f11 * A(s1.id[5]);
             tg = sc * sumA + sc1 * sumB + tauself + taufor + taun2;
-            fr = interp(tab<R>(T_LW15_FRACREFA), NG, jpl, ig, fpl);
+            fr = interpv<V>(tab<R>(T_LW15_FRACREFA), NG, jpl, ig, fpl);
         } else {
-            tg = 0;
-            fr = 0;
+            tg = vall<V>((R)0);
+            fr = vall<V>((R)0);
         }
         break;
     }
     default:
-        tg = 0;
-        fr = 0;
+        tg = vall<V>((R)0);
+        fr = vall<V>((R)0);
     }
 }
 
@@ -1056,9 +1055,10 @@ __device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink si
         if (lane == 0) lw_overlap(s, nlay);
         __syncwarp();
     }
-    for_each_band_flat(c_lw_ns, 16, nlay, &s.task_next, lane, [&](int g, int k0, int band) {
-        R tg, fr;
-        lw_gas(s, g, k0, tg, fr, band);
+    using V = typename S::Gas;
+    for_each_band_flat<S::kGas>(c_lw_ns, 16, nlay, &s.task_next, lane, [&](int g, int k0, int band) {
+        V tg, fr;
+        lw_gas<R, V>(s, g, k0, tg, fr, band);
         sink(g, k0, tg + s.tauaer[band][k0], fr);
     });
     __syncthreads();

@@ -62,7 +62,7 @@ __host__ __device__ constexpr int64_t lw3_block_floats(int nlay) { return (LW3_H
 // per CTA share a column's (g-point, layer) tasks and hide the gathers' latency.  Measured over the LW of 262,144
 // columns: 160 threads 66.1 ms, 192 63.3, 224 61.4, 256 60.5, 288 60.0, 320 63.8 (spills); 4 CTAs of 224 / 256
 // threads 64.0 / 70.1, 2 of 320 / 384 threads 64.0 / 62.6.  Same bits for every shape.
-constexpr int LW3_OPT_THREADS = 288;
+constexpr int LW3_OPT_THREADS = 256;
 constexpr int LW3_OPT_MINB = 3;        // CTAs per SM the optics kernel is compiled for
 
 __global__ void __launch_bounds__(LW3_OPT_THREADS, LW3_OPT_MINB) lw3_optics_kernel(const __grid_constant__ LwBatch bt, int64_t c0,
@@ -82,9 +82,9 @@ __global__ void __launch_bounds__(LW3_OPT_THREADS, LW3_OPT_MINB) lw3_optics_kern
     }
     float* blk = scr + (int64_t)blockIdx.x * lw3_block_floats(nlay);
     float* row = blk + LW3_HEAD;
-    lw_setup_core<float, LW3_OPT_THREADS>(s, a, col, tid, [&](int g, int k0, float tg, float fr) {
-        row[k0 * LW3_ROW + g] = tg;
-        row[k0 * LW3_ROW + LW_NGPT + g] = fr;
+    lw_setup_core<float, LW3_OPT_THREADS>(s, a, col, tid, [&](int g, int k0, P2 tg, P2 fr) {
+        *reinterpret_cast<float2*>(row + k0 * LW3_ROW + g) = make_float2(tg.x, tg.y);
+        *reinterpret_cast<float2*>(row + k0 * LW3_ROW + LW_NGPT + g) = make_float2(fr.x, fr.y);
     });
     float* aux = row + 2 * LW_NGPT;                // layer k's record at aux + (k - 1) LW3_ROW
     for (int i = tid; i < nlay * 64; i += LW3_OPT_THREADS) {

@@ -119,8 +119,8 @@ __device__ __forceinline__ void sw_species(const S& s, int slot, int k0, R x1, R
 // ------------------------------------------------------------------------------------------------------
 // Gas and Rayleigh optical depths of SW g-point g (0..111) at layer k0 (phys_rrtm_sw_taumol16..29.cu with
 // the reference's handling of the layer k = laytrop).
-template <class R, class S>
-__device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = -1)
+template <class R, class V, class S>
+__device__ void sw_gas(const S& s, int g, int k0, V& tg, V& tr, int band_of_g = -1)
 {
     const int k = k0 + 1, lt = s.laytrop;
     const int jpk = s.jp[k0], jtk = s.jt[k0], jt1k = s.jt1[k0];
@@ -148,14 +148,14 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
         const R fac001 = fs1 * f01, fac011 = fs1 * f11, fac101 = fs * f01, fac111 = fs * f11;
         const int i01 = max(1, min(msa, id0 + js)), i02 = min(msa, i01 + 1), i03 = min(msa, i01 + o1), i04 = min(msa, i01 + o2);
         const int i11 = max(1, min(msa, id1 + js)), i12 = min(msa, i11 + 1), i13 = min(msa, i11 + o1), i14 = min(msa, i11 + o2);
-        auto a = [&](int i) { return ldt(A + (size_t)(i - 1) * ng + ig); };
+        auto a = [&](int i) { return ldv<V>(A + ((i - 1) * ng + ig)); };
         return fac000 * a(i01) + fac100 * a(i02) + fac010 * a(i03) + fac110 * a(i04) + fac001 * a(i11) +
                fac101 * a(i12) + fac011 * a(i13) + fac111 * a(i14);
     };
     auto sum4 = [&](const R* A, int ng, int ms, int id0, int id1) {
         const int i01 = max(1, min(ms, id0 + 1)), i02 = min(ms, i01 + 1);
         const int i11 = max(1, min(ms, id1 + 1)), i12 = min(ms, i11 + 1);
-        auto a = [&](int i) { return ldt(A + (size_t)(i - 1) * ng + ig); };
+        auto a = [&](int i) { return ldv<V>(A + ((i - 1) * ng + ig)); };
         return f00 * a(i01) + f10 * a(i02) + f01 * a(i11) + f11 * a(i12);
     };
     // key-species ratio parameter of the band's layer (sw_species); sc = x1 + strr x2 multiplies the sum
@@ -163,15 +163,15 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
         sc = x1 + strr * x2;
         sw_species<R>(s, slot, k0, x1, sc, mult, om, guard, js, fs);
     };
-    auto SF = [&](int id, int ng) { return sfac * interp(tab<R>(id), ng, inds, ig, sfrac); };
-    auto FF = [&](int id, int ng) { return ffac * interp(tab<R>(id), ng, indf, ig, ffrac); };
+    auto SF = [&](int id, int ng) { return sfac * interpv<V>(tab<R>(id), ng, inds, ig, sfrac); };
+    auto FF = [&](int id, int ng) { return ffac * interpv<V>(tab<R>(id), ng, indf, ig, ffrac); };
     int id0, id1;
     switch (jb) {
     case 16: {
         const int NG = 6;
         idx(16, id0, id1);
-        tr = cm * ldt(tab<R>(T_SW16_RAYL));
-        tg = 0;
+        tr = vall<V>(cm * ldt(tab<R>(T_SW16_RAYL)));
+        tg = vall<V>((R)0);
         if (k <= lt) {
             R sc, fs; int js;
             jsfs(0, c1, ldt(tab<R>(T_SW16_STRRAT)), c5, (R)8, oneminus, sc, js, fs);
@@ -184,23 +184,23 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
     case 17: {
         const int NG = 12;
         const R strr = (R)ldt(tab<R>(T_SW_STRRAT) + 1);
-        tr = cm * (R)6.86e-10f;
+        tr = vall<V>(cm * (R)6.86e-10f);
         R sc, fs; int js;
         if (k0 < lt) {
             jsfs(1, c1, strr, c2, (R)8, oneminus, sc, js, fs);
             const int i0 = ((jpk - 1) * 5 + (jtk - 1)) * 9, i1 = (jpk * 5 + (jt1k - 1)) * 9;
-            const R selfpart = inds > 0 ? SF(T_SW17_SELFREF, NG) : (R)0;
+            const V selfpart = inds > 0 ? SF(T_SW17_SELFREF, NG) : vall<V>((R)0);
             tg = sc * sum8(tab<R>(T_SW17_ABSA), NG, 585, i0, i1, js, fs, 9, 10) + c1 * (selfpart + FF(T_SW17_FORREF, NG));
         } else {
             jsfs(1, c1, strr, c2, (R)4, oneminus, sc, js, fs);
             const int i0 = ((jpk - 13) * 5 + (jtk - 1)) * 5, i1 = ((jpk - 12) * 5 + (jt1k - 1)) * 5;
-            tg = sc * sum8(tab<R>(T_SW17_ABSB), NG, 1175, i0, i1, js, fs, 5, 6) + (c1 * ffac) * interp(tab<R>(T_SW17_FORREF), NG, indf, ig, ffrac);
+            tg = sc * sum8(tab<R>(T_SW17_ABSB), NG, 1175, i0, i1, js, fs, 5, 6) + (c1 * ffac) * interpv<V>(tab<R>(T_SW17_FORREF), NG, indf, ig, ffrac);
         }
         break;
     }
     case 18: {
         const int NG = 8;
-        tr = cm * ldt(tab<R>(T_SW18_RAYL));
+        tr = vall<V>(cm * ldt(tab<R>(T_SW18_RAYL)));
         idx(18, id0, id1);
         if (k <= lt) {
             R sc, fs; int js;
@@ -214,9 +214,9 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
     }
     case 19: {
         const int NG = 8;
-        tr = cm * (R)2.29e-09f;
+        tr = vall<V>(cm * (R)2.29e-09f);
         idx(19, id0, id1);
-        tg = 0;
+        tg = vall<V>((R)0);
         if (k <= lt) {
             R sc, fs; int js;
             jsfs(3, c1, (R)5.49281e+0f, c2, (R)8, swom, sc, js, fs);
@@ -228,25 +228,25 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
     }
     case 20: {
         const int NG = 10;
-        tr = cm * ldt(tab<R>(T_SW20_RAYL));
-        const R ch4 = ldt(tab<R>(T_SW20_ABSCH4) + ig);
+        tr = vall<V>(cm * ldt(tab<R>(T_SW20_RAYL)));
+        const V ch4 = ldv<V>(tab<R>(T_SW20_ABSCH4) + ig);
         if (k <= lt) {
             const int i0 = (jpk - 1) * 5 + (jtk - 1), i1 = jpk * 5 + (jt1k - 1);
-            tg = c1 * ((sum4(tab<R>(T_SW20_ABSA), NG, 65, i0, i1)) + sfac * interp(tab<R>(T_SW20_SELFREF), NG, inds, ig, sfrac) +
-                       ffac * interp(tab<R>(T_SW20_FORREF), NG, indf, ig, ffrac)) + c5 * ch4;
+            tg = c1 * ((sum4(tab<R>(T_SW20_ABSA), NG, 65, i0, i1)) + sfac * interpv<V>(tab<R>(T_SW20_SELFREF), NG, inds, ig, sfrac) +
+                       ffac * interpv<V>(tab<R>(T_SW20_FORREF), NG, indf, ig, ffrac)) + c5 * ch4;
         } else {
             const int i0 = (jpk - 13) * 5 + (jtk - 1), i1 = (jpk - 12) * 5 + (jt1k - 1);
-            tg = c1 * ((sum4(tab<R>(T_SW20_ABSB), NG, 235, i0, i1)) + ffac * interp(tab<R>(T_SW20_FORREF), NG, indf, ig, ffrac)) + c5 * ch4;
+            tg = c1 * ((sum4(tab<R>(T_SW20_ABSB), NG, 235, i0, i1)) + ffac * interpv<V>(tab<R>(T_SW20_FORREF), NG, indf, ig, ffrac)) + c5 * ch4;
         }
         break;
     }
     case 21: {
         const int NG = 10;
-        tr = cm * (R)9.41e-09f;
+        tr = vall<V>(cm * (R)9.41e-09f);
         const R strr = (R)4.53210e-03f;
         if (k <= lt) { id0 = ((jpk - 1) * 5 + (jtk - 1)) * 9; id1 = (jpk * 5 + (jt1k - 1)) * 9; }
         else { id0 = ((jpk - 13) * 5 + (jtk - 1)) * 5; id1 = ((jpk - 12) * 5 + (jt1k - 1)) * 5; }
-        tg = 0;
+        tg = vall<V>((R)0);
         R sc, fs; int js;
         if (k < lt) {
             jsfs(4, c1, strr, c2, (R)8, oneminus, sc, js, fs);
@@ -256,14 +256,14 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
         if (k >= lt) {
             jsfs(4, c1, strr, c2, (R)4, oneminus, sc, js, fs);
             tg = sc * sum8(tab<R>(T_SW21_ABSB), NG, 1175, id0, id1, js, fs, 5, 6) +
-                 c1 * ffac * interp(tab<R>(T_SW21_FORREF), NG, indf, ig, ffrac);
+                 c1 * ffac * interpv<V>(tab<R>(T_SW21_FORREF), NG, indf, ig, ffrac);
         }
         break;
     }
     case 22: {
         const int NG = 2;
         idx(22, id0, id1);
-        tr = cm * (R)1.54e-08f;
+        tr = vall<V>(cm * (R)1.54e-08f);
         const R o2cont = (R)4.35e-4f / ((R)350.0f * (R)2.0f) * c6;
         if (k <= lt) {
             R sc, fs; int js;
@@ -277,13 +277,13 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
     }
     case 23: {
         const int NG = 10;
-        tr = cm * ldt(tab<R>(T_SW23_RAYL) + ig);
+        tr = cm * ldv<V>(tab<R>(T_SW23_RAYL) + ig);
         const bool zero_cond = (k >= s.kmin8 + 1) && (k >= lt);
         if ((k <= lt) && !zero_cond) {
             const int i0 = (jpk - 1) * 5 + (jtk - 1), i1 = jpk * 5 + (jt1k - 1);
             tg = c1 * ((R)1.029f * sum4(tab<R>(T_SW23_ABSA), NG, 65, i0, i1) + SF(T_SW23_SELFREF, NG) + FF(T_SW23_FORREF, NG));
         } else {
-            tg = 0;
+            tg = vall<V>((R)0);
         }
         break;
     }
@@ -293,37 +293,37 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
         if (k <= lt) {
             R sc, fs; int js;
             jsfs(6, c1, (R)1.24692e-1f, c6, (R)8, swom, sc, js, fs);
-            tg = sc * sum8(tab<R>(T_SW24_ABSA), NG, 585, id0, id1, js, fs, 9, 10) + c3 * ldt(tab<R>(T_SW24_ABSO3A) + ig) +
+            tg = sc * sum8(tab<R>(T_SW24_ABSA), NG, 585, id0, id1, js, fs, 9, 10) + c3 * ldv<V>(tab<R>(T_SW24_ABSO3A) + ig) +
                  c1 * (SF(T_SW24_SELFREF, NG) + FF(T_SW24_FORREF, NG));
-            const R r0 = ldt(tab<R>(T_SW24_RAYLA) + (size_t)(js - 1) * NG + ig), r1 = ldt(tab<R>(T_SW24_RAYLA) + (size_t)js * NG + ig);
+            const V r0 = ldv<V>(tab<R>(T_SW24_RAYLA) + ((js - 1) * NG + ig)), r1 = ldv<V>(tab<R>(T_SW24_RAYLA) + (js * NG + ig));
             tr = cm * (r0 + fs * (r1 - r0));
         } else {
-            tg = c6 * sum4(tab<R>(T_SW24_ABSB), NG, 235, id0, id1) + c3 * ldt(tab<R>(T_SW24_ABSO3B) + ig);
-            tr = cm * ldt(tab<R>(T_SW24_RAYLB) + ig);
+            tg = c6 * sum4(tab<R>(T_SW24_ABSB), NG, 235, id0, id1) + c3 * ldv<V>(tab<R>(T_SW24_ABSO3B) + ig);
+            tr = cm * ldv<V>(tab<R>(T_SW24_RAYLB) + ig);
         }
         break;
     }
     case 25: {
         const int NG = 6;
-        tr = cm * ldt(tab<R>(T_SW25_RAYL) + ig);
-        tg = 0;
+        tr = cm * ldv<V>(tab<R>(T_SW25_RAYL) + ig);
+        tg = vall<V>((R)0);
         if (k <= lt) {
             idx(25, id0, id1);
-            tg = c1 * sum4(tab<R>(T_SW25_ABSA), NG, 65, id0, id1) + c3 * ldt(tab<R>(T_SW25_ABSO3A) + ig);
+            tg = c1 * sum4(tab<R>(T_SW25_ABSA), NG, 65, id0, id1) + c3 * ldv<V>(tab<R>(T_SW25_ABSO3A) + ig);
         }
-        if (k >= s.kminw + 1 && k >= lt) tg = c3 * ldt(tab<R>(T_SW25_ABSO3B) + ig);
+        if (k >= s.kminw + 1 && k >= lt) tg = c3 * ldv<V>(tab<R>(T_SW25_ABSO3B) + ig);
         break;
     }
     case 26:
-        tg = 0;
-        tr = cm * ldt(tab<R>(T_SW26_RAYL) + ig);
+        tg = vall<V>((R)0);
+        tr = cm * ldv<V>(tab<R>(T_SW26_RAYL) + ig);
         break;
     case 27: {
         const int NG = 8;
-        tr = cm * ldt(tab<R>(T_SW27_RAYL) + ig);
+        tr = cm * ldv<V>(tab<R>(T_SW27_RAYL) + ig);
         if (k <= lt) { id0 = (jpk - 1) * 5 + (jtk - 1); id1 = jpk * 5 + (jt1k - 1); }
         else { id0 = (jpk - 13) * 5 + (jtk - 1); id1 = (jpk - 12) * 5 + (jt1k - 1); }
-        tg = 0;
+        tg = vall<V>((R)0);
         if (k < lt) tg = c3 * sum4(tab<R>(T_SW27_ABSA), NG, 65, id0, id1);
         if (k >= lt) tg = c3 * sum4(tab<R>(T_SW27_ABSB), NG, 235, id0, id1);
         break;
@@ -331,9 +331,9 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
     case 28: {
         const int NG = 6;
         idx(28, id0, id1);
-        tr = cm * ldt(tab<R>(T_SW28_RAYL));
+        tr = vall<V>(cm * ldt(tab<R>(T_SW28_RAYL)));
         const R strr = ldt(tab<R>(T_SW28_STRRAT));
-        tg = 0;
+        tg = vall<V>((R)0);
         if (k <= lt) {
             R sc, fs; int js;
             jsfs(7, c3, strr, c6, (R)8, swom, sc, js, fs);
@@ -348,7 +348,7 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
     }
     default: {   // 29
         const int NG = 12;
-        tr = cm * (R)9.30e-11f;
+        tr = vall<V>(cm * (R)9.30e-11f);
         const bool low = k <= lt;
         const int i0 = low ? (jpk - 1) * 5 + (jtk - 1) : (jpk - 13) * 5 + (jtk - 1);
         const int i1 = low ? jpk * 5 + (jt1k - 1) : (jpk - 12) * 5 + (jt1k - 1);
@@ -356,12 +356,12 @@ __device__ void sw_gas(const S& s, int g, int k0, R& tg, R& tr, int band_of_g = 
             const int indsp = min(inds + 1, 10), indfp = min(indf + 1, 4);
             const R* Sref = tab<R>(T_SW29_SELFREF);
             const R* Fref = tab<R>(T_SW29_FORREF);
-            auto Sv = [&](int i) { return ldt(Sref + (size_t)(i - 1) * NG + ig); };
-            auto Fv = [&](int i) { return ldt(Fref + (size_t)(i - 1) * NG + ig); };
+            auto Sv = [&](int i) { return ldv<V>(Sref + ((i - 1) * NG + ig)); };
+            auto Fv = [&](int i) { return ldv<V>(Fref + ((i - 1) * NG + ig)); };
             tg = c1 * ((sum4(tab<R>(T_SW29_ABSA), NG, 65, i0, i1)) + sfac * (Sv(inds) + sfrac * (Sv(indsp) - Sv(inds))) +
-                       ffac * (Fv(indf) + ffrac * (Fv(indfp) - Fv(indf)))) + c2 * ldt(tab<R>(T_SW29_ABSCO2) + ig);
+                       ffac * (Fv(indf) + ffrac * (Fv(indfp) - Fv(indf)))) + c2 * ldv<V>(tab<R>(T_SW29_ABSCO2) + ig);
         } else {
-            tg = c2 * (sum4(tab<R>(T_SW29_ABSB), NG, 235, i0, i1)) + c1 * ldt(tab<R>(T_SW29_ABSH2O) + ig);
+            tg = c2 * (sum4(tab<R>(T_SW29_ABSB), NG, 235, i0, i1)) + c1 * ldv<V>(tab<R>(T_SW29_ABSH2O) + ig);
         }
         break;
     }
@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(SW_THREADS) sw_column_kernel(const __grid_cons
     for (int p = tid; p < SW_NGPT * nlay; p += SW_THREADS) {
         const int g = p / nlay, k0 = p - g * nlay;
         R tg, tr;
-        sw_gas(s, g, k0, tg, tr);
+        sw_gas<R>(s, g, k0, tg, tr);
         s.taug[g][k0] = tg;
         s.taur[g][k0] = tr;
     }

@@ -49,7 +49,8 @@ struct Sw4Hdr {
     float albbm[2], albdf[2], zcf0, zcf1, pad0[2];
     int cloudy;                      // the cloudy pass runs
     int ncl;                         // layers with a cloudy-pass R/T
-    int pad1[2];
+    int clr5;                        // the clear rows hold no e4 (it is e3: no delta scaling in the clear pass)
+    int pad1;
     signed char slot[NLAY_MAX];      // cloudy-pass slot of each layer; -1: the clear R/T serve both passes
 };
 static_assert(sizeof(Sw4Hdr) % 16 == 0, "the header is copied in 16-byte pieces");
@@ -265,11 +266,11 @@ sw4_gas_kernel(const __grid_constant__ SwBatch bt, int any_aer, int* err, int d0
     int4* im = img + (size_t)blockIdx.x * (sw4_image_bytes(any_aer) / 16);
     float* img_taug = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(im) + (offsetof(SwSh2, taug) - sw4_image_begin()));
     sw2_setup<SW4_GAS_THREADS>(s, aer, a, col, d, tid);
-    for_each_band_flat(c_sw_ns, 14, nlay, &s.task_next, tid & 31, [&](int g, int k0, int b) {
-        float tg, tr;
+    for_each_band_flat<2>(c_sw_ns, 14, nlay, &s.task_next, tid & 31, [&](int g, int k0, int b) {
+        P2 tg, tr;
         sw_gas<float>(s, g, k0, tg, tr, b);
-        img_taug[k0 * SW_NGPT + g] = tg;
-        if (g >= 66 && g < 74 && k0 < s.laytrop) s.taur24[g - 66][k0] = tr;
+        *reinterpret_cast<float2*>(img_taug + k0 * SW_NGPT + g) = make_float2(tg.x, tg.y);
+        if (b == 8 && k0 < s.laytrop) { s.taur24[g - 66][k0] = tr.x; s.taur24[g - 65][k0] = tr.y; }
     });
     __syncthreads();
     const int4* sm = reinterpret_cast<const int4*>(smem_raw + sw4_image_begin());
@@ -330,7 +331,7 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
     if (tid == 0) { qnear = 0; qres = 0; }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const bool cloudy = mc ? s.zcf1 > 0.0f : s.zcf1 > 1.0e-6f;
+    const bool cloudy = mc ? s.zcf1 > 0.0f : s.zcf1 > 1.0e-6f, clr5 = a.iswmode != 1 && !aer;
     // layers with a cloudy-pass R/T, counted from the surface (every warp forms the two words of layer bits)
     unsigned cw[2];
 #pragma unroll
@@ -356,6 +357,7 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
     }
     if (tid == 0) {
         H.ncl = ncl;
+        H.clr5 = clr5 ? 1 : 0;
         H.cloudy = cloudy ? 1 : 0;
         H.albbm[0] = s.albbm[0]; H.albbm[1] = s.albbm[1];
         H.albdf[0] = s.albdf[0]; H.albdf[1] = s.albdf[1];
@@ -393,9 +395,10 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
         wf = zs * (1.0f / SW2_FLUX_T);
         wk = zs * (1.5f * 86400.0f / SW2_HEAT_T) * rdf[k0];
     };
-    auto put = [&](float* p, const SwRT2& r) {   // p: the pair's place in field 0 of its layer's rows
+    auto put = [&](float* p, const SwRT2& r, bool e4) {   // p: the pair's place in field 0 of its layer's rows
         st2(p, r.rb); st2(p + SW_NGPT, r.rd); st2(p + 2 * SW_NGPT, r.tb); st2(p + 3 * SW_NGPT, r.td);
-        st2(p + 4 * SW_NGPT, r.e3); st2(p + 5 * SW_NGPT, r.e4);
+        st2(p + 4 * SW_NGPT, r.e3);
+        if (e4) st2(p + 5 * SW_NGPT, r.e4);
     };
     auto run = [&](auto mode_tag) {
         constexpr int MODE = decltype(mode_tag)::value;
@@ -409,12 +412,12 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
                 SwRT2 r;
                 int q0, q1;
                 sw4_rt<MODE, decltype(asy_tag)::value>(t0, ab, s0, y0, cz, snt, wk, wf, r, q0, q1);
-                put(rtc + (size_t)k0 * SW4_LAYER + g, r);
+                put(rtc + (size_t)k0 * SW4_LAYER + g, r, decltype(asy_tag)::value);
                 if (q0) enqueue(k0, g, q0);
                 if (q1) enqueue(k0, g + 1, q1);
             }
         };
-        if (MODE == 1 || aer) clear(std::true_type{});
+        if (!clr5) clear(std::true_type{});
         else clear(std::false_type{});
         __syncthreads();
         // cloudy pass: the layers with a slot, mixture R/T blended with the clear R/T (or, McICA, taken
@@ -430,7 +433,7 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
                                snt, wk, wf, m, q0, q1);
             const float* pc = rtc + (size_t)k0 * SW4_LAYER + g;
             const SwRT2 c{ld2(pc), ld2(pc + SW_NGPT), ld2(pc + 2 * SW_NGPT), ld2(pc + 3 * SW_NGPT), ld2(pc + 4 * SW_NGPT),
-                          ld2(pc + 5 * SW_NGPT)};
+                          ld2(pc + (clr5 ? 4 : 5) * SW_NGPT)};
             if (mc) {
                 const unsigned w = s.mcw[g >> 5][k0] >> (g & 31);
                 const bool b0 = w & 1u, b1 = w & 2u;
@@ -445,7 +448,7 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
                 m.rb = mix(m.rb, c.rb); m.rd = mix(m.rd, c.rd); m.tb = mix(m.tb, c.tb); m.td = mix(m.td, c.td);
                 m.e3 = mix(m.e3, c.e3); m.e4 = mix(m.e4, c.e4);
             }
-            put(rto + (size_t)sl * SW4_LAYER + g, m);
+            put(rto + (size_t)sl * SW4_LAYER + g, m, true);
             if (q0) enqueue(k0, g, q0);
             if (q1) enqueue(k0, g + 1, q1);
         }
@@ -579,7 +582,7 @@ sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int* err, int d0, int nc, c
     while (g >= c_sw_ns[ib0 + 1]) ++ib0;
     const int ibd = ib0 == 8 ? 0 : ((ib0 >= 9 && ib0 <= 12) ? 2 : 1);   // idxsfc
     const bool mc = a.mask != nullptr;
-    const bool cloudy = H.cloudy != 0;
+    const bool cloudy = H.cloudy != 0, clr5 = H.clr5 != 0;
     const float zsolar = act ? H.zsolar[g] : 0.0f;
     const float ab = ibd ? H.albbm[ibd - 1] : 0.5f * (H.albbm[0] + H.albbm[1]);
     const float ad = ibd ? H.albdf[ibd - 1] : 0.5f * (H.albdf[0] + H.albdf[1]);
@@ -595,7 +598,7 @@ sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int* err, int d0, int nc, c
         }
         const float* p = rtc + (size_t)k0 * SW4_LAYER + g;
         c.rb = __ldg(p); c.rd = __ldg(p + SW_NGPT); c.tb = __ldg(p + 2 * SW_NGPT); c.td = __ldg(p + 3 * SW_NGPT);
-        c.e3 = __ldg(p + 4 * SW_NGPT); c.e4 = __ldg(p + 5 * SW_NGPT);
+        c.e3 = __ldg(p + 4 * SW_NGPT); c.e4 = clr5 ? c.e3 : __ldg(p + 5 * SW_NGPT);
         const int sl = H.slot[k0];
         if (cloudy && sl >= 0) {
             const float* q = rto + (size_t)sl * SW4_LAYER + g;
