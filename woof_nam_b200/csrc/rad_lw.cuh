@@ -776,18 +776,17 @@ __device__ __forceinline__ void lw_setcoef_layer(S& s, int k0)
 // adjustments of taugb03 / taugb09 (N2O), taugb06, taugb07, taugb08 (CO2) and taugb13 (CO2), each the statement
 // of its band kernel (adjcol), evaluated once per layer rather than in every g-point's task.
 template <class R, class S>
-__device__ __forceinline__ void lw_keys_layer(S& s, int k0)
+__device__ __forceinline__ void lw_adjcol(S& s, int i, int k0)   // term i of LW_NADJ
 {
     const R* chi = tab<R>(T_LW_CHI_MLS);
     auto CHI = [&](int gg, int lev) { return ldt(chi + ((lev - 1) * 7 + (gg - 1))); };
     const int jpk = s.jp[k0];
-    const R c2 = s.colamt[1][k0], c4 = s.colamt[3][k0], dry = s.coldry[k0];
-    const R t2 = dry * CHI(2, jpk + 1);
-    s.adjc[0][k0] = adjcol(c4, dry * CHI(4, jpk + 1), (R)1.5f, (R)0.5f, (R)0.65f);
-    s.adjc[1][k0] = adjcol(c2, t2, (R)3, (R)2, (R)0.77f);
-    s.adjc[2][k0] = s.lower[k0] ? adjcol(c2, t2, (R)3, (R)3, (R)0.79f) : adjcol(c2, t2, (R)3, (R)2, (R)0.79f);
-    s.adjc[3][k0] = adjcol(c2, t2, (R)3, (R)2, (R)0.65f);
-    s.adjc[4][k0] = adjcol(c2, dry * (R)3.55e-4f, (R)3, (R)2, (R)0.68f);
+    const R dry = s.coldry[k0], col = s.colamt[i == 0 ? 3 : 1][k0];
+    const R tem = i == 4 ? dry * (R)3.55e-4f : dry * CHI(i == 0 ? 4 : 2, jpk + 1);
+    // threshold, offset and exponent of taugb03 / 09, 06, 07, 08, 13
+    const R thr = i == 0 ? (R)1.5f : (R)3, off = i == 0 ? (R)0.5f : i == 2 && s.lower[k0] ? (R)3 : (R)2;
+    const R ex = i == 0 ? (R)0.65f : i == 1 ? (R)0.77f : i == 2 ? (R)0.79f : i == 3 ? (R)0.65f : (R)0.68f;
+    s.adjc[i][k0] = adjcol(col, tem, thr, off, ex);
 }
 // The column-independent ratios of reference mixing ratios the band kernels key their minor-gas and Planck-
 // fraction species by (taugb03, 07, 09, 12, 13, 16), formed once per column by threads 0..LW_NCHIR-1.
@@ -889,89 +888,85 @@ __device__ __forceinline__ R lw_secdiff(int b, R pwvcm)
                                              : fminR((R)1.80f, fmaxR((R)1.50f, (R)A0[b] + (R)A1[b] * rexp((R)A2[b] * pwvcm)));
 }
 
-// Maximum-random overlap factors of rtrnmr (phys_rrtm_lw_rtrnmr_body.cuh:51-172): a serial recurrence in k
-// over the layer cloud fractions, run by one thread.
+// Maximum-random overlap factors of rtrnmr (phys_rrtm_lw_rtrnmr_body.cuh:51-172): a serial recurrence in k over the
+// layer cloud fractions, run by one warp: its lanes clear the arrays, then lane 0 walks up and lane 1 down (the
+// downward statements are the upward ones with the levels mirrored, k <-> nlay + 1 - k).
 template <class R>
-__device__ void lw_overlap(LwSetup<R>& s, int nlay)
+__device__ void lw_overlap(LwSetup<R>& s, int nlay, int lane)
 {
     const R eps = (R)1.0e-6f;
     const int nlp1 = nlay + 1;
-    const R* cf = s.cldfrc;
-    for (int k = 0; k <= nlp1; ++k) {
+    for (int k = lane; k <= nlp1; k += 32) {
         s.faccld1u[k] = 0; s.faccld2u[k] = 0; s.facclr1u[k] = 0; s.facclr2u[k] = 0; s.faccmb1u[k] = 0; s.faccmb2u[k] = 0;
         s.faccld1d[k] = 0; s.faccld2d[k] = 0; s.facclr1d[k] = 0; s.facclr2d[k] = 0; s.faccmb1d[k] = 0; s.faccmb2d[k] = 0;
         s.lstu[k] = 0; s.lstd[k] = 0;
     }
-    s.lstu[1] = cf[1] > eps ? 1 : 0;
-    R rat1 = 0, rat2 = 0;
-    for (int k = 1; k <= nlay - 1; ++k) {
-        s.lstu[k + 1] = (cf[k + 1] > eps && cf[k] <= eps) ? 1 : 0;
-        if (cf[k] > eps) {
-            if (cf[k + 1] >= cf[k]) {
-                if (s.lstu[k]) {
-                    if (cf[k] < (R)1) s.facclr2u[k + 1] = (cf[k + 1] - cf[k]) / ((R)1 - cf[k]);
-                    s.facclr2u[k] = 0; s.faccld2u[k] = 0;
-                } else {
-                    const R fmx = fmaxR(cf[k], cf[k - 1]);
-                    if (cf[k + 1] > fmx) { s.facclr1u[k + 1] = rat2; s.facclr2u[k + 1] = (cf[k + 1] - fmx) / ((R)1 - fmx); }
-                    else if (cf[k + 1] < fmx) s.facclr1u[k + 1] = (cf[k + 1] - cf[k]) / (cf[k - 1] - cf[k]);
-                    else s.facclr1u[k + 1] = rat2;
+    __syncwarp();
+    if (lane < 2) {
+        const bool up = lane == 0;
+        const int o = up ? 0 : nlp1, sg = up ? 1 : -1;             // level k of the walk is level o + sg k
+        R *const clr1 = up ? s.facclr1u : s.facclr1d, *const clr2 = up ? s.facclr2u : s.facclr2d;
+        R *const cld1 = up ? s.faccld1u : s.faccld1d, *const cld2 = up ? s.faccld2u : s.faccld2d;
+        R *const cmb1 = up ? s.faccmb1u : s.faccmb1d, *const cmb2 = up ? s.faccmb2u : s.faccmb2d;
+        int* const lst = up ? s.lstu : s.lstd;
+        R rat1 = 0, rat2 = 0, cp = s.cldfrc[o], c = s.cldfrc[o + sg];   // fractions of levels k - 1 and k
+        bool st = c > eps;                                          // lst of level k
+        lst[o + sg] = st ? 1 : 0;
+        R lr2 = 0, ld2 = 0;                                         // clr2 and cld2 of level k
+        for (int k = 1; k <= nlay - 1; ++k) {
+            const int i = o + sg * k, n = i + sg;
+            const R cn = s.cldfrc[n];
+            const bool stn = cn > eps && c <= eps;
+            if (stn) lst[n] = 1;
+            R r1 = 0, r2 = 0, d1 = 0, d2 = 0;                       // clr1, clr2, cld1, cld2 of level k + 1
+            if (c > eps) {
+                if (st) {
+                    clr2[i] = 0; cld2[i] = 0;
+                    lr2 = 0; ld2 = 0;
                 }
-                if (s.facclr1u[k + 1] > 0 || s.facclr2u[k + 1] > 0) { rat1 = 1; rat2 = 0; } else { rat1 = 0; rat2 = 0; }
-            } else {
-                if (s.lstu[k]) {
-                    s.faccld2u[k + 1] = (cf[k] - cf[k + 1]) / cf[k];
-                    s.facclr2u[k] = 0; s.faccld2u[k] = 0;
+                if (cn >= c) {
+                    if (st) {
+                        if (c < (R)1) r2 = (cn - c) / ((R)1 - c);
+                    } else {
+                        const R fmx = fmaxR(c, cp);
+                        if (cn > fmx) { r1 = rat2; r2 = (cn - fmx) / ((R)1 - fmx); }
+                        else if (cn < fmx) r1 = (cn - c) / (cp - c);
+                        else r1 = rat2;
+                    }
+                    if (r1 > 0 || r2 > 0) { rat1 = 1; rat2 = 0; } else { rat1 = 0; rat2 = 0; }
                 } else {
-                    const R fmn = fminR(cf[k], cf[k - 1]);
-                    if (cf[k + 1] <= fmn) { s.faccld1u[k + 1] = rat1; s.faccld2u[k + 1] = (fmn - cf[k + 1]) / fmn; }
-                    else s.faccld1u[k + 1] = (cf[k] - cf[k + 1]) / (cf[k] - fmn);
+                    if (st) {
+                        d2 = (c - cn) / c;
+                    } else {
+                        const R fmn = fminR(c, cp);
+                        if (cn <= fmn) { d1 = rat1; d2 = (fmn - cn) / fmn; }
+                        else d1 = (c - cn) / (c - fmn);
+                    }
+                    if (d1 > 0 || d2 > 0) { rat1 = 0; rat2 = 1; } else { rat1 = 0; rat2 = 0; }
                 }
-                if (s.faccld1u[k + 1] > 0 || s.faccld2u[k + 1] > 0) { rat1 = 0; rat2 = 1; } else { rat1 = 0; rat2 = 0; }
+                clr1[n] = r1; clr2[n] = r2; cld1[n] = d1; cld2[n] = d2;
+                cmb1[n] = r1 * ld2 * cp;
+                cmb2[n] = d1 * lr2 * ((R)1 - cp);
             }
-            s.faccmb1u[k + 1] = s.facclr1u[k + 1] * s.faccld2u[k] * cf[k - 1];
-            s.faccmb2u[k + 1] = s.faccld1u[k + 1] * s.facclr2u[k] * ((R)1 - cf[k - 1]);
+            cp = c; c = cn; st = stn; lr2 = r2; ld2 = d2;
         }
     }
-    s.lstd[nlay] = cf[nlay] > eps ? 1 : 0;
-    rat1 = 0; rat2 = 0;
-    for (int k = nlay; k >= 2; --k) {
-        s.lstd[k - 1] = (cf[k - 1] > eps && cf[k] <= eps) ? 1 : 0;
-        if (cf[k] > eps) {
-            if (cf[k - 1] >= cf[k]) {
-                if (s.lstd[k]) {
-                    if (cf[k] < (R)1) s.facclr2d[k - 1] = (cf[k - 1] - cf[k]) / ((R)1 - cf[k]);
-                    s.facclr2d[k] = 0; s.faccld2d[k] = 0;
-                } else {
-                    const R fmx = fmaxR(cf[k], cf[k + 1]);
-                    if (cf[k - 1] > fmx) { s.facclr1d[k - 1] = rat2; s.facclr2d[k - 1] = (cf[k - 1] - fmx) / ((R)1 - fmx); }
-                    else if (cf[k - 1] < fmx) s.facclr1d[k - 1] = (cf[k - 1] - cf[k]) / (cf[k + 1] - cf[k]);
-                    else s.facclr1d[k - 1] = rat2;
-                }
-                if (s.facclr1d[k - 1] > 0 || s.facclr2d[k - 1] > 0) { rat1 = 1; rat2 = 0; } else { rat1 = 0; rat2 = 0; }
-            } else {
-                if (s.lstd[k]) {
-                    s.faccld2d[k - 1] = (cf[k] - cf[k - 1]) / cf[k];
-                    s.facclr2d[k] = 0; s.faccld2d[k] = 0;
-                } else {
-                    const R fmn = fminR(cf[k], cf[k + 1]);
-                    if (cf[k - 1] <= fmn) { s.faccld1d[k - 1] = rat1; s.faccld2d[k - 1] = (fmn - cf[k - 1]) / fmn; }
-                    else s.faccld1d[k - 1] = (cf[k] - cf[k - 1]) / (cf[k] - fmn);
-                }
-                if (s.faccld1d[k - 1] > 0 || s.faccld2d[k - 1] > 0) { rat1 = 0; rat2 = 1; } else { rat1 = 0; rat2 = 0; }
-            }
-            s.faccmb1d[k - 1] = s.facclr1d[k - 1] * s.faccld2d[k] * cf[k + 1];
-            s.faccmb2d[k - 1] = s.faccld1d[k - 1] * s.facclr2d[k] * ((R)1 - cf[k + 1]);
-        }
-    }
+    __syncwarp();
 }
 
 // ------------------------------------------------------------------------------------------------------
 // Phases A and B of the LW column (everything before the sweeps), shared by the column kernels:
 // absorber amounts, cloud optics, setcoef, Planck functions, gas optics per (g, layer) and the
-// max-random overlap factors of rtrnmr, all in shared memory.  NT threads, tid = threadIdx.x.
-template <class R, int NT, class Sink, class S>
-__device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink sink)
+// max-random overlap factors of rtrnmr, all in shared memory.  NT threads, tid = threadIdx.x.  sink takes each task's
+// result; ready() is run by every thread before its first task (the layer data is complete, the overlap factors are
+// not), layers(lane) by the warp that has formed the overlap factors.
+struct LwNoHook {
+    __device__ __forceinline__ void operator()() const {}
+    __device__ __forceinline__ void operator()(int) const {}
+};
+template <class R, int NT, class Sink, class S, class Ready = LwNoHook, class Layers = LwNoHook>
+__device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink sink, Ready ready = Ready(),
+                              Layers layers = Layers())
 {
     const int nlay = a.nlay, nlp1 = nlay + 1;
     const int64_t N = a.ncol;
@@ -988,26 +983,31 @@ __device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink si
         s.cldfrc[k0 + 1] = IN(a.clouds, kin);
     }
     __syncthreads();
-    // ---- column reductions in the reference's order (thread 0): pwvcm, lcf1, laytrop flags
-    if (tid == 0) {
-        s.cldfrc[0] = 1;
-        s.cldfrc[nlay + 1] = 0;
-        R tem1 = 0, tem2 = 0;
-        for (int k0 = 0; k0 < nlay; ++k0) {
-            tem1 = tem1 + s.coldry[k0] + s.colamt[0][k0];
-            tem2 = tem2 + s.colamt[0][k0];
-        }
-        const R amdw = (R)28.9644 / (R)18.0154;
-        s.pwvcm = (R)10.0 * tem2 / (amdw * tem1 * (R)9.80665) * IN(a.plvl, nlay);
-        int lcf = 0;
-        for (int k = 1; k <= nlay; ++k)
-            if (s.cldfrc[k] > eps) { lcf = 1; break; }
-        s.lcf1 = lcf;
-        s.stemp = (R)__ldg(a.tsfg + col);
+    // ---- column reductions (the first warp): precipitable water in float64, lcf1, laytrop
+    if (tid < 32) {
+        double tem1 = 0, tem2 = 0;
         int lt = 0;
-        for (int k0 = 0; k0 < nlay; ++k0) lt += s.lower[k0] ? 1 : 0;
-        s.laytrop = lt;
-        s.task_next = 0;
+        bool cl = false;
+        for (int k0 = tid; k0 < nlay; k0 += 32) {
+            tem1 += (double)s.coldry[k0] + (double)s.colamt[0][k0];
+            tem2 += (double)s.colamt[0][k0];
+            cl = cl || s.cldfrc[k0 + 1] > eps;
+            lt += s.lower[k0] ? 1 : 0;
+        }
+        tem1 = warp_sum(tem1);
+        tem2 = warp_sum(tem2);
+        lt = __reduce_add_sync(0xffffffffu, lt);
+        cl = __any_sync(0xffffffffu, cl);
+        if (tid == 0) {
+            const double amdw = 28.9644 / 18.0154;
+            s.cldfrc[0] = 1;
+            s.cldfrc[nlay + 1] = 0;
+            s.pwvcm = (R)(10.0 * tem2 / (amdw * tem1 * 9.80665) * (double)IN(a.plvl, nlay));
+            s.lcf1 = cl ? 1 : 0;
+            s.stemp = (R)__ldg(a.tsfg + col);
+            s.laytrop = lt;
+            s.task_next = 0;
+        }
     }
     __syncthreads();
     // ---- phase A2: secdiff/semiss, cldprop, setcoef, Planck functions
@@ -1028,7 +1028,6 @@ __device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink si
     auto layer_a2 = [&](int k0) {
         lw_cldprop_layer<R>(s, a, col, k0, s.lcf1, ilwcliq);
         lw_setcoef_layer<R>(s, k0);
-        lw_keys_layer<R>(s, k0);
     };
     if constexpr (NT >= 256) {
         if (tid < NLAY_MAX) {
@@ -1044,16 +1043,21 @@ __device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink si
         planck(tid, NT);
     }
     __syncthreads();
-    if constexpr (S::kKeys) {   // the species keys of bands 3, 4, 5, 7, 9 per layer (they read the chi ratios)
-        for (int i = tid; i < LW_NKEYB * nlay; i += NT) lw_keys_band<R>(s, i / nlay, i % nlay);
-        __syncthreads();
+    // the minor-gas column adjustments and the species keys of bands 3, 4, 5, 7, 9 per layer (they read the setcoef
+    // results and the chi ratios), an item per thread
+    for (int i = tid; i < (LW_NADJ + (S::kKeys ? LW_NKEYB : 0)) * nlay; i += NT) {
+        const int q = i / nlay, k0 = i - q * nlay;
+        if (q < LW_NADJ) lw_adjcol<R>(s, q, k0);
+        else if constexpr (S::kKeys) lw_keys_band<R>(s, q - LW_NADJ, k0);
     }
+    __syncthreads();
     // ---- phase B: gas optics per (g, layer), band by band; the last warp first computes the overlap
     // factors of rtrnmr (a serial recurrence in k, one lane) and then joins the task queue
     const int warp = tid >> 5, lane = tid & 31;
+    ready();
     if (warp == NT / 32 - 1) {
-        if (lane == 0) lw_overlap(s, nlay);
-        __syncwarp();
+        lw_overlap(s, nlay, lane);
+        layers(lane);
     }
     using V = typename S::Gas;
     for_each_band_flat<S::kGas>(c_lw_ns, 16, nlay, &s.task_next, lane, [&](int g, int k0, int band) {

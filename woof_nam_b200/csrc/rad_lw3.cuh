@@ -51,7 +51,6 @@ constexpr int R_FACU = 73;      // [6] upward factors at k + 1, same order
 constexpr int H_PKLAY0 = 0;     // [16] pklay[0] (surface)
 constexpr int H_SECDIFF = 16;   // [16]
 constexpr int H_SEMISS = 32;    // [16]
-constexpr int H_FP64 = 48;      // int: 1 when the column is to be solved in float64 (lw3_fp64_kernel)
 
 constexpr float LW3_THIN = LW_THIN;   // hPa: a cloudy layer thinner than this sends the column to float64
 
@@ -82,38 +81,43 @@ __global__ void __launch_bounds__(LW3_OPT_THREADS, LW3_OPT_MINB) lw3_optics_kern
     }
     float* blk = scr + (int64_t)blockIdx.x * lw3_block_floats(nlay);
     float* row = blk + LW3_HEAD;
-    lw_setup_core<float, LW3_OPT_THREADS>(s, a, col, tid, [&](int g, int k0, P2 tg, P2 fr) {
-        *reinterpret_cast<float2*>(row + k0 * LW3_ROW + g) = make_float2(tg.x, tg.y);
-        *reinterpret_cast<float2*>(row + k0 * LW3_ROW + LW_NGPT + g) = make_float2(fr.x, fr.y);
-    });
     float* aux = row + 2 * LW_NGPT;                // layer k's record at aux + (k - 1) LW3_ROW
-    for (int i = tid; i < nlay * 64; i += LW3_OPT_THREADS) {
-        const int k = 1 + (i >> 6), w = i & 63, b = w & 15;
-        aux[(k - 1) * LW3_ROW + w] = w < 16 ? s.pklay[k][b] : w < 32 ? s.pklev[k][b] : w < 48 ? s.pklev[k - 1][b] : s.taucld[b][k - 1];
-    }
-    for (int k = 1 + tid; k <= nlay; k += LW3_OPT_THREADS) {
-        float* r = aux + (k - 1) * LW3_ROW;
-        r[R_CLDFRC] = s.cldfrc[k];
-        r[R_LSTU] = __int_as_float(s.lstu[k]);
-        r[R_LSTD] = __int_as_float(s.lstd[k]);
-        const float fd[6] = {s.facclr1d[k - 1], s.faccld1d[k - 1], s.faccmb1d[k - 1], s.faccmb2d[k - 1],
-                             s.facclr2d[k - 1], s.faccld2d[k - 1]};
-        const float fu[6] = {s.facclr1u[k + 1], s.faccld1u[k + 1], s.faccmb1u[k + 1], s.faccmb2u[k + 1],
-                             s.facclr2u[k + 1], s.faccld2u[k + 1]};
-        for (int f = 0; f < 6; ++f) { r[R_FACD + f] = fd[f]; r[R_FACU + f] = fu[f]; }
-    }
-    if (tid < 16) {
-        blk[H_PKLAY0 + tid] = s.pklay[0][tid];
-        blk[H_SECDIFF + tid] = s.secdiff[tid];
-        blk[H_SEMISS + tid] = s.semiss[tid];
-    }
-    if (tid == 0) {
-        int fp64 = 0;
-        for (int k0 = 0; k0 < nlay; ++k0)
-            fp64 |= s.delp[k0] < LW3_THIN && s.cldfrc[k0 + 1] > 1.0e-6f;
-        blk[H_FP64] = __int_as_float(fp64);
-        if (fp64) fp64list[1 + atomicAdd(fp64list, 1)] = blockIdx.x;    // the chunk's list for lw3_fp64_kernel
-    }
+    lw_setup_core<float, LW3_OPT_THREADS>(
+        s, a, col, tid,
+        [&](int g, int k0, P2 tg, P2 fr) {
+            *reinterpret_cast<float2*>(row + k0 * LW3_ROW + g) = make_float2(tg.x, tg.y);
+            *reinterpret_cast<float2*>(row + k0 * LW3_ROW + LW_NGPT + g) = make_float2(fr.x, fr.y);
+        },
+        // the records' Planck functions and cloud depths, and the head
+        [&]() {
+            for (int i = tid; i < nlay * 64; i += LW3_OPT_THREADS) {
+                const int k = 1 + (i >> 6), w = i & 63, b = w & 15;
+                aux[(k - 1) * LW3_ROW + w] = w < 16 ? s.pklay[k][b] : w < 32 ? s.pklev[k][b] : w < 48 ? s.pklev[k - 1][b] : s.taucld[b][k - 1];
+            }
+            if (tid < 16) {
+                blk[H_PKLAY0 + tid] = s.pklay[0][tid];
+                blk[H_SECDIFF + tid] = s.secdiff[tid];
+                blk[H_SEMISS + tid] = s.semiss[tid];
+            }
+        },
+        // the records' cloud fractions and overlap factors, and the float64 flag
+        [&](int lane) {
+            bool thin = false;
+            for (int k = 1 + lane; k <= nlay; k += 32) {
+                float* r = aux + (k - 1) * LW3_ROW;
+                r[R_CLDFRC] = s.cldfrc[k];
+                r[R_LSTU] = __int_as_float(s.lstu[k]);
+                r[R_LSTD] = __int_as_float(s.lstd[k]);
+                const float fd[6] = {s.facclr1d[k - 1], s.faccld1d[k - 1], s.faccmb1d[k - 1], s.faccmb2d[k - 1],
+                                     s.facclr2d[k - 1], s.faccld2d[k - 1]};
+                const float fu[6] = {s.facclr1u[k + 1], s.faccld1u[k + 1], s.faccmb1u[k + 1], s.faccmb2u[k + 1],
+                                     s.facclr2u[k + 1], s.faccld2u[k + 1]};
+                for (int f = 0; f < 6; ++f) { r[R_FACD + f] = fd[f]; r[R_FACU + f] = fu[f]; }
+                thin = thin || (s.delp[k - 1] < LW3_THIN && s.cldfrc[k] > 1.0e-6f);
+            }
+            // the chunk's list for lw3_fp64_kernel
+            if (__any_sync(0xffffffffu, thin) && lane == 0) fp64list[1 + atomicAdd(fp64list, 1)] = blockIdx.x;
+        });
 }
 
 // The flagged columns of a chunk in float64: list = [count, chunk-local columns...] appended by the optics
