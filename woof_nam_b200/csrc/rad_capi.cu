@@ -636,7 +636,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 const int64_t swc = sw4_chunk(cfg);
                 const size_t smem0 = sw4_gas_smem(any_aer);
                 const size_t smem1 = sw4_rt_smem(any_aer);    // the image without taug (read from the image)
-                const size_t smem2 = (size_t)(SW2_NSEG - 1) * 4 * SW2_THREADS * sizeof(float);
+                const size_t smem2 = (size_t)(SW2_NSEG - 1) * 2 * SW4_SWEEP_THREADS * sizeof(float2);
                 const size_t bb = sw4_block_bytes(nlay);
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_gas_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0));
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_rt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
@@ -652,11 +652,11 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                     sw4_fix_kernel<<<(unsigned)(SW4_FIX_MINB * h->nsm), SW4_FIX_THREADS, smem1, st>>>(
                         bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, h->d_sw4item);
                     if (diag_sw) {
-                        sw4_sweep_kernel<true><<<(unsigned)nc, SW2_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
+                        sw4_sweep_kernel<true><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
                                                                                         h->d_sw4, bb, h->d_swpg);
                         k_sw_diag<<<(unsigned)((nc + 3) / 4), 128, 0, st>>>(bt, (int)d0, (int)nc, h->d_sw4, bb, h->d_swpg, dout);
                     } else {
-                        sw4_sweep_kernel<false><<<(unsigned)nc, SW2_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
+                        sw4_sweep_kernel<false><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
                                                                                          h->d_sw4, bb);
                     }
                 }

@@ -38,7 +38,9 @@ constexpr int SW4_LAYER = SW4_FIELDS * SW_NGPT;     // floats per layer and pass
 // per SM against 160 x 5, 192 x 4, 256 x 3, 320 x 2, 384 x 2 (SW +0.2 to +9.8 %).
 constexpr int SW4_RT_THREADS = 128;                 // threads of an R/T CTA
 constexpr int SW4_OPT_MINB = 6;                     // CTAs per SM the R/T kernel is compiled for (4: 4.62, 5: 4.41, 6: 4.30 ms)
-constexpr int SW4_SWEEP_MINB = 6;                   // ... and the sweep kernel
+constexpr int SW4_SWEEP_WARPS = 4;                   // warps of a sweep CTA (one column)
+constexpr int SW4_SWEEP_THREADS = 32 * SW4_SWEEP_WARPS;
+constexpr int SW4_SWEEP_MINB = 5;                    // CTAs per SM it is compiled for (4: 5.64, 5: 5.06, 6: 5.89, 7: 6.78 ms)
 constexpr int SW4_GAS_THREADS = 128;               // threads of a gas-optics CTA
 constexpr int SW4_GAS_MINB = 6;                     // ... and the gas-optics kernel
 constexpr bool SW4_L2PF = true;                     // the sweeps prefetch the R/T rows two segments ahead into L2
@@ -523,44 +525,83 @@ sw4_fix_kernel(const __grid_constant__ SwBatch bt, int any_aer, const float* ex,
 }
 
 // Per-g-point level fluxes of one sunlit column for swrad's optional outputs (DIAG sweeps):
-// [nlay + 1][SW4_PGQ][SW_NGPT] floats at level L (surface first), each x zsolar: up total, down total, up clear,
-// down clear, net (down - up) total, net clear.
+// [nlay + 1][SW4_PGQ][SW_NGPT] floats at level L (surface first), each x zsolar: up, down and net (down - up) of the clear
+// pass (q 0..2), then of the cloudy pass (q 3..5, written for a cloudy column).
 constexpr int SW4_PGQ = 6;
 __host__ __device__ constexpr int64_t sw4_pg_floats(int nlay) { return (int64_t)(nlay + 1) * SW4_PGQ * SW_NGPT; }
 
-// One level of the DIAG profile of g-point g (see sw4_pg_floats): clear fluxes fu / fd, cloudy-pass fuo / fdo,
-// pass weights w0 / w1 and the sweep's net total.
-__device__ __forceinline__ void sw4_pg_level(float* pg, int L, int g, float zsolar, bool cloudy, double w0, double w1,
-                                             float fu, float fd, float fuo, float fdo, double net)
+// One level of the DIAG profile of the pair g, g + 1 in one pass (see sw4_pg_floats).
+__device__ __forceinline__ void sw4_pg_level(float* pg, int L, int g, int pass, F2 zsolar, F2 fu, F2 fd)
 {
-    const double zs = (double)zsolar;
-    float* p = pg + (size_t)L * SW4_PGQ * SW_NGPT + g;
-    p[0] = (float)(zs * (cloudy ? w0 * fu + w1 * fuo : (double)fu));
-    p[SW_NGPT] = (float)(zs * (cloudy ? w0 * fd + w1 * fdo : (double)fd));
-    p[2 * SW_NGPT] = (float)(zs * fu);
-    p[3 * SW_NGPT] = (float)(zs * fd);
-    p[4 * SW_NGPT] = (float)(zs * net);
-    p[5 * SW_NGPT] = (float)(zs * ((double)fd - (double)fu));
+    float* p = pg + ((size_t)L * SW4_PGQ + 3 * pass) * SW_NGPT + g;
+    auto one = [&](float* q, double z, double u, double d) {
+        q[0] = (float)(z * u);
+        q[SW_NGPT] = (float)(z * d);
+        q[2 * SW_NGPT] = (float)(z * (d - u));
+    };
+    one(p, zsolar.x, fu.x, fd.x);
+    one(p + 1, zsolar.y, fu.y, fd.y);
 }
 
-// The adding method of one sunlit column from its block (sw2_column phase C with the R/T read instead of
-// formed; the same operations in the same order).
+// The steps of the adding method (sw2_up, sw2_flux, sw2_down) on a pair of g-points.
+__device__ __forceinline__ void sw4_up(const SwRT2& L, F2& ub, F2& ud)
+{
+    const F2 den = rcp2(nma2(ud, L.rd, f2(1.0f)));
+    ub = fma2(L.td * fma2(L.tb - L.e3, ud, L.e3 * ub), den, L.rb);
+    ud = fma2(L.td * L.td * ud, den, L.rd);
+}
+__device__ __forceinline__ void sw4_flux(F2 ub, F2 ud, F2 tdn, F2 rdn, F2 tdb, F2& fu, F2& fd)
+{
+    const F2 den = rcp2(nma2(rdn, ud, f2(1.0f))), dif = tdn - tdb, bu = tdb * ub;
+    fu = fma2(dif, ud, bu) * den;
+    fd = fma2(fma2(bu, rdn, dif), den, tdb);
+}
+__device__ __forceinline__ void sw4_down(const SwRT2& L, F2& tdn, F2& rdn, F2& tdb)
+{
+    const F2 den = rcp2(nma2(L.rd, rdn, f2(1.0f)));
+    tdn = fma2(L.td * fma2(tdb * L.rb, rdn, tdn - tdb), den, tdb * L.tb);
+    rdn = fma2(L.td * L.td * rdn, den, L.rd);
+    tdb = L.e3 * tdb;
+}
+
+// Sums of four doubles over the warp: lane 8 j holds v[j]'s (a fixed tree: the four values are folded into the lanes as
+// the sums halve, 12 shuffles and 6 additions instead of four warp_sum's 40 and 20).
+__device__ __forceinline__ double warp_sum4(const double* v, int lane)
+{
+    const bool h = lane & 16, q = lane & 8;
+    double a = h ? v[2] : v[0], b = h ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, h ? v[1] : v[3], 16);
+    double c = q ? b : a;
+    c += __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
+// The adding method of one sunlit column from its block (sw2_column phase C with the R/T read instead of formed).  Four
+// warps per column: warps 0 and 1 run the clear pass, warps 2 and 3 the cloudy one (idle in a cloudless column), a lane
+// per pair of g-points (28 lanes each), so a pass's chain of layers is not lengthened by the other's.  Bound: the latency
+// of a segment's rows and of the recurrence (2.8 TB/s of R/T rows read).  Measured per 131,072 columns (65,536 sunlit):
+// 6.47 ms with both passes and one g-point per lane at 80 registers; the same with pairs and both passes in two warps
+// (168 registers, 6 CTAs per SM: latency); 5.06 ms with the passes in warps of their own and the four levels of a segment
+// summed together.
 template <bool DIAG = false>
-__global__ void __launch_bounds__(SW2_THREADS, SW4_SWEEP_MINB)
+__global__ void __launch_bounds__(SW4_SWEEP_THREADS, SW4_SWEEP_MINB)
 sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int* err, int d0, int nc, const unsigned char* scr,
                  size_t blk_bytes, float* __restrict__ pg = nullptr)
 {
-    extern __shared__ __align__(16) float ckpt[];                  // [(nseg - 1) x 4][SW2_THREADS]
+    extern __shared__ __align__(16) float2 ckpt[];                 // [(nseg - 1) x 2][SW4_SWEEP_THREADS]
     __shared__ __align__(16) Sw4Hdr H;
-    __shared__ double fn[SW2_WARPS][NLAY_MAX + 2];
-    __shared__ double scs[SW2_WARPS][18];
+    __shared__ double fn[SW4_SWEEP_WARPS][NLAY_MAX + SW2_SEG + 1];
+    __shared__ double scs[SW4_SWEEP_WARPS][9];
     const int i = (int)blockIdx.x;
     const int d = d0 + i;
     if (i >= nc || d >= *bt.req[0].nday) return;
     const int64_t gcol = bt.req[0].daycol[d];
     const int rq = bt.find(gcol);
     const SwIn& a = bt.req[rq];
-    const int nlay = a.nlay, nlp1 = nlay + 1;
+    const int nlay = a.nlay;
     if (nlay > NLAY_MAX) return;                                   // flagged by the optics kernel
     const int64_t N = a.ncol;
     const int64_t col = gcol - bt.off[rq];
@@ -569,175 +610,153 @@ sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int* err, int d0, int nc, c
     {
         const int4* src = reinterpret_cast<const int4*>(blk);
         int4* dst = reinterpret_cast<int4*>(&H);
-        for (int j = tid; j < (int)(sizeof(Sw4Hdr) / 16); j += SW2_THREADS) dst[j] = __ldg(src + j);
+        for (int j = tid; j < (int)(sizeof(Sw4Hdr) / 16); j += SW4_SWEEP_THREADS) dst[j] = __ldg(src + j);
     }
     __syncthreads();
     const float* rtc = reinterpret_cast<const float*>(blk + sw4_hdr_bytes());
     const float* rto = rtc + (size_t)nlay * SW4_LAYER;
     if (DIAG) pg += (int64_t)i * sw4_pg_floats(nlay);
     const int warp = tid >> 5, lane = tid & 31;
-    bool act;
-    const int g = sw2_lane_g(tid, act);
-    int ib0 = 0;
-    while (g >= c_sw_ns[ib0 + 1]) ++ib0;
+    constexpr int LANES = SW_NGPT / 4;
+    const int pass = warp >> 1;                                    // 0 clear, 1 cloudy
+    const bool act = lane < LANES;                                 // idle lanes mirror the warp's last pair
+    const int g = 2 * ((warp & 1) * LANES + min(lane, LANES - 1));
+    const int ib0 = c_sw_band[g];
     const int ibd = ib0 == 8 ? 0 : ((ib0 >= 9 && ib0 <= 12) ? 2 : 1);   // idxsfc
     const bool mc = a.mask != nullptr;
     const bool cloudy = H.cloudy != 0, clr5 = H.clr5 != 0;
-    const float zsolar = act ? H.zsolar[g] : 0.0f;
-    const float ab = ibd ? H.albbm[ibd - 1] : 0.5f * (H.albbm[0] + H.albbm[1]);
-    const float ad = ibd ? H.albdf[ibd - 1] : 0.5f * (H.albdf[0] + H.albdf[1]);
-    const int nseg = (nlay + SW2_SEG - 1) / SW2_SEG;
-    float* ck = ckpt + tid;
-    auto CK = [&](int sg, int q) -> float& { return ck[((sg - 1) * 4 + q) * SW2_THREADS]; };
-    // R/T of layer k0, both passes (transparent padding above the model top)
-    auto load = [&](int k0, SwLayerRT& c, SwLayerRT& o) {
-        if (k0 >= nlay) {
-            c.rb = 0; c.rd = 0; c.tb = 1; c.td = 1; c.e3 = 1; c.e4 = 1;
-            o = c;
-            return;
-        }
-        const float* p = rtc + (size_t)k0 * SW4_LAYER + g;
-        c.rb = __ldg(p); c.rd = __ldg(p + SW_NGPT); c.tb = __ldg(p + 2 * SW_NGPT); c.td = __ldg(p + 3 * SW_NGPT);
-        c.e3 = __ldg(p + 4 * SW_NGPT); c.e4 = clr5 ? c.e3 : __ldg(p + 5 * SW_NGPT);
-        const int sl = H.slot[k0];
-        if (cloudy && sl >= 0) {
-            const float* q = rto + (size_t)sl * SW4_LAYER + g;
-            o.rb = __ldg(q); o.rd = __ldg(q + SW_NGPT); o.tb = __ldg(q + 2 * SW_NGPT); o.td = __ldg(q + 3 * SW_NGPT);
-            o.e3 = __ldg(q + 4 * SW_NGPT); o.e4 = __ldg(q + 5 * SW_NGPT);
-        } else {
-            o = c;
-        }
-    };
-    // The R/T rows of segment sg into L2 ahead of its loads (thread 0, one bulk prefetch per pass): the clear rows
-    // of its layers and the cloudy rows of their slots, each a contiguous run inside the column's block.
-    auto prefetch = [&](int sg) {
-        if (!SW4_L2PF || tid != 0 || sg < 0 || sg >= nseg) return;
-        const int k0 = sg * SW2_SEG, k1 = min(nlay, k0 + SW2_SEG);
-        if (k0 >= k1) return;
-        l2_prefetch(rtc + (size_t)k0 * SW4_LAYER, (uint32_t)((k1 - k0) * SW4_LAYER * sizeof(float)));
-        if (!cloudy) return;
-        int s0 = -1, s1 = -1;
-        for (int k = k0; k < k1; ++k)
-            if (H.slot[k] >= 0) { if (s0 < 0) s0 = H.slot[k]; s1 = H.slot[k]; }
-        if (s0 >= 0) l2_prefetch(rto + (size_t)s0 * SW4_LAYER, (uint32_t)((s1 - s0 + 1) * SW4_LAYER * sizeof(float)));
-    };
-    // ---- upward sweep: reflectances of the atmosphere below each level, clear (c) and cloudy (o) passes
-    float ubc = ab, udc = ad, ubo = ab, udo = ad;
-    prefetch(0);
-    prefetch(1);
-    for (int sg = 0; sg < nseg; ++sg) {
-        prefetch(sg + 2);
-        if (sg > 0) { CK(sg, 0) = ubc; CK(sg, 1) = udc; CK(sg, 2) = ubo; CK(sg, 3) = udo; }
-        SwLayerRT Lc[SW2_SEG], Lo[SW2_SEG];
-#pragma unroll
-        for (int j = 0; j < SW2_SEG; ++j) load(sg * SW2_SEG + j, Lc[j], Lo[j]);
-#pragma unroll
-        for (int j = 0; j < SW2_SEG; ++j) {
-            sw2_up(Lc[j], ubc, udc);
-            if (cloudy) sw2_up(Lo[j], ubo, udo);
-        }
-    }
-    // ---- downward sweep, segment by segment from the top: the segment's R/T again, its upward states from
-    // the checkpoint, then the walk down through it
     const double w0 = cloudy ? (mc ? 0.0 : (double)H.zcf0) : 1.0, w1 = cloudy ? (mc ? 1.0 : (double)H.zcf1) : 0.0;
-    float tdnc = 1, rdnc = 0, tdbc = 1, tdbc0 = 1, tdno = 1, rdno = 0, tdbo = 1, tdbo0 = 1;
-    float toa_c = 0, toa_o = 0;
-    prefetch(nseg - 2);
-    for (int sg = nseg - 1; sg >= 0; --sg) {
-        prefetch(sg - 2);
-        SwLayerRT Lc[SW2_SEG], Lo[SW2_SEG];
-        float zubc[SW2_SEG + 1], zudc[SW2_SEG + 1], zubo[SW2_SEG + 1], zudo[SW2_SEG + 1];
-        zubc[0] = sg ? CK(sg, 0) : ab;
-        zudc[0] = sg ? CK(sg, 1) : ad;
-        zubo[0] = sg ? CK(sg, 2) : ab;
-        zudo[0] = sg ? CK(sg, 3) : ad;
-#pragma unroll
-        for (int j = 0; j < SW2_SEG; ++j) load(sg * SW2_SEG + j, Lc[j], Lo[j]);
-        float e4c = 1, e4o = 1;
-#pragma unroll
-        for (int j = 0; j < SW2_SEG; ++j) {
-            e4c = e4c * Lc[j].e4;
-            if (cloudy) e4o = e4o * Lo[j].e4;
-            zubc[j + 1] = zubc[j]; zudc[j + 1] = zudc[j];
-            sw2_up(Lc[j], zubc[j + 1], zudc[j + 1]);
-            if (cloudy) {
-                zubo[j + 1] = zubo[j]; zudo[j + 1] = zudo[j];
-                sw2_up(Lo[j], zubo[j + 1], zudo[j + 1]);
+    const int nseg = (nlay + SW2_SEG - 1) / SW2_SEG;
+    if (pass == 0 || cloudy) {
+        const F2 zsolar = act ? F2{H.zsolar[g], H.zsolar[g + 1]} : f2(0.0f);
+        const F2 ab = f2(ibd ? H.albbm[ibd - 1] : 0.5f * (H.albbm[0] + H.albbm[1]));
+        const F2 ad = f2(ibd ? H.albdf[ibd - 1] : 0.5f * (H.albdf[0] + H.albdf[1]));
+        float2* ck = ckpt + tid;
+        auto save = [&](int sg, int q, F2 v) { ck[((sg - 1) * 2 + q) * SW4_SWEEP_THREADS] = make_float2(v.x, v.y); };
+        auto saved = [&](int sg, int q) { const float2 v = ck[((sg - 1) * 2 + q) * SW4_SWEEP_THREADS]; return F2{v.x, v.y}; };
+        auto ld2 = [](const float* p) { const float2 v = __ldg(reinterpret_cast<const float2*>(p)); return F2{v.x, v.y}; };
+        // R/T of layer k0 in this warp's pass (transparent padding above the model top)
+        auto load = [&](int k0, SwRT2& c) {
+            if (k0 >= nlay) {
+                c.rb = c.rd = f2(0.0f);
+                c.tb = c.td = c.e3 = c.e4 = f2(1.0f);
+                return;
             }
-        }
-#pragma unroll
-        for (int j = SW2_SEG - 1; j >= 0; --j) {
-            const int lev = sg * SW2_SEG + j + 2;        // level above layer j (1 = surface)
-            if (lev <= nlp1) {
-                float fu, fd, fuo = 0, fdo = 0;
-                sw2_flux(zubc[j + 1], zudc[j + 1], tdnc, rdnc, tdbc, fu, fd);
-                double net = w0 * ((double)fd - (double)fu);
-                if (lev == nlp1) toa_c = fu;
-                if (cloudy) {
-                    sw2_flux(zubo[j + 1], zudo[j + 1], tdno, rdno, tdbo, fuo, fdo);
-                    net += w1 * ((double)fdo - (double)fuo);
-                    if (lev == nlp1) toa_o = fuo;
-                }
-                const double v = warp_sum(act ? (double)zsolar * net : 0.0);
-                if (lane == 0) fn[warp][lev - 1] = v;
-                if (DIAG && act) sw4_pg_level(pg, lev - 1, g, zsolar, cloudy, w0, w1, fu, fd, fuo, fdo, net);
+            const int sl = pass ? (int)H.slot[k0] : -1;
+            const float* p = (sl >= 0 ? rto + (size_t)sl * SW4_LAYER : rtc + (size_t)k0 * SW4_LAYER) + g;
+            c.rb = ld2(p); c.rd = ld2(p + SW_NGPT); c.tb = ld2(p + 2 * SW_NGPT); c.td = ld2(p + 3 * SW_NGPT);
+            c.e3 = ld2(p + 4 * SW_NGPT);
+            c.e4 = clr5 && sl < 0 ? c.e3 : ld2(p + 5 * SW_NGPT);
+        };
+        // The R/T rows of segment sg into L2 ahead of its loads (one bulk prefetch per pass by its first thread): the
+        // clear rows of its layers, the cloudy rows of their slots, each a contiguous run inside the column's block.
+        auto prefetch = [&](int sg) {
+            if (!SW4_L2PF || (tid & 63) != 0 || sg < 0 || sg >= nseg) return;
+            const int k0 = sg * SW2_SEG, k1 = min(nlay, k0 + SW2_SEG);
+            if (pass == 0) {
+                l2_prefetch(rtc + (size_t)k0 * SW4_LAYER, (uint32_t)((k1 - k0) * SW4_LAYER * sizeof(float)));
+                return;
             }
-            sw2_down(Lc[j], tdnc, rdnc, tdbc);
-            if (cloudy) sw2_down(Lo[j], tdno, rdno, tdbo);
-        }
-        tdbc0 = tdbc0 * e4c;
-        tdbo0 = tdbo0 * e4o;
-    }
-    // ---- surface level, the per-lane scalars (zero for idle lanes), column end and swrad_post
-    double scv[18];
+            int s0 = -1, s1 = -1;
+            for (int k = k0; k < k1; ++k)
+                if (H.slot[k] >= 0) { if (s0 < 0) s0 = H.slot[k]; s1 = H.slot[k]; }
+            if (s0 >= 0) l2_prefetch(rto + (size_t)s0 * SW4_LAYER, (uint32_t)((s1 - s0 + 1) * SW4_LAYER * sizeof(float)));
+        };
+        // ---- upward sweep: reflectances of the atmosphere below each level
+        F2 ub = ab, ud = ad;
+        prefetch(0);
+        prefetch(1);
+        for (int sg = 0; sg < nseg; ++sg) {
+            prefetch(sg + 2);
+            if (sg > 0) { save(sg, 0, ub); save(sg, 1, ud); }
+            SwRT2 L[SW2_SEG];
 #pragma unroll
-    for (int q = 0; q < 18; ++q) scv[q] = 0;
-    {
-        float fu, fd, fuo = 0, fdo = 0;
-        sw2_flux(ab, ad, tdnc, rdnc, tdbc, fu, fd);
-        double net = w0 * ((double)fd - (double)fu);
-        if (cloudy) {
-            sw2_flux(ab, ad, tdno, rdno, tdbo, fuo, fdo);
-            net += w1 * ((double)fdo - (double)fuo);
+            for (int j = 0; j < SW2_SEG; ++j) load(sg * SW2_SEG + j, L[j]);
+#pragma unroll
+            for (int j = 0; j < SW2_SEG; ++j) sw4_up(L[j], ub, ud);
         }
-        const double v = warp_sum(act ? (double)zsolar * net : 0.0);
+        // ---- downward sweep, segment by segment from the top: the segment's R/T again, its upward states from the
+        // checkpoint, then the walk down through it
+        const double wp = pass ? w1 : w0, zx = wp * (double)zsolar.x, zy = wp * (double)zsolar.y;   // 0 in idle lanes
+        auto net = [&](F2 fu, F2 fd) { return zx * ((double)fd.x - (double)fu.x) + zy * ((double)fd.y - (double)fu.y); };
+        F2 tdn = f2(1.0f), rdn = f2(0.0f), tdb = f2(1.0f), tdb0 = f2(1.0f), toa = f2(0.0f);
+        prefetch(nseg - 2);
+        for (int sg = nseg - 1; sg >= 0; --sg) {
+            prefetch(sg - 2);
+            SwRT2 L[SW2_SEG];
+            F2 zub[SW2_SEG + 1], zud[SW2_SEG + 1];
+            zub[0] = sg ? saved(sg, 0) : ab;
+            zud[0] = sg ? saved(sg, 1) : ad;
+#pragma unroll
+            for (int j = 0; j < SW2_SEG; ++j) load(sg * SW2_SEG + j, L[j]);
+            F2 e4 = f2(1.0f);
+#pragma unroll
+            for (int j = 0; j < SW2_SEG; ++j) {
+                e4 = e4 * L[j].e4;
+                zub[j + 1] = zub[j]; zud[j + 1] = zud[j];
+                sw4_up(L[j], zub[j + 1], zud[j + 1]);
+            }
+            double nv[SW2_SEG];
+#pragma unroll
+            for (int j = SW2_SEG - 1; j >= 0; --j) {
+                const int lev = sg * SW2_SEG + j + 1;    // level above layer j (0 = surface); past the top: not used
+                F2 fu, fd;
+                sw4_flux(zub[j + 1], zud[j + 1], tdn, rdn, tdb, fu, fd);
+                if (lev == nlay) toa = fu;
+                nv[j] = net(fu, fd);
+                if (DIAG && act && lev <= nlay) sw4_pg_level(pg, lev, g, pass, zsolar, fu, fd);
+                sw4_down(L[j], tdn, rdn, tdb);
+            }
+            static_assert(SW2_SEG == 4, "warp_sum4 takes a segment's four levels");
+            const double v = warp_sum4(nv, lane);
+            if ((lane & 7) == 0) fn[warp][sg * SW2_SEG + (lane >> 3) + 1] = v;
+            tdb0 = tdb0 * e4;
+        }
+        // ---- surface level, the per-lane scalars (zero for idle lanes)
+        double o[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) o[q] = 0;
+        F2 fu, fd;
+        sw4_flux(ab, ad, tdn, rdn, tdb, fu, fd);
+        const double v = warp_sum(net(fu, fd));
         if (lane == 0) fn[warp][0] = v;
-        if (DIAG && act) sw4_pg_level(pg, 0, g, zsolar, cloudy, w0, w1, fu, fd, fuo, fdo, net);
+        if (DIAG && act) sw4_pg_level(pg, 0, g, pass, zsolar, fu, fd);
         if (act) {
-            const double zs = (double)zsolar;
             // slots: 0 toa up, 1 sfc up, 2 sfc dn, 3 uv-b, 4 nir beam, 5 nir diffuse, 6 vis beam, 7 vis diffuse, 8 toa down
-            auto fill = [&](double* o, float tu, float su, float sd, float sdir) {
-                o[0] = zs * (double)tu;
-                o[1] = zs * (double)su;
-                o[2] = zs * (double)sd;
-                o[3] = ib0 == 11 ? zs * (double)sd : 0.0;
-                const double zb1 = (double)(zsolar * sdir), zb2 = (double)(zsolar * (sd - sdir));
-                if (ibd == 1) { o[4] = zb1; o[5] = zb2; }
-                else if (ibd == 2) { o[6] = zb1; o[7] = zb2; }
-                else { o[4] = 0.5 * zb1; o[5] = 0.5 * zb2; o[6] = 0.5 * zb1; o[7] = 0.5 * zb2; }
-                o[8] = zs;
+            auto fill = [&](float z, float tu, float su, float sd, float sdir) {
+                const double zs = (double)z;
+                o[0] += zs * (double)tu;
+                o[1] += zs * (double)su;
+                o[2] += zs * (double)sd;
+                o[3] += ib0 == 11 ? zs * (double)sd : 0.0;
+                const double zb1 = (double)(z * sdir), zb2 = (double)(z * (sd - sdir));
+                if (ibd == 1) { o[4] += zb1; o[5] += zb2; }
+                else if (ibd == 2) { o[6] += zb1; o[7] += zb2; }
+                else { o[4] += 0.5 * zb1; o[5] += 0.5 * zb2; o[6] += 0.5 * zb1; o[7] += 0.5 * zb2; }
+                o[8] += zs;
             };
-            fill(scv, toa_c, fu, fd, tdbc0);
-            if (cloudy) fill(scv + 9, toa_o, fuo, fdo, tdbo0);
+            fill(zsolar.x, toa.x, fu.x, fd.x, tdb0.x);
+            fill(zsolar.y, toa.y, fu.y, fd.y, tdb0.y);
         }
-    }
 #pragma unroll
-    for (int q = 0; q < 18; ++q) {
-        const double v = warp_sum(scv[q]);
-        if (lane == 0) scs[warp][q] = v;
+        for (int q = 0; q < 9; ++q) {
+            const double t = warp_sum(o[q]);
+            if (lane == 0) scs[warp][q] = t;
+        }
     }
     __syncthreads();
+    // ---- column end and swrad_post
     auto tot = [&](double clr, double cld) { return cloudy ? w1 * cld + w0 * clr : clr; };
-    for (int k = tid; k < nlay; k += SW2_THREADS) {
-        double f0 = 0, f1 = 0;
-        for (int w = 0; w < SW2_WARPS; ++w) { f0 += fn[w][k]; f1 += fn[w][k + 1]; }
+    for (int k = tid; k < nlay; k += SW4_SWEEP_THREADS) {
+        double f0 = fn[0][k] + fn[1][k], f1 = fn[0][k + 1] + fn[1][k + 1];
+        if (cloudy) { f0 += fn[2][k] + fn[3][k]; f1 += fn[2][k + 1] + fn[3][k + 1]; }
         a.htsw[(size_t)(nlay - 1 - k) * N + col] = (float)((f1 - f0) * H.rdelp[k]);
     }
     if (tid == 0) {
         double c[9], t[9];
         for (int q = 0; q < 9; ++q) {
-            c[q] = 0; t[q] = 0;
-            for (int w = 0; w < SW2_WARPS; ++w) { c[q] += scs[w][q]; t[q] += scs[w][9 + q]; }
+            c[q] = scs[0][q] + scs[1][q];
+            t[q] = cloudy ? scs[2][q] + scs[3][q] : 0.0;
         }
         a.topfsw[col] = (float)tot(c[0], t[0]);
         a.topfsw[N + col] = (float)c[8];
@@ -787,11 +806,15 @@ __global__ void __launch_bounds__(128) k_sw_diag(const __grid_constant__ SwBatch
         for (int g = g0; g < g1; ++g) v += (double)p[((size_t)L * SW4_PGQ + f) * SW_NGPT + g];
         return v;
     };
+    // fields f of the clear pass and the total sky (weights as in the sweeps)
+    const bool cloudy = H.cloudy != 0, mc = a.mask != nullptr;
+    const double w0 = cloudy ? (mc ? 0.0 : (double)H.zcf0) : 1.0, w1 = cloudy ? (mc ? 1.0 : (double)H.zcf1) : 0.0;
+    auto T = [&](int L, int f) { return cloudy ? w0 * S(L, f) + w1 * S(L, 3 + f) : S(L, f); };
     if (q < 14) {
         if (htswb) {
-            double f0 = S(0, 4);
+            double f0 = T(0, 2);
             for (int k0 = 0; k0 < nlay; ++k0) {
-                const double f1 = S(k0 + 1, 4);
+                const double f1 = T(k0 + 1, 2);
                 htswb[((size_t)q * nlay + (nlay - 1 - k0)) * N + col] = (float)((f1 - f0) * H.rdelp[k0]);
                 f0 = f1;
             }
@@ -799,16 +822,16 @@ __global__ void __launch_bounds__(128) k_sw_diag(const __grid_constant__ SwBatch
         return;
     }
     if (hsw0) {
-        double f0 = S(0, 5);
+        double f0 = S(0, 2);
         for (int k0 = 0; k0 < nlay; ++k0) {
-            const double f1 = S(k0 + 1, 5);
+            const double f1 = S(k0 + 1, 2);
             hsw0[(size_t)(nlay - 1 - k0) * N + col] = (float)((f1 - f0) * H.rdelp[k0]);
             f0 = f1;
         }
     }
     if (flx)
         for (int L = 0; L < nlp1; ++L)
-            for (int f = 0; f < 4; ++f) flx[((size_t)f * nlp1 + (nlp1 - 1 - L)) * N + col] = (float)S(L, f);
+            for (int f = 0; f < 4; ++f) flx[((size_t)f * nlp1 + (nlp1 - 1 - L)) * N + col] = (float)(f < 2 ? T(L, f) : S(L, f - 2));
 }
 
 }  // namespace rad
