@@ -546,11 +546,11 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 sweep<<<g2, LW3_SWEEP_WARPS * 32, lw3_sweep_smem(), st>>>(bt, c0, nc, h->d_lw3, fl, pg);
                 h->launches += 2;
                 if (!mc) {
-                    lw3_fp64_kernel<<<(unsigned)h->nsm, LW_THREADS, smemd, st>>>(bt, c0, h->d_lw3list, dl, h->d_err);
+                    lw3_fp64_kernel<<<(unsigned)h->nsm, LW3_FP64_THREADS, smemd, st>>>(bt, c0, h->d_lw3list, dl, h->d_err);
                     h->launches += 1;
                 }
                 if (diag_lw) {
-                    k_lw_diag<<<(unsigned)((nc + 3) / 4), 128, 0, st>>>(bt, c0, nc, pg, dout);
+                    k_lw_diag<<<(unsigned)nc, LW3_DIAG_WARPS * 32, 0, st>>>(bt, c0, pg, dout);
                     h->launches += 1;
                 }
             }
@@ -570,7 +570,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
             RAD_CUDA(h, cudaFuncSetAttribute((void*)lw3_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemd));
             RAD_CUDA(h, cudaMemsetAsync(sc.pos, 0, sizeof(int), st));
             lw2_column_kernel<R, false><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, sc.pos);
-            lw3_fp64_kernel<<<(unsigned)h->nsm, LW_THREADS, smemd, st>>>(bt, 0, sc.pos, dl, h->d_err);
+            lw3_fp64_kernel<<<(unsigned)h->nsm, LW3_FP64_THREADS, smemd, st>>>(bt, 0, sc.pos, dl, h->d_err);
             h->launches += 2;
         } else {
             lw_column_kernel<R><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err);
@@ -654,7 +654,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                     if (diag_sw) {
                         sw4_sweep_kernel<true><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
                                                                                         h->d_sw4, bb, h->d_swpg);
-                        k_sw_diag<<<(unsigned)((nc + 3) / 4), 128, 0, st>>>(bt, (int)d0, (int)nc, h->d_sw4, bb, h->d_swpg, dout);
+                        k_sw_diag<<<(unsigned)nc, SW4_DIAG_WARPS * 32, 0, st>>>(bt, (int)d0, h->d_sw4, bb, h->d_swpg, dout);
                     } else {
                         sw4_sweep_kernel<false><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
                                                                                          h->d_sw4, bb);

@@ -1082,7 +1082,7 @@ using LwBatch = ReqBatch<LwIn>;
 
 // The whole LW column gc (of the launch's concatenated column space) by one CTA: set-up, gas optics and the
 // rtrnmr sweeps (rtrn when a.rnd) with one g-point per thread.  R = double is the plain FP64 kernel.
-template <class R>
+template <class R, int NT = LW_THREADS>
 __device__ __forceinline__ void lw_column_body(const LwBatch& bt, const LwLut<R>& lut, int* err, int64_t gc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1097,7 +1097,8 @@ __device__ __forceinline__ void lw_column_body(const LwBatch& bt, const LwLut<R>
         if (tid == 0 && nlay > NLAY_MAX) atomicExch(err, RAD_DEV_NLAY);
         return;
     }
-    lw_setup<R, LW_THREADS>(s, a, col, tid);
+    lw_setup<R, NT>(s, a, col, tid);
+    if (tid < LW_THREADS) {                          // the sweeps take the first LW_WARPS warps
     const R eps = (R)1.0e-6f;
     const bool rnd = a.rnd != 0;
     // ---- phase C: rtrnmr (or rtrn) sweeps, one g-point per lane
@@ -1224,6 +1225,7 @@ __device__ __forceinline__ void lw_column_body(const LwBatch& bt, const LwLut<R>
         v0 = warp_sum(v0); v1 = warp_sum(v1);
         if (lane == 0) { s.scal[warp][0] = v0; s.scal[warp][1] = v1; }
     }
+    }
     __syncthreads();
     // ---- outputs: fluxes x flxfac, heating rates from float64 net-flux differences
     const double fluxfac = sizeof(R) == 4 ? (double)(float)(2.0 * 3.14159265358979323846 / 2.0 * 2.0) * 0.0 : 0.0;
@@ -1231,7 +1233,7 @@ __device__ __forceinline__ void lw_column_body(const LwBatch& bt, const LwLut<R>
     const double pi = 3.14159265358979323846;
     const double flxfac = 0.5 * (sizeof(R) == 4 ? (double)(float)((double)(float)pi * 2.0e4) : pi * 2.0e4);
     const double heatfac = sizeof(R) == 4 ? (double)(9.80665f * 1.0e-2f / 1.0046e3f) : 9.80665 * 1.0e-2 / 1.0046e3;
-    for (int k = tid; k < nlay; k += LW_THREADS) {
+    for (int k = tid; k < nlay; k += NT) {
         double fk = 0, fk1 = 0;
         for (int w = 0; w < LW_WARPS; ++w) { fk += s.fnet[w][k]; fk1 += s.fnet[w][k + 1]; }
         const double h = (fk - fk1) * flxfac * (heatfac / (double)s.delp[k]);

@@ -121,14 +121,16 @@ __global__ void __launch_bounds__(LW3_OPT_THREADS, LW3_OPT_MINB) lw3_optics_kern
 }
 
 // The flagged columns of a chunk in float64: list = [count, chunk-local columns...] appended by the optics
-// kernel; a grid of one CTA per SM walks it (the float64 layout's shared memory allows one CTA per SM).
-__global__ void __launch_bounds__(LW_THREADS) lw3_fp64_kernel(const __grid_constant__ LwBatch bt, int64_t c0,
+// kernel; a grid of one CTA per SM walks it (the float64 layout's shared memory allows one CTA per SM, so the CTA has
+// as many warps as its registers allow: the gas optics' tasks spread over them, the sweeps take the first five).
+constexpr int LW3_FP64_THREADS = 512;
+__global__ void __launch_bounds__(LW3_FP64_THREADS) lw3_fp64_kernel(const __grid_constant__ LwBatch bt, int64_t c0,
                                                               const int* __restrict__ list, LwLut<double> lutd,
                                                               int* err)
 {
     const int n = list[0];
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
-        lw_column_body<double>(bt, lutd, err, c0 + list[1 + i]);
+        lw_column_body<double, LW3_FP64_THREADS>(bt, lutd, err, c0 + list[1 + i]);
         __syncthreads();                          // shared memory is reused by the next column
     }
 }
@@ -453,21 +455,24 @@ lw3_sweep_kernel(const __grid_constant__ LwBatch bt, int64_t c0, int64_t nc, con
         lw3_sweep_column<OVR, DIAG>(W, lut, bt, c0, lc, scr, pg0, lane);
 }
 
-// lwrad's optional outputs of a chunk from the DIAG sweeps' profiles: one warp per column, lane q < 16 band q
-// (hlwb: htrb of rtrnmr's lhlwb block, from the band's per-layer changes), lane 16 the totals (lwflxprf, the
-// level fluxes; hlw0 from the clear-sky per-layer changes).  Sums over g-points in float64 in g order, times
-// flxfac; heating as the sweeps form htlw: -(dU + dD) flxfac heatfac / delp.
 // Optional-output pointers of a launch's requests: hlw0, hlwb, lwflxprf, hsw0, htswb, swflxprf (null = not wanted).
 struct DiagOuts {
     float* p[RAD_MAXREQ][6];
 };
-__global__ void __launch_bounds__(128) k_lw_diag(const __grid_constant__ LwBatch bt, int64_t c0, int64_t nc,
-                                                 const float* __restrict__ pg, const __grid_constant__ DiagOuts outs)
+// lwrad's optional outputs of a chunk from the DIAG sweeps' profiles: one CTA per column, a warp per level.  The level's
+// eight fields (4,480 contiguous bytes) go to shared memory, lane q of each half warp sums band q of one field at a time
+// over its g-points in float64, and the totals are summed over the bands' lanes: hlwb (htrb of rtrnmr's lhlwb block)
+// from a band's per-layer changes, hlw0 from the total clear-sky changes, lwflxprf the level fluxes x flxfac; heating as
+// the sweeps form htlw: -(dU + dD) flxfac heatfac / delp.  Bound: the profile's bytes (278 KB per column); 5.0 -> 0.57 ms
+// per 7,632 columns against one lane per band over strided words.
+constexpr int LW3_DIAG_WARPS = 4;
+__global__ void __launch_bounds__(LW3_DIAG_WARPS * 32) k_lw_diag(const __grid_constant__ LwBatch bt, int64_t c0,
+                                                                 const float* __restrict__ pg, const __grid_constant__ DiagOuts outs)
 {
-    const int64_t lc = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    const int q = threadIdx.x & 31;
-    if (lc >= nc || q > 16) return;
-    const int64_t gc = c0 + lc;
+    constexpr int ROW = LW3_PGQ * LW_NGPT;
+    __shared__ __align__(16) float sm[LW3_DIAG_WARPS][ROW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 15, half = lane >> 4;
+    const int64_t gc = c0 + blockIdx.x;
     const int rq = bt.find(gc);
     const LwIn& a = bt.req[rq];
     const int nlay = a.nlay;
@@ -476,28 +481,40 @@ __global__ void __launch_bounds__(128) k_lw_diag(const __grid_constant__ LwBatch
     float* hlw0 = outs.p[rq][0];
     float* hlwb = outs.p[rq][1];
     float* flx = outs.p[rq][2];
-    const float* p = pg + lc * lw3_pg_floats(nlay);
+    const float4* p = reinterpret_cast<const float4*>(pg + blockIdx.x * lw3_pg_floats(nlay));
     const double flxfac = 0.5 * 3.14159265358979323846 * 2.0e4;
     const double heatfac = 9.80665 * 1.0e-2 / 1.0046e3;
-    const int g0 = q < 16 ? c_lw_ns[q] : 0, g1 = q < 16 ? c_lw_ns[q + 1] : LW_NGPT;
-    auto S = [&](int L, int f) {
-        double v = 0.0;
-        for (int g = g0; g < g1; ++g) v += (double)p[((size_t)L * LW3_PGQ + f) * LW_NGPT + g];
-        return v;
-    };
-    for (int k = 1; k <= nlay; ++k) {
-        const int kin = nlay - k;   // top-first index of layer k
-        const double dl = (double)__ldg(a.plvl + (size_t)(kin + 1) * N + col) - (double)__ldg(a.plvl + (size_t)kin * N + col);
-        const double rf = flxfac * (heatfac / dl);
-        if (q < 16) {
-            if (hlwb) hlwb[((size_t)q * nlay + kin) * N + col] = (float)(-(S(k, 4) + S(k, 5)) * rf);
-        } else if (hlw0) {
-            hlw0[(size_t)kin * N + col] = (float)(-(S(k, 6) + S(k, 7)) * rf);
+    const int g0 = c_lw_ns[q], g1 = c_lw_ns[q + 1];
+    float* w = sm[warp];
+    for (int L = warp; L <= nlay; L += LW3_DIAG_WARPS) {
+        __syncwarp();                              // the previous level's sums have been read
+        for (int i = lane; i < ROW / 4; i += 32) reinterpret_cast<float4*>(w)[i] = __ldg(p + (size_t)L * (ROW / 4) + i);
+        __syncwarp();
+        double v[4], t[4];                         // band q of field 2 i + half, and the field's total
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* f = w + (2 * i + half) * LW_NGPT;
+            double x = 0.0;
+            for (int g = g0; g < g1; ++g) x += (double)f[g];
+            v[i] = x;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            t[i] = x;
+        }
+        const int kin = nlay - L;                  // top-first index of layer L and of level L
+        if (flx && q == 0) {
+            flx[((size_t)half * (nlay + 1) + kin) * N + col] = (float)(t[0] * flxfac);
+            flx[((size_t)(2 + half) * (nlay + 1) + kin) * N + col] = (float)(t[1] * flxfac);
+        }
+        const double db = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);      // fields 4 + 5 of the band
+        const double dc = t[3] + __shfl_xor_sync(0xffffffffu, t[3], 16);      // fields 6 + 7 in total
+        if (L > 0 && half == 0) {
+            const double dl = (double)__ldg(a.plvl + (size_t)(kin + 1) * N + col) - (double)__ldg(a.plvl + (size_t)kin * N + col);
+            const double rf = flxfac * (heatfac / dl);
+            if (hlwb) hlwb[((size_t)q * nlay + kin) * N + col] = (float)(-db * rf);
+            if (hlw0 && q == 0) hlw0[(size_t)kin * N + col] = (float)(-dc * rf);
         }
     }
-    if (q == 16 && flx)
-        for (int L = 0; L <= nlay; ++L)
-            for (int f = 0; f < 4; ++f) flx[((size_t)f * (nlay + 1) + (nlay - L)) * N + col] = (float)(S(L, f) * flxfac);
 }
 
 }  // namespace rad
