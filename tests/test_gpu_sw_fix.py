@@ -44,3 +44,25 @@ def test_resonant_columns(nlay, mode, tile):
     assert_within(outs[0], {k: ref[k] for k in outs[0]}, what=f"resonant columns, {nlay} layers, mode {mode}")
     for k in outs[0]:
         assert np.array_equal(outs[0][k], outs[1][k]), k
+
+
+def test_recompute_lists_and_their_overflow():
+    """A tile of 4,096 columns or more hands its float64 recomputes to sw4_exact_kernel through per-band lists (here
+    with more resonant g-points than the lists hold, so some stay with sw4_fix_kernel); smaller tiles run them all in
+    sw4_fix_kernel.  Same bits either way, and within tolerance of the oracle."""
+    import torch
+    from woof_nam_b200.solver import RadSolver
+    cols = _resonant(4600, 61, 2, 77)
+    outs = []
+    for t in (0, 4096, 1000):
+        s = RadSolver(parts="sw", sw_sweep_chunk=t)
+        out = s.solve(s.to_device(cols), cols.solcon)
+        torch.cuda.synchronize()
+        assert s.device_error() == 0
+        outs.append({k: v.cpu().numpy() for k, v in out.items()})
+    for o in outs[1:]:
+        for k in o:
+            assert np.array_equal(o[k], outs[0][k]), k
+    head = cols.slice(0, 256)
+    ref = oracle.solve(head, precision="double")
+    assert_within({k: outs[0][k][..., :256] for k in outs[0]}, {k: ref[k] for k in outs[0]}, what="recompute lists")

@@ -84,7 +84,7 @@ struct RadHandle {
     int64_t lwpg_cap = 0, swpg_cap = 0;            // columns they hold
     int4* d_sw4img = nullptr;                      // chunked SW: set-up and gas-optics images of one chunk's columns
     unsigned char* d_sw4 = nullptr;                // chunked SW: header and layer R/T of one chunk's columns
-    int* d_sw4item = nullptr;                      // chunked SW: work items of the float64 fix-up
+    void* d_sw4list = nullptr;                     // chunked SW: work lists of the float64 fix-up (Sw4Lists)
     int64_t sw4_cap = 0;                           // columns d_sw4 and d_sw4img hold
     float* d_aerf = nullptr;                       // aerosol band tables of the loaded month (AF_* offsets)
     int* d_aeri = nullptr;                         // their integer part (AI_* offsets)
@@ -391,14 +391,14 @@ int ensure_launch_scratch(RadHandle* h, int64_t ntot, int64_t ncmin)
         if (h->d_sw4) cudaFree(h->d_sw4);
         h->d_sw4 = nullptr;
         h->d_sw4img = nullptr;
-        h->d_sw4item = nullptr;
+        h->d_sw4list = nullptr;
         h->sw4_cap = 0;
         const int64_t need = std::min(swc, ntot);
         // blocks, images and the work list in one allocation
         const size_t blocks = (size_t)need * sw4_block_bytes(h->cfg.nlay), images = (size_t)need * sw4_image_bytes(true);
-        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4, blocks + images + (size_t)sw4_item_bytes(h->cfg.nlay, need)));
+        RAD_CUDA(h, cudaMalloc((void**)&h->d_sw4, blocks + images + (size_t)sw4_list_bytes(h->cfg.nlay, need)));
         h->d_sw4img = (int4*)(h->d_sw4 + blocks);
-        h->d_sw4item = (int*)(h->d_sw4 + blocks + images);
+        h->d_sw4list = h->d_sw4 + blocks + images;
         h->sw4_cap = need;
     }
     if (h->cfg.route == RAD_ROUTE_MCICA && ntot * h->cfg.nlay > h->mask_cap) {
@@ -643,14 +643,19 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_sweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_sweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+                Sw4Lists lists = sw4_lists(h->d_sw4list, nlay, h->sw4_cap);
+                if (std::min(swc, ntot) < SW4_EXACT_MIN) lists.cap = 0;
                 for (int64_t d0 = 0; d0 < ntot; d0 += swc) {
                     const int64_t nc = std::min(swc, ntot - d0);
                     sw4_gas_kernel<<<(unsigned)nc, SW4_GAS_THREADS, smem0, st>>>(bt, any_aer ? 1 : 0, h->d_err, (int)d0, h->d_sw4img,
-                                                                                 h->d_sw4item);
+                                                                                 lists);
                     sw4_rt_kernel<<<(unsigned)nc, SW4_RT_THREADS, smem1, st>>>(bt, any_aer ? 1 : 0, (int)d0, h->d_sw4img, h->d_sw4,
-                                                                               bb, h->d_sw4item);
+                                                                               bb, lists.head, lists.items);
                     sw4_fix_kernel<<<(unsigned)(SW4_FIX_MINB * h->nsm), SW4_FIX_THREADS, smem1, st>>>(
-                        bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, h->d_sw4item);
+                        bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, lists);
+                    if (lists.cap > 0)
+                        sw4_exact_kernel<<<(unsigned)(SW4_EXACT_MINB * h->nsm), SW4_EXACT_THREADS, 0, st>>>(
+                        bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, lists);
                     if (diag_sw) {
                         sw4_sweep_kernel<true><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
                                                                                         h->d_sw4, bb, h->d_swpg);
@@ -660,7 +665,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                                                                                          h->d_sw4, bb);
                     }
                 }
-                nlaunch = (diag_sw ? 5 : 4) * ((ntot + swc - 1) / swc);
+                nlaunch = (4 + (lists.cap > 0) + (diag_sw ? 1 : 0)) * ((ntot + swc - 1) / swc);
             } else {       // SW2_CTAS_PER_SM CTAs per SM walk the day list, each with its R/T store
                 RAD_CUDA(h, cudaFuncSetAttribute((void*)sw2_column_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 sw2_column_kernel<true><<<(unsigned)(SW2_CTAS_PER_SM * h->nsm), SW2_THREADS, smem, st>>>(
@@ -875,7 +880,7 @@ int64_t rad_workspace_bytes(const RadHandle* h, int64_t ncol)
         if (h->cfg.precision == RAD_PREC_MIXED && (h->cfg.parts & RAD_PART_SW) && swc <= 0) b += sw2_rt_bytes(h->nsm);
         if (swc > 0 && (h->cfg.parts & RAD_PART_SW))
             b += std::min(swc, ncol) * (int64_t)(sw4_block_bytes(h->cfg.nlay) + sw4_image_bytes(true)) +
-                 sw4_item_bytes(h->cfg.nlay, std::min(swc, ncol));
+                 sw4_list_bytes(h->cfg.nlay, std::min(swc, ncol));
     }
     return b;
 }

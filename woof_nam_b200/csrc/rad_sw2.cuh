@@ -414,6 +414,7 @@ struct SwExactCtx {
     double cz, snt;
     const double* exd;
     float wh, wf;
+    int* defer = nullptr;   // set where a recompute is due, instead of running it (the layer's R/T are then not final)
 };
 
 // The layer's clear (cloud = false) or cloud-mixture optical properties recomputed from the column
@@ -574,7 +575,8 @@ __device__ __forceinline__ void sw2_rt_mixed(float t0, float tabs, float s0, flo
         float am;
         exact = fabsf(sw2_expm_alt(zb4, ex, am) - sw_expm(zb4, ex, true)) * x.wf > 1.0f;
     }
-    if (exact) {
+    if (exact && x.defer) *x.defer = 1;
+    else if (exact) {
         double a, b, c, d, f3, f4;
         sw2_exact(x, k0, g, ib, cloud, a, b, c, d, f3, f4);
         rb = (float)a; rd = (float)b; tb = (float)c; td = (float)d; e3 = (float)f3; e4 = (float)f4;

@@ -68,12 +68,33 @@ __host__ __device__ constexpr size_t sw4_block_bytes(int nlay)
 {
     return sw4_queue_offset(nlay) + (size_t)nlay * SW_NGPT * sizeof(uint16_t);
 }
-// Work items of sw4_fix_kernel: at most SW4_FIX_THREADS queue entries of one column, {column of the tile,
-// first entry | entries << 16}; the list's head is the item count.
+// The tile's work lists: a head of counters, the items of sw4_fix_kernel (at most SW4_FIX_THREADS queue entries of one
+// column, {column of the tile, first entry | entries << 16}), then per band the g-points left to sw4_exact_kernel
+// ({column of the tile, k0 * SW_NGPT + g}; a full list's g-points are formed by sw4_fix_kernel itself).
 constexpr int SW4_FIX_THREADS = 64;
 constexpr int SW4_FIX_MINB = 8;                     // CTAs per SM the fix kernel is compiled for
+constexpr int SW4_LIST_HEAD = 32;                   // words: [0] items, [1 + b] exact g-points of band b
 __host__ __device__ constexpr int64_t sw4_max_items(int nlay) { return nlay * SW_NGPT / SW4_FIX_THREADS + 2; }
-__host__ __device__ constexpr int64_t sw4_item_bytes(int nlay, int64_t cols) { return 16 + cols * sw4_max_items(nlay) * (int64_t)sizeof(int2); }
+__host__ __device__ constexpr int64_t sw4_exact_cap(int64_t cols) { return cols > 256 ? cols : 256; }   // per band
+struct Sw4Lists {
+    int* head;                                      // [SW4_LIST_HEAD]
+    int2* items;                                    // [cols * sw4_max_items]
+    int2* exact;                                    // [14][cap]
+    int cap;
+};
+__host__ __device__ constexpr int64_t sw4_list_bytes(int nlay, int64_t cols)
+{
+    return SW4_LIST_HEAD * (int64_t)sizeof(int) + (cols * sw4_max_items(nlay) + 14 * sw4_exact_cap(cols)) * (int64_t)sizeof(int2);
+}
+inline Sw4Lists sw4_lists(void* base, int nlay, int64_t cols)
+{
+    Sw4Lists l;
+    l.head = static_cast<int*>(base);
+    l.items = reinterpret_cast<int2*>(l.head + SW4_LIST_HEAD);
+    l.exact = l.items + cols * sw4_max_items(nlay);
+    l.cap = (int)sw4_exact_cap(cols);
+    return l;
+}
 static_assert(sw4_hdr_bytes() % 16 == 0 && (SW4_LAYER * sizeof(float)) % 16 == 0 && SW_NGPT * sizeof(uint16_t) % 16 == 0,
               "16-byte aligned parts");
 
@@ -247,11 +268,11 @@ __host__ __device__ inline const float* sw4_image_taug(const int4* im)
 
 // Set-up, cloud optics and gas optics of one sunlit column (one CTA, six per SM) into its image.
 __global__ void __launch_bounds__(SW4_GAS_THREADS, SW4_GAS_MINB)
-sw4_gas_kernel(const __grid_constant__ SwBatch bt, int any_aer, int* err, int d0, int4* img, int* items)
+sw4_gas_kernel(const __grid_constant__ SwBatch bt, int any_aer, int* err, int d0, int4* img, Sw4Lists lists)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SwSh2& s = *reinterpret_cast<SwSh2*>(smem_raw);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *items = 0;           // the tile's work list, filled by sw4_rt_kernel
+    if (blockIdx.x == 0 && threadIdx.x < SW4_LIST_HEAD) lists.head[threadIdx.x] = 0;   // the tile's work lists start empty
     const int d = d0 + (int)blockIdx.x;
     if (d >= *bt.req[0].nday) return;
     const int64_t gcol = bt.req[0].daycol[d];
@@ -300,7 +321,7 @@ __host__ __device__ constexpr size_t sw4_rt_smem(bool aer) { return sw4_gas_smem
 
 __global__ void __launch_bounds__(SW4_RT_THREADS, SW4_OPT_MINB)
 sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int4* img, unsigned char* scr, size_t blk_bytes,
-              int* items)
+              int* list_head, int2* items)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int d = d0 + (int)blockIdx.x;
@@ -463,7 +484,7 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
     if (tid == 0) {
         const int n1 = (qnear + SW4_FIX_THREADS - 1) / SW4_FIX_THREADS, n2 = (qres + SW4_FIX_THREADS - 1) / SW4_FIX_THREADS;
         if (n1 + n2 > 0) {
-            int2* it = reinterpret_cast<int2*>(items + 4) + atomicAdd(items, n1 + n2);
+            int2* it = items + atomicAdd(list_head, n1 + n2);
             for (int j = 0; j < n1; ++j) {
                 const int e = j * SW4_FIX_THREADS;
                 it[j] = make_int2((int)blockIdx.x, e | min(SW4_FIX_THREADS, qnear - e) << 16);
@@ -476,51 +497,100 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
     }
 }
 
-// The queued g-points of a tile: the complete layer function (sw2_layer, float64 steps included) over the float R/T
-// that sw4_rt_kernel wrote.  A column has ~50 near-entry tests and, in the 1 % of columns with mu0 near a two-stream
-// resonance that all strongly absorbing layers share, thousands of float64 R/T; so the tile's queue is cut into items
-// of at most 64 entries of one column, which a grid of resident CTAs walks.
+// The complete layer function of queue entry i = k0 * SW_NGPT + g of column c of the tile over the float R/T that
+// sw4_rt_kernel wrote.  s, aer: the column's image, in shared or global memory.  With defer, a g-point that needs the
+// float64 recompute from the column's inputs (sw2_exact) is left alone and true returned.
+__device__ __forceinline__ bool sw4_fix_entry(const SwIn& a, int64_t col, const SwSh2& s, const SwAer* aer, const float* taug,
+                                              unsigned char* blk, const float* ex, const double* exd, int i, bool defer)
+{
+    const int nlay = a.nlay, k0 = i / SW_NGPT, g = i - k0 * SW_NGPT;
+    const Sw4Hdr& H = *reinterpret_cast<const Sw4Hdr*>(blk);
+    const float zsolar = H.zsolar[g];
+    const double czd = (double)__ldg(a.coszen + col);
+    int pending = 0;
+    const SwExactCtx x{&a, col, s.laytrop, s.kmin8, s.kminw, a.iswmode, czd, 1.0 / czd, exd,
+                       zsolar * (1.5f * 86400.0f / SW2_HEAT_T), zsolar * (1.0f / SW2_FLUX_T), defer ? &pending : nullptr};
+    const SwLayerRT2 L = sw2_layer(s, aer, x, k0, g, c_sw_band[g], H.cloudy != 0, a.mask != nullptr, s.cosz, s.sntz, ex,
+                                   __ldg(taug + i));
+    if (pending) return true;
+    float* pc = reinterpret_cast<float*>(blk + sw4_hdr_bytes()) + (size_t)k0 * SW4_LAYER + g;
+    pc[0] = L.c.rb; pc[SW_NGPT] = L.c.rd; pc[2 * SW_NGPT] = L.c.tb; pc[3 * SW_NGPT] = L.c.td;
+    pc[4 * SW_NGPT] = L.c.e3; pc[5 * SW_NGPT] = L.c.e4;
+    const int sl = H.slot[k0];
+    if (sl >= 0) {
+        float* po = pc + (size_t)(nlay - k0 + sl) * SW4_LAYER;
+        po[0] = L.o.rb; po[SW_NGPT] = L.o.rd; po[2 * SW_NGPT] = L.o.tb; po[3 * SW_NGPT] = L.o.td;
+        po[4 * SW_NGPT] = L.o.e3; po[5 * SW_NGPT] = L.o.e4;
+    }
+    return false;
+}
+
+// The queued g-points of a tile.  A column has ~50 near-entry tests and, in the 1 % of columns with mu0 near a two-stream
+// resonance that all strongly absorbing layers share, thousands of float64 R/T; so the tile's queue is cut into items of
+// at most 64 entries of one column, which a grid of resident CTAs walks.  The ~2.5 g-points per column that need the
+// recompute from the inputs go to sw4_exact_kernel (cap > 0): in here each of them holds its warp alone, half of the
+// kernel's time -- 3.41 ms per 131,072 columns against 1.70 + 0.23 ms.  A small tile has warps to spare and would pay the
+// second kernel's latency instead (1,024 columns: 37 us against 20 + 42 us), so from SW4_EXACT_MIN columns on.
+constexpr int64_t SW4_EXACT_MIN = 4096;
 __global__ void __launch_bounds__(SW4_FIX_THREADS, SW4_FIX_MINB)
 sw4_fix_kernel(const __grid_constant__ SwBatch bt, int any_aer, const float* ex, const double* exd, int d0, const int4* img,
-               unsigned char* scr, size_t blk_bytes, const int* items)
+               unsigned char* scr, size_t blk_bytes, Sw4Lists lists)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = items[0], tid = threadIdx.x;
+    const int n = lists.head[0], tid = threadIdx.x;
     for (int w = blockIdx.x; w < n; w += gridDim.x) {
-        const int2 it = reinterpret_cast<const int2*>(items + 4)[w];
+        const int2 it = lists.items[w];
         const int64_t gcol = bt.req[0].daycol[d0 + it.x];
         const int rq = bt.find(gcol);
         const SwIn& a = bt.req[rq];
-        const int nlay = a.nlay;
-        const int64_t col = gcol - bt.off[rq];
         const int4* im = img + (size_t)it.x * (sw4_image_bytes(any_aer) / 16);
-        SwSh2& s = *sw4_load_image(smem_raw, im, any_aer, tid, SW4_FIX_THREADS);
+        const SwSh2& s = *sw4_load_image(smem_raw, im, any_aer, tid, SW4_FIX_THREADS);
         const SwAer* aer = a.faersw ? reinterpret_cast<const SwAer*>(smem_raw + sw4_rt_smem(false)) : nullptr;
         unsigned char* blk = scr + (size_t)it.x * blk_bytes;
-        const Sw4Hdr& H = *reinterpret_cast<const Sw4Hdr*>(blk);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         const int e0 = it.y & 0xffff, ne = it.y >> 16;
         if (tid < ne) {
-            const int i = reinterpret_cast<const uint16_t*>(blk + sw4_queue_offset(nlay))[e0 + tid];
-            const int k0 = i / SW_NGPT, g = i - k0 * SW_NGPT;
-            const float zsolar = H.zsolar[g];
-            const double czd = (double)__ldg(a.coszen + col);
-            const SwExactCtx x{&a, col, s.laytrop, s.kmin8, s.kminw, a.iswmode, czd, 1.0 / czd, exd,
-                               zsolar * (1.5f * 86400.0f / SW2_HEAT_T), zsolar * (1.0f / SW2_FLUX_T)};
-            const SwLayerRT2 L = sw2_layer(s, aer, x, k0, g, c_sw_band[g], H.cloudy != 0, a.mask != nullptr, s.cosz, s.sntz,
-                                           ex, __ldg(sw4_image_taug(im) + i));
-            float* pc = reinterpret_cast<float*>(blk + sw4_hdr_bytes()) + (size_t)k0 * SW4_LAYER + g;
-            pc[0] = L.c.rb; pc[SW_NGPT] = L.c.rd; pc[2 * SW_NGPT] = L.c.tb; pc[3 * SW_NGPT] = L.c.td;
-            pc[4 * SW_NGPT] = L.c.e3; pc[5 * SW_NGPT] = L.c.e4;
-            const int sl = H.slot[k0];
-            if (sl >= 0) {
-                float* po = pc + (size_t)(nlay - k0 + sl) * SW4_LAYER;
-                po[0] = L.o.rb; po[SW_NGPT] = L.o.rd; po[2 * SW_NGPT] = L.o.tb; po[3 * SW_NGPT] = L.o.td;
-                po[4 * SW_NGPT] = L.o.e3; po[5 * SW_NGPT] = L.o.e4;
+            const int i = reinterpret_cast<const uint16_t*>(blk + sw4_queue_offset(a.nlay))[e0 + tid];
+            bool defer = lists.cap > 0;
+            while (sw4_fix_entry(a, gcol - bt.off[rq], s, aer, sw4_image_taug(im), blk, ex, exd, i, defer)) {
+                const int b = c_sw_band[i % SW_NGPT], j = atomicAdd(lists.head + 1 + b, 1);
+                if (j < lists.cap) {
+                    lists.exact[(size_t)b * lists.cap + j] = make_int2(it.x, i);
+                    break;
+                }
+                defer = false;                     // the band's list is full: here after all
             }
         }
         __syncthreads();                           // shared memory is reused by the next item
+    }
+}
+
+// The g-points that sw4_fix_kernel left to the float64 recompute, warp by warp from one band's list, so that the lanes
+// of a warp run the same band's gas optics.
+constexpr int SW4_EXACT_THREADS = 128, SW4_EXACT_MINB = 4;
+__global__ void __launch_bounds__(SW4_EXACT_THREADS, SW4_EXACT_MINB)
+sw4_exact_kernel(const __grid_constant__ SwBatch bt, int any_aer, const float* ex, const double* exd, int d0, const int4* img,
+                 unsigned char* scr, size_t blk_bytes, Sw4Lists lists)
+{
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (SW4_EXACT_THREADS / 32);
+    int w = blockIdx.x * (SW4_EXACT_THREADS / 32) + (threadIdx.x >> 5);     // this warp's next 32 entries
+    for (int b = 0; b < 14; ++b) {
+        const int n = min(lists.head[1 + b], lists.cap), nt = (n + 31) >> 5;
+        for (; w < nt; w += nw) {
+            const int j = 32 * w + lane;
+            if (j >= n) continue;
+            const int2 e = lists.exact[(size_t)b * lists.cap + j];
+            const int64_t gcol = bt.req[0].daycol[d0 + e.x];
+            const int rq = bt.find(gcol);
+            const SwIn& a = bt.req[rq];
+            const unsigned char* im = reinterpret_cast<const unsigned char*>(img + (size_t)e.x * (sw4_image_bytes(any_aer) / 16));
+            const SwSh2& s = *reinterpret_cast<const SwSh2*>(im - sw4_image_begin());
+            const SwAer* aer = a.faersw ? reinterpret_cast<const SwAer*>(im + sizeof(SwSh2) - sw4_image_begin()) : nullptr;
+            sw4_fix_entry(a, gcol - bt.off[rq], s, aer, sw4_image_taug(reinterpret_cast<const int4*>(im)),
+                          scr + (size_t)e.x * blk_bytes, ex, exd, e.y, false);
+        }
+        w -= nt;
     }
 }
 
