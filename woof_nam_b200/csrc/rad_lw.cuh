@@ -56,7 +56,7 @@ struct LwSetup {
 // 07, 09 for the two temperature neighbours, the branch each selects, and the minor-gas and Planck-fraction keys),
 // formed once per (band, layer) instead of in each of the band's g-point tasks.  Slots: bands 3, 4, 5, 7, 9.
 template <class R>
-struct LwKey {
+struct alignas(16) LwKey {
     R sc, sc1, fs, fs1, fm, fpl;
     int js, js1, jm, jpl, br0, br1;
 };
@@ -68,6 +68,8 @@ struct LwSetupK : LwSetup<R> {
     static constexpr bool kKeys = true;
     using Gas = P2;
     static constexpr int kGas = 2;
+    // the sixteen per-layer words every band's task reads first, as four 16-byte words per layer (lw_pack)
+    float4 pk[NLAY_MAX][4];
     LwKey<R> key[LW_NKEYB][NLAY_MAX];
 };
 
@@ -161,12 +163,23 @@ __device__ __forceinline__ V minor2d(const R* t, int nj, int ng, int j, R fj, in
 template <class R, class V, class S>
 __device__ void lw_gas(const S& s, int g, int k0, V& tg, V& fr, int band_of_g = -1)
 {
-    const bool low = s.lower[k0];
-    const int jpk = s.jp[k0], jtk = s.jt[k0], jt1k = s.jt1[k0];
-    const R f00 = s.fac00[k0], f01 = s.fac01[k0], f10 = s.fac10[k0], f11 = s.fac11[k0];
-    const int inds = s.indself[k0], indf = s.indfor[k0], indm = s.indminor[k0];
-    const R sfac = s.selffac[k0], sfr = s.selffrac[k0], ffac = s.forfac[k0], ffr = s.forfrac[k0],
-            mf = s.minorfrac[k0];
+    bool low;
+    int jpk, jtk, jt1k, inds, indf, indm;
+    R f00, f01, f10, f11, sfac, sfr, ffac, ffr, mf;
+    if constexpr (S::kKeys) {
+        const float4 a = s.pk[k0][0], b = s.pk[k0][1], c = s.pk[k0][2], d = s.pk[k0][3];
+        f00 = a.x; f01 = a.y; f10 = a.z; f11 = a.w;
+        sfac = b.x; sfr = b.y; ffac = b.z; ffr = b.w;
+        mf = c.x; jpk = __float_as_int(c.y); jtk = __float_as_int(c.z); jt1k = __float_as_int(c.w);
+        inds = __float_as_int(d.x); indf = __float_as_int(d.y); indm = __float_as_int(d.z); low = __float_as_int(d.w) != 0;
+    } else {
+        low = s.lower[k0];
+        jpk = s.jp[k0]; jtk = s.jt[k0]; jt1k = s.jt1[k0];
+        f00 = s.fac00[k0]; f01 = s.fac01[k0]; f10 = s.fac10[k0]; f11 = s.fac11[k0];
+        inds = s.indself[k0]; indf = s.indfor[k0]; indm = s.indminor[k0];
+        sfac = s.selffac[k0]; sfr = s.selffrac[k0]; ffac = s.forfac[k0]; ffr = s.forfrac[k0];
+        mf = s.minorfrac[k0];
+    }
     auto A4 = [&](const R* t, int ng, int ig, int i0, int i1) {
         auto a = [&](int id) { return ldv<V>(t + ((id - 1) * ng + ig)); };
         return f00 * a(i0) + f10 * a(i0 + 1) + f01 * a(i1) + f11 * a(i1 + 1);
@@ -175,7 +188,11 @@ __device__ void lw_gas(const S& s, int g, int k0, V& tg, V& fr, int band_of_g = 
     auto keys = [&](int q, R& sc, R& sc1, R& fs, R& fs1, int& js, int& js1, int& jm, R& fm, int& jpl, R& fpl, int& br0,
                     int& br1) {
         if constexpr (S::kKeys) {
-            const LwKey<R>& K = s.key[q][k0];
+            LwKey<R> K;
+            const int4* src = reinterpret_cast<const int4*>(&s.key[q][k0]);
+            int4* dst = reinterpret_cast<int4*>(&K);
+#pragma unroll
+            for (int w = 0; w < (int)(sizeof(K) / 16); ++w) dst[w] = src[w];
             sc = K.sc; sc1 = K.sc1; fs = K.fs; fs1 = K.fs1; js = K.js; js1 = K.js1; jm = K.jm; fm = K.fm;
             jpl = K.jpl; fpl = K.fpl; br0 = K.br0; br1 = K.br1;
         }
@@ -856,6 +873,17 @@ __device__ __forceinline__ void lw_keys_band(S& s, int q, int k0)
     }
 }
 
+// Layer k0's words for lw_gas into s.pk (LwSetupK), after setcoef.
+template <class S>
+__device__ __forceinline__ void lw_pack(S& s, int k0)
+{
+    s.pk[k0][0] = make_float4(s.fac00[k0], s.fac01[k0], s.fac10[k0], s.fac11[k0]);
+    s.pk[k0][1] = make_float4(s.selffac[k0], s.selffrac[k0], s.forfac[k0], s.forfrac[k0]);
+    s.pk[k0][2] = make_float4(s.minorfrac[k0], __int_as_float(s.jp[k0]), __int_as_float(s.jt[k0]), __int_as_float(s.jt1[k0]));
+    s.pk[k0][3] = make_float4(__int_as_float(s.indself[k0]), __int_as_float(s.indfor[k0]), __int_as_float(s.indminor[k0]),
+                              __int_as_float(s.lower[k0]));
+}
+
 // Planck functions of band i at level / layer k (k = 0: the surface; phys_rrtm_lw_setcoef.cu:135-160).
 template <class R>
 __device__ __forceinline__ void lw_planck(const LwIn& a, int64_t col, int k, int i, R& lay, R& lev)
@@ -1045,10 +1073,13 @@ __device__ void lw_setup_core(S& s, const LwIn& a, int64_t col, int tid, Sink si
     __syncthreads();
     // the minor-gas column adjustments and the species keys of bands 3, 4, 5, 7, 9 per layer (they read the setcoef
     // results and the chi ratios), an item per thread
-    for (int i = tid; i < (LW_NADJ + (S::kKeys ? LW_NKEYB : 0)) * nlay; i += NT) {
+    for (int i = tid; i < (LW_NADJ + (S::kKeys ? LW_NKEYB + 1 : 0)) * nlay; i += NT) {
         const int q = i / nlay, k0 = i - q * nlay;
         if (q < LW_NADJ) lw_adjcol<R>(s, q, k0);
-        else if constexpr (S::kKeys) lw_keys_band<R>(s, q - LW_NADJ, k0);
+        else if constexpr (S::kKeys) {
+            if (q < LW_NADJ + LW_NKEYB) lw_keys_band<R>(s, q - LW_NADJ, k0);
+            else lw_pack(s, k0);
+        }
     }
     __syncthreads();
     // ---- phase B: gas optics per (g, layer), band by band; the last warp first computes the overlap
