@@ -131,14 +131,16 @@ __device__ __forceinline__ V major12(const R* absa, int ng, int ig, R sc, const 
                                      const Sel<R>& s1, R f01, R f11)
 {
     auto A = [&](int id) { return ldv<V>(absa + ((id - 1) * ng + ig)); };
+    // the third species point: no load where the interpolation is linear (weight 0)
+    auto A3 = [&](int id, R fk2) { return fk2 != (R)0 ? A(id) : vall<V>((R)0); };
     const R fac000 = s0.fk0 * f00, fac100 = s0.fk1 * f00, fac200 = s0.fk2 * f00;
     const R fac010 = s0.fk0 * f10, fac110 = s0.fk1 * f10, fac210 = s0.fk2 * f10;
     const R fac001 = s1.fk0 * f01, fac101 = s1.fk1 * f01, fac201 = s1.fk2 * f01;
     const R fac011 = s1.fk0 * f11, fac111 = s1.fk1 * f11, fac211 = s1.fk2 * f11;
     const V t0 = sc * (fac000 * A(s0.id[0]) + fac010 * A(s0.id[1]) + fac100 * A(s0.id[2]) + fac110 * A(s0.id[3]) +
-                       fac200 * A(s0.id[4]) + fac210 * A(s0.id[5]));
+                       fac200 * A3(s0.id[4], s0.fk2) + fac210 * A3(s0.id[5], s0.fk2));
     const V t1 = sc1 * (fac001 * A(s1.id[0]) + fac011 * A(s1.id[1]) + fac101 * A(s1.id[2]) + fac111 * A(s1.id[3]) +
-                        fac201 * A(s1.id[4]) + fac211 * A(s1.id[5]));
+                        fac201 * A3(s1.id[4], s1.fk2) + fac211 * A3(s1.id[5], s1.fk2));
     return t0 + t1;
 }
 template <class R>
