@@ -66,10 +66,10 @@ typedef struct {
                                 cited at namgpu/physics/rrtm/rrtm_call.py:37); the other part's inputs and
                                 outputs may then be NULL */
     int32_t lw_chunk;        /* mixed precision: columns per LW chunk of the two-kernel LW (gas optics through
-                                ~95 KB per column of scratch, then the sweeps); 0 = 32768; negative = the
+                                ~88 KB per column of scratch, then the sweeps); 0 = 32768; negative = the
                                 single-kernel LW (gas optics in shared memory, no scratch) */
     int32_t sw_sweep_chunk;  /* mixed precision: day columns per chunk of the two-kernel SW (set-up, optics and
-                                the layer reflectances / transmittances through ~330 KB per column of scratch, then
+                                the layer reflectances / transmittances through ~345 KB per column of scratch, then
                                 the adding sweeps); 0 = 16384; negative = the single-kernel SW (no scratch besides
                                 the R/T stores) */
 } RadConfig;

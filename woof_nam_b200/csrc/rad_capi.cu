@@ -11,6 +11,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <type_traits>
 #include <cstdio>
@@ -152,36 +153,35 @@ __global__ void k_scatter(const int* flag, const int* pos, int64_t n, int* dayco
     if (c < n && flag[c]) daycol[pos[c]] = (int)c;
     if (c == n) *nday = pos[n];
 }
-// SW setcoef laytrop of each day column (setcoef.cu:28-73): the last layer (surface first) with
-// ln(p) > 4.56, nlay when there is none.
-__global__ void k_laytrop(const __grid_constant__ DayBatch b, int nlay, const int* daycol, const int* nday, int* lt,
-                          int* cmin, int chunk, const int* pos)
+// SW setcoef laytrop of a column (setcoef.cu:28-73): the last layer (surface first) with ln(p) > 4.56, nlay when there is
+// none.  It is the first that qualifies from the top; ln is monotone and exp(4.56) = 95.58, so only a pressure near the
+// bound takes the logarithm.
+__device__ __forceinline__ int day_laytrop(const DayReq& q, int64_t c, int nlay)
 {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= *nday) return;
+    for (int k = 0; k < nlay; ++k) {
+        const float p = __ldg(q.plyr + (size_t)k * q.ncol + c);
+        if (p > 95.0f && (p > 96.0f || log((double)p) > (double)4.56f)) return nlay - k;
+    }
+    return nlay;
+}
+// Day column d: its laytrop, into lt and the minimum of its chunk.
+__device__ __forceinline__ void day_lay(const DayBatch& b, int nlay, int d, const int* daycol, int* lt, int* cmin, int chunk,
+                                        const int* pos)
+{
     const int64_t g = daycol[d];
     const int r = b.find(g);
     const DayReq& q = b.req[r];
     const int64_t c = g - b.off[r];
-    // the last layer that qualifies is the first from the top; ln is monotone and exp(4.56) = 95.58, so only a pressure
-    // near the bound takes the logarithm
-    int l = 0;
-    for (int k = 0; k < nlay && l == 0; ++k) {
-        const float p = __ldg(q.plyr + (size_t)k * q.ncol + c);
-        if (p > 95.0f && (p > 96.0f || log((double)p) > (double)4.56f)) l = nlay - k;
-    }
-    if (l == 0) l = nlay;
+    const int l = day_laytrop(q, c, nlay);
     lt[d] = l;
     const int w = (int)(c / q.wc);
     const int dw0 = pos[b.off[r] + (int64_t)w * q.wc];
-    const int ci = (d - dw0) / chunk;
-    atomicMin(cmin + q.cmin_off + (int64_t)w * q.maxc + ci, l);
+    atomicMin(cmin + q.cmin_off + (int64_t)w * q.maxc + (d - dw0) / chunk, l);
 }
-__global__ void k_groups(const __grid_constant__ DayBatch b, const int* daycol, const int* nday, const int* lt,
-                         const int* cmin, int chunk, const int* pos, int* k8, int* kw)
+// Day column d: the minima of its 8-column group and of its chunk.
+__device__ __forceinline__ void day_group(const DayBatch& b, int d, const int* daycol, const int* lt, const int* cmin, int chunk,
+                                          const int* pos, int* k8, int* kw)
 {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= *nday) return;
     const int64_t g = daycol[d];
     const int r = b.find(g);
     const DayReq& q = b.req[r];
@@ -199,6 +199,70 @@ __global__ void k_groups(const __grid_constant__ DayBatch b, const int* daycol, 
     for (int i = g0; i < g1; ++i) m = min(m, lt[i]);
     k8[d] = m;
     kw[d] = cmin[q.cmin_off + (int64_t)w * q.maxc + ci];
+}
+__global__ void k_laytrop(const __grid_constant__ DayBatch b, int nlay, const int* daycol, const int* nday, int* lt,
+                          int* cmin, int chunk, const int* pos)
+{
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d < *nday) day_lay(b, nlay, d, daycol, lt, cmin, chunk, pos);
+}
+__global__ void k_groups(const __grid_constant__ DayBatch b, const int* daycol, const int* nday, const int* lt,
+                         const int* cmin, int chunk, const int* pos, int* k8, int* kw)
+{
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d < *nday) day_group(b, d, daycol, lt, cmin, chunk, pos, k8, kw);
+}
+// All of the above for a launch of at most DAY_SMALL columns in one CTA: seven launches of 1-3 us each are most of the
+// day list's cost there (a solve of 1 column 309 -> 283 us, of 1,024 columns 529 -> 506 us).  Above, one CTA's two columns
+// per thread no longer cover the launch and the wide kernels take over.
+constexpr int DAY_SMALL = 2048;
+__global__ void __launch_bounds__(DAY_SMALL / 2) k_daylist_small(const __grid_constant__ DayBatch b, int n, int64_t ncmin, int nlay,
+                                                                 int chunk, int* pos, int* daycol, int* nday, int* lt, int* cmin,
+                                                                 int* k8, int* kw)
+{
+    __shared__ int wsum[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, c0 = 2 * t;   // two columns per thread
+    int f[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        f[j] = 0;
+        if (c0 + j < n) {
+            const int r = b.find(c0 + j);
+            f[j] = b.req[r].coszen[c0 + j - b.off[r]] >= 1.0e-4f ? 1 : 0;
+        }
+    }
+    const int s = f[0] + f[1];
+    int x = s;                                     // inclusive scan of the pairs' counts
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    for (int64_t i = t; i < ncmin; i += DAY_SMALL / 2) cmin[i] = INT_MAX;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < DAY_SMALL / 64; ++w) {
+        if (w < warp) before += wsum[w];
+        total += wsum[w];
+    }
+    const int e = before + x - s;
+    if (c0 < n) {
+        pos[c0] = e;
+        if (f[0]) daycol[e] = c0;
+    }
+    if (c0 + 1 < n) {
+        pos[c0 + 1] = e + f[0];
+        if (f[1]) daycol[e + f[0]] = c0 + 1;
+    }
+    if (t == 0) {
+        pos[n] = total;
+        *nday = total;
+    }
+    __syncthreads();
+    for (int d = t; d < total; d += DAY_SMALL / 2) day_lay(b, nlay, d, daycol, lt, cmin, chunk, pos);
+    __syncthreads();
+    for (int d = t; d < total; d += DAY_SMALL / 2) day_group(b, d, daycol, lt, cmin, chunk, pos, k8, kw);
 }
 __global__ void k_fill_int(int* p, int64_t n, int v)
 {
@@ -587,6 +651,11 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
     // ---- SW day list, laytrop, groups
     const int T = 256;
     const unsigned gb = (unsigned)((ntot + 1 + T - 1) / T);
+    if (ntot <= DAY_SMALL) {
+        k_daylist_small<<<1, DAY_SMALL / 2, 0, st>>>(db, (int)ntot, ncmin, nlay, chunk, sc.pos, sc.daycol, sc.nday, sc.lt, sc.cmin,
+                                                     sc.k8, sc.kw);
+        h->launches += 1;
+    } else {
     k_dayflags<<<gb, T, 0, st>>>(db, ntot, sc.flag);
     size_t tb = sc.cub_bytes;
     RAD_CUDA(h, cub::DeviceScan::ExclusiveSum(sc.cub, tb, sc.flag, sc.pos, (int)(ntot + 1), st));
@@ -595,6 +664,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
     k_laytrop<<<gb, T, 0, st>>>(db, nlay, sc.daycol, sc.nday, sc.lt, sc.cmin, chunk, sc.pos);
     k_groups<<<gb, T, 0, st>>>(db, sc.daycol, sc.nday, sc.lt, sc.cmin, chunk, sc.pos, sc.k8, sc.kw);
     h->launches += 7;   // day flags, scan (2 kernels), scatter, fill, laytrop, groups
+    }
     RAD_CUDA(h, cudaGetLastError());
     // ---- SW over the day columns; zeros first (night columns keep them, as swrad does)
     for (int r = 0; r < nreq; ++r) {

@@ -4,11 +4,11 @@
 // 68 KB) in shared memory, so two CTAs fit an SM and the latency-bound table gathers and sweep recurrences
 // run with ten warps per SM.  Here the gas optics go through HBM instead:
 //
-//   lw3_optics_kernel  one CTA (288 threads) per column: phases A and B of lw_setup_core (absorber amounts,
-//                      cldprop, setcoef, Planck functions, taugb01..16, the max-random overlap factors of
-//                      rtrnmr), with taug / fracs written straight to the chunk's scratch and the sweep inputs
-//                      copied after them.  Shared memory is the set-up data and the species keys of bands 3,
-//                      4, 5, 7 and 9 (LwSetupK, ~50 KB).
+//   lw3_optics_kernel  one CTA (256 threads) per column: phases A and B of lw_setup_core (absorber amounts,
+//                      cldprop, setcoef, Planck functions, taugb01..16 by pairs of g-points, the max-random overlap
+//                      factors of rtrnmr), with taug / fracs and the sweep inputs written straight to the chunk's
+//                      scratch.  Shared memory is the set-up data, the species keys of bands 3, 4, 5, 7 and 9 and
+//                      the layers' packed words (LwSetupK, ~54 KB).
 //   lw3_sweep_kernel   one warp per column, the two sweeps with the g-points in packed pairs (rad_f32x2.cuh), reading
 //                      each layer's row of the scratch staged through shared memory by asynchronous copies.  Per
 //                      layer each g-point's radiance CHANGE across the layer is formed directly (source minus
@@ -56,11 +56,13 @@ constexpr float LW3_THIN = LW_THIN;   // hPa: a cloudy layer thinner than this s
 
 __host__ __device__ constexpr int64_t lw3_block_floats(int nlay) { return (LW3_HEAD + (int64_t)nlay * LW3_ROW + 31) / 32 * 32; }
 
-// Optics CTA: 9 warps, 3 CTAs per SM (27 warps, at most 72 registers a thread, no spills).  The CTAs per SM set
-// how many columns share an SM's L1 for the table gathers, and more than 3 cost more than they gain; more warps
-// per CTA share a column's (g-point, layer) tasks and hide the gathers' latency.  Measured over the LW of 262,144
-// columns: 160 threads 66.1 ms, 192 63.3, 224 61.4, 256 60.5, 288 60.0, 320 63.8 (spills); 4 CTAs of 224 / 256
-// threads 64.0 / 70.1, 2 of 320 / 384 threads 64.0 / 62.6.  Same bits for every shape.
+// Optics CTA: 8 warps, 3 CTAs per SM (24 warps, 80 registers a thread, no spills).  The CTAs per SM set how many
+// columns share an SM's L1 for the table gathers, and more than 3 cost more than they gain; more warps per CTA share a
+// column's tasks and hide the gathers' latency, until the registers run out.  Bound: the L1 data pipe (67 % of its peak
+// wavefronts: every task's gathers touch a line per layer of the warp) and phase A's barriers.  Measured per 131,072
+// columns of 61 layers: one g-point per task 17.4 ms; pairs 13.2 (288 x 3: 13.3, 224 x 4: 14.9, 320 x 3: 14.4, 384 x 2
+// 14.1, 448 x 2: 14.1); phase A and the records spread out 12.6; packed layer words 12.35 (288 x 3: 12.5, 192 x 4: 13.5);
+// no load of a species point of weight zero 12.16.  Same bits for every shape.
 constexpr int LW3_OPT_THREADS = 256;
 constexpr int LW3_OPT_MINB = 3;        // CTAs per SM the optics kernel is compiled for
 

@@ -2,15 +2,15 @@
 fastest per (device, layers, route, column-count bucket).
 
 * lw_chunk: the column tile of the LW gas-optics / sweep kernel pair -- how many columns share one scratch
-  pass (95 KB per column) before the sweeps read it back.
-* sw_sweep_chunk: the tile of sunlit columns of the SW's three kernels (gas optics into the image, layer R/T
-  into the blocks, adding sweeps; ~330 KB per column).
+  pass (88 KB per column) before the sweeps read it back.
+* sw_sweep_chunk: the tile of sunlit columns of the SW's kernels (gas optics into the image, layer R/T into the
+  blocks, float64 fix-ups, adding sweeps; ~345 KB per column).
 
 Small tiles keep more of the scratch in L2 but launch more often and leave the GPU idle at each tile's tail;
 large tiles do the opposite and hold more HBM.  Every candidate gives the same bits (each column's arithmetic
 is independent of the tiling; tests/test_tune.py checks it on the device), so the tuner changes speed only.
-The split of g-points over lanes is fixed by the kernels (five per lane in the LW sweeps, one per thread of
-the SW's R/T and sweeps) and is not a runtime choice.
+The split of g-points over lanes is fixed by the kernels (two pairs and a single per lane in the LW sweeps, a
+pair per thread of the SW's R/T and sweeps) and is not a runtime choice.
 
     from woof_nam_b200.tune import tuned_config
     cfg = tuned_config(ncol=796590)          # SolverConfig with the fastest lw_chunk / sw_sweep_chunk here
