@@ -213,8 +213,8 @@ __global__ void k_groups(const __grid_constant__ DayBatch b, const int* daycol, 
     if (d < *nday) day_group(b, d, daycol, lt, cmin, chunk, pos, k8, kw);
 }
 // All of the above for a launch of at most DAY_SMALL columns in one CTA: seven launches of 1-3 us each are most of the
-// day list's cost there (a solve of 1 column 309 -> 283 us, of 1,024 columns 529 -> 506 us).  Above, one CTA's two columns
-// per thread no longer cover the launch and the wide kernels take over.
+// day list's cost there (a solve of 1 column 309 -> 283 us, of 512 434 -> 420, of 2,048 798 -> 782).  Above, a CTA's
+// threads would take more than two columns each one after the other, where the wide kernels spread them.
 constexpr int DAY_SMALL = 2048;
 __global__ void __launch_bounds__(DAY_SMALL / 2) k_daylist_small(const __grid_constant__ DayBatch b, int n, int64_t ncmin, int nlay,
                                                                  int chunk, int* pos, int* daycol, int* nday, int* lt, int* cmin,

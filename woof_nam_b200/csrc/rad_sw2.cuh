@@ -586,44 +586,6 @@ __device__ __forceinline__ void sw2_rt_mixed(float t0, float tabs, float s0, flo
     e4 = sw_expm(zb4, ex, true);
 }
 
-// Entry int(10^4 zb / (bpade + zb) + 1/2) of the reference's exp table, exp(-bpade i / (10^4 - i)) (1e-20 for
-// the last), evaluated instead of loaded (the float R/T of sw2_rt_float; within a few float ulps of the table's
-// float value for the arguments that matter, ~1e-5 relative where exp is below 1e-13), with the series below
-// 0.06 as sw_expm; em = its complement.
-__device__ __forceinline__ float sw2_tblexp(float zb, float& em)
-{
-    if (zb <= 0.06f) {
-        em = zb - 0.5f * zb * zb;
-        return 1.0f - zb + 0.5f * zb * zb;
-    }
-    const float ftind = zb / ((float)1.0f / (float)0.278f + zb);
-    const int it = min(10000, (int)(ftind * (float)10000 + (float)0.5f));
-    const float e = it >= 10000 ? 1.0e-20f : __expf(-(3.59712230f * (float)it) / (float)(10000 - it));
-    em = 1.0f - e;
-    return e;
-}
-
-// The float R/T of sw2_rt_mixed alone: false (and nothing final) where sw2_rt_mixed would take any float64 step
-// or test the neighbouring table entry -- the resonance, an argument near a table-entry bound with a weight.
-// Where it returns true the outputs are exactly sw2_rt_mixed's.
-__device__ __forceinline__ bool sw2_rt_float(float t0, float tabs, float s0, float y0, float cz, float snt,
-                                             const float* ex, int mode, float wk, float wf, float& rb, float& rd,
-                                             float& tb, float& td, float& e3, float& e4)
-{
-    const SwPro<float> p = sw2_prologue<float>(t0, tabs, s0, y0, mode, cz);
-    if (fabsf(p.zrpp) < SW2_RESONANCE) return false;
-    if (wk > 0.0f && (sw2_near(fminf(p.zrk * p.ztau1, 500.0f)) || sw2_near(fminf(p.ztau1 * snt, 500.0f)))) return false;
-    const float zb4 = t0 * snt;
-    if (wf * 4.0e-4f > 1.0f && sw2_near(zb4)) return false;
-    float em1, em2, em;
-    const float e1 = sw2_tblexp(fminf(p.zrk * p.ztau1, 500.0f), em1);
-    const float e2 = sw2_tblexp(fminf(p.ztau1 * snt, 500.0f), em2);
-    sw2_rt_core<float>(p, cz, e1, em1, e2, em2, rb, rd, tb, td);
-    e3 = sw2_tblexp(p.ztau1 * snt, em);
-    e4 = sw2_tblexp(zb4, em);
-    return true;
-}
-
 struct SwLayerRT {
     float rb, rd, tb, td, e3, e4;
 };

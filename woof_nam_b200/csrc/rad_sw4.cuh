@@ -128,7 +128,8 @@ __device__ __forceinline__ void sw4_near(F2 zb, const SwPos2& p, bool& n0, bool&
     n1 = sw4_near1(zb.y, p.pos.y, p.it.y, m.y);
 }
 // The table entry exp(-bpade it / (10^4 - it)) (1e-20 for the last) and its complement, the series below 0.06
-// (sw2_tblexp without branches; bpade log2(e) folded into one constant).
+// (evaluated instead of loaded, within a few float ulps of the table's float value for the arguments that matter; bpade
+// log2(e) folded into one constant).
 __device__ __forceinline__ float sw4_entry(float it)
 {
     const float e = ex2a(__fdividef(-5.18955054f * it, 10000.0f - it));
@@ -144,7 +145,7 @@ __device__ __forceinline__ F2 sw4_tblexp(F2 zb, const SwPos2& p, F2& em)
 }
 // What a float R/T is left with: nothing, a neighbouring table entry to test, or the resonance in float64.
 enum : int { SW4_Q_NONE = 0, SW4_Q_NEAR = 1, SW4_Q_RES = 2 };
-// sw2_rt_float (prologue of two-stream mode MODE, R/T, direct transmissions) without branches; q0 / q1 say where
+// The float R/T of sw2_rt_mixed (prologue of two-stream mode MODE, R/T, direct transmissions) without branches; q0 / q1 say where
 // sw2_rt_mixed would take a float64 step or test a neighbouring table entry (the outputs are then not used).
 // ASY = false: the asymmetry is zero (the clear pass without aerosol, 85 % of the work), so delta scaling changes
 // nothing and the three direct-beam exponentials are one.
