@@ -46,7 +46,10 @@ __device__ __forceinline__ F2 min2(F2 a, float b) { return F2{fminf(a.x, b), fmi
 __device__ __forceinline__ F2 clamp01(F2 a) { return F2{__saturatef(a.x), __saturatef(a.y)}; }
 __device__ __forceinline__ F2 sqrt2(F2 a) { return F2{sqrtf(a.x), sqrtf(a.y)}; }
 // a / b within 2 ulp for 2^-126 <= |b| <= 2^126 (div.approx: the same bound as the compiler's non-IEEE division,
-// without its rescaling of the operands).
+// without its rescaling of the operands).  Above 2^126 the reciprocal, and with it the quotient, is flushed to zero; so
+// a divisor that may be larger (an optical depth the caller gives) is divided by as F2_DOWN times it, a power of two
+// that changes no rounding, and F2_DOWN goes into the quotient's next factor.
+constexpr float F2_DOWN = 0.0625f;
 __device__ __forceinline__ F2 div2(F2 a, F2 b) { return F2{__fdividef(a.x, b.x), __fdividef(a.y, b.y)}; }
 __device__ __forceinline__ F2 rcp2(F2 a) { return F2{__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)}; }
 // a / b from r = rcp2(b) with one Newton step on the quotient (q + r (a - q b)): within an ulp of the quotient.

@@ -29,13 +29,17 @@ struct LwTerms {
     R atrt;        // cloudy: total absorptance 1 - trnt, likewise
 };
 
+// A depth that has the last entry of the tables; above it the product with the diffusivity may be infinite, whose
+// position is NaN (entry 0).
+constexpr float LW_OD_MAX = 1.0e30f;
+
 template <class R>
 __device__ __forceinline__ LwTerms<R> lw2_terms(const LwShared<R>& s, const LwLut<R>& lut, int g, int band, int k,
                                                 R sdif, bool cloudy)
 {
     const R bpade = (R)1.0f / (R)0.278f, tblint = (R)10000, rec_6 = (R)0.166667f, c06 = (R)0.06f;
     LwTerms<R> t;
-    R odepth = fmaxR((R)0, sdif * s.taug[g][k - 1]);
+    R odepth = fminR((R)LW_OD_MAX, fmaxR((R)0, sdif * s.taug[g][k - 1]));
     R atrgas, gasfac;
     if (odepth <= c06) {
         atrgas = odepth - (R)0.5f * odepth * odepth;
@@ -55,7 +59,7 @@ __device__ __forceinline__ LwTerms<R> lw2_terms(const LwShared<R>& s, const LwLu
     t.atrg = atrgas;
     t.trnt = 1; t.totsrcd = 0; t.totsrcu = 0; t.atrt = 0;
     if (cloudy) {
-        const R odtot = odepth + sdif * s.taucld[band][k - 1];
+        const R odtot = fminR((R)LW_OD_MAX, odepth + sdif * s.taucld[band][k - 1]);
         R totfac, atrtot;
         if (odtot < c06) {
             totfac = rec_6 * odtot; atrtot = odtot - (R)0.5f * odtot * odtot; t.trnt = (R)1 - atrtot;

@@ -140,13 +140,14 @@ __global__ void __launch_bounds__(LW3_FP64_THREADS) lw3_fp64_kernel(const __grid
 // The entry of rtrnmr's transmittance / Planck-fraction tables for optical depth od: position 10^4 od / (bpade + od) +
 // 1/2, its integer part taken by adding 2^23 rounded down (entry number in the sum's low bits; clamped, so a NaN depth
 // reads the last entry).  lut[i] = {exp, tfn}, one 8-byte load.  The quotient takes a Newton step: a depth's rounding
-// decides which of two entries, 3e-4 apart, it gets.
+// decides which of two entries, 3e-4 apart, it gets.  The divisor is scaled (F2_DOWN), so that every finite depth has its
+// entry; an infinite one (cloud times diffusivity past the largest float) has a NaN position, the last entry.
 constexpr float LW3_TWO23 = 8388608.0f;
 template <class V>
 __device__ __forceinline__ V lw3_pos(V od)
 {
-    const V d = od + vset<V>(1.0f / 0.278f);
-    return f2_add_rm(fma2(quot2(od, d, rcp2(d)), vset<V>(10000.0f), vset<V>(0.5f)), vset<V>(LW3_TWO23));
+    const V d = fma2(od, vset<V>(F2_DOWN), vset<V>(F2_DOWN * (1.0f / 0.278f)));
+    return f2_add_rm(fma2(quot2(od, d, rcp2(d)), vset<V>(10000.0f * F2_DOWN), vset<V>(0.5f)), vset<V>(LW3_TWO23));
 }
 __device__ __forceinline__ float2 lw3_entry(const float2* lut, float pr)
 {

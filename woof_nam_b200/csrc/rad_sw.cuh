@@ -413,11 +413,13 @@ __device__ void sw_sfluxzen(S& s, int b, int nlay)
 
 // ------------------------------------------------------------------------------------------------------
 // exp(-zb) as spcvrtc evaluates it (spcvrtc.cu:20-43): expansion below 0.06, else the table; `clamped`
-// selects the direct-beam index form.
+// selects the direct-beam index form, whose argument may be any depth times 1 / mu0, infinite in float (1e30 has the
+// last entry already).
 template <class R>
 __device__ __forceinline__ R sw_expm(R zb, const R* ex, bool clamped)
 {
     if (zb <= (R)0.06f) return (R)1 - zb + (R)0.5f * zb * zb;
+    if (clamped && zb > (R)1.0e30f) zb = (R)1.0e30f;
     const R ftind = zb / ((R)1.0f / (R)0.278f + zb);
     int it = clamped ? (int)((R)0.5f + (R)10000 * ftind) : (int)(ftind * (R)10000 + (R)0.5f);
     if (clamped) it = max(0, min(10000, it));

@@ -103,15 +103,16 @@ struct SwRT2 {
     F2 rb, rd, tb, td, e3, e4;
 };
 // Position of zb in the reference's exp table: ft = zb / (bpade + zb), pos = 10^4 ft + 1/2, it = floor(pos) as a float
-// (adding 2^23 rounded down leaves the integer part, so no float <-> integer conversion is needed).
+// (adding 2^23 rounded down leaves the integer part, so no float <-> integer conversion is needed).  q = ft / F2_DOWN:
+// the divisor is scaled, so that every finite zb has its entry.
 struct SwPos2 {
-    F2 ft, pos, it;
+    F2 q, pos, it;
 };
 __device__ __forceinline__ SwPos2 sw4_pos(F2 zb)
 {
     SwPos2 p;
-    p.ft = div2(zb, zb + (float)1.0f / (float)0.278f);
-    p.pos = fma2(p.ft, f2(10000.0f), f2(0.5f));
+    p.q = div2(zb, fma2(zb, f2(F2_DOWN), f2(F2_DOWN * ((float)1.0f / (float)0.278f))));
+    p.pos = fma2(p.q, f2(10000.0f * F2_DOWN), f2(0.5f));
     p.it = f2_add_rm(p.pos, f2(8388608.0f)) - 8388608.0f;
     return p;
 }
@@ -123,7 +124,7 @@ __device__ __forceinline__ bool sw4_near1(float zb, float pos, float it, float m
 }
 __device__ __forceinline__ void sw4_near(F2 zb, const SwPos2& p, bool& n0, bool& n1)
 {
-    const F2 m = (p.ft * 10000.0f) * fma2(f2(1.0f) - p.ft, f2(SW2_ZB_EPS), f2(3.0e-7f));
+    const F2 m = (p.q * (10000.0f * F2_DOWN)) * fma2(nma2(p.q, f2(F2_DOWN), f2(1.0f)), f2(SW2_ZB_EPS), f2(3.0e-7f));
     n0 = sw4_near1(zb.x, p.pos.x, p.it.x, m.x);
     n1 = sw4_near1(zb.y, p.pos.y, p.it.y, m.y);
 }
@@ -143,6 +144,8 @@ __device__ __forceinline__ F2 sw4_tblexp(F2 zb, const SwPos2& p, F2& em)
     em = F2{s0 ? h.x : ec.x, s1 ? h.y : ec.y};
     return F2{s0 ? es.x : et.x, s1 ? es.y : et.y};
 }
+// A depth along the beam with the last entry instead of an infinite one (a NaN stays).
+__device__ __forceinline__ F2 sw4_cap(F2 zb) { return F2{zb.x > 1.0e30f ? 1.0e30f : zb.x, zb.y > 1.0e30f ? 1.0e30f : zb.y}; }
 // What a float R/T is left with: nothing, a neighbouring table entry to test, or the resonance in float64.
 enum : int { SW4_Q_NONE = 0, SW4_Q_NEAR = 1, SW4_Q_RES = 2 };
 // The float R/T of sw2_rt_mixed (prologue of two-stream mode MODE, R/T, direct transmissions) without branches; q0 / q1 say where
@@ -155,11 +158,12 @@ __device__ __forceinline__ void sw4_rt(F2 t0, F2 tabs, F2 s0, F2 y0, float cz, f
 {
     const float ftiny = 1.0e-12f;
     const float cwmin = (float)(1.0 - ((double)1.0f - (double)1.0e-6f));
-    const F2 cw = max2(quot2(tabs, t0, rcp2(t0)), cwmin);
-    const F2 zssaw = 1.0f - cw;
-    F2 ztau1, zssa1, cw1, zasy1, zasy3;
+    // co-albedo over F2_DOWN, from a scaled divisor: the depth may be any finite float
+    const F2 ts = t0 * F2_DOWN, cw = max2(quot2(tabs, ts, rcp2(ts)), cwmin / F2_DOWN);
+    const F2 zssaw = nma2(cw, f2(F2_DOWN), f2(1.0f));
+    F2 ztau1, zssa1, cw1, zasy1, zasy3;      // cw1 over F2_DOWN as cw
     if constexpr (ASY) {
-        const F2 sm = max2(s0, ftiny), zasyw = quot2(y0, sm, rcp2(sm));
+        const F2 sm = max2(s0, ftiny) * F2_DOWN, zasyw = quot2(y0, sm, rcp2(sm)) * F2_DOWN;
         const F2 za2s = zssaw * (zasyw * zasyw);
         const F2 om = 1.0f - za2s, ro = rcp2(om);
         ztau1 = om * t0;
@@ -176,7 +180,7 @@ __device__ __forceinline__ void sw4_rt(F2 t0, F2 tabs, F2 s0, F2 y0, float cz, f
         g1 = ASY ? nma2(zssa1, zasy3 + 1.25f, f2(2.0f)) : fma2(zssa1, f2(-1.25f), f2(2.0f));
         g2 = ASY ? (zssa1 * 0.75f) * (1.0f - zasy1) : zssa1 * 0.75f;
         g3 = ASY ? nma2(zasy3, f2(cz), f2(0.5f)) : f2(0.5f);
-        gm = cw1 + cw1;
+        gm = cw1 * (2.0f * F2_DOWN);
         gp = ASY ? nma2(zssa1, fma2(zasy1, f2(1.5f), f2(0.5f)), f2(2.0f)) : fma2(zssa1, f2(-0.5f), f2(2.0f));
     } else if constexpr (MODE == 1) {
         g1 = nma2(zssa1, zasy3 + 1.0f, f2(1.75f));
@@ -189,14 +193,14 @@ __device__ __forceinline__ void sw4_rt(F2 t0, F2 tabs, F2 s0, F2 y0, float cz, f
         g1 = nma2(zssa1, zasy1 + 1.0f, f2(2.0f)) * zsr3 * 0.5f;
         g2 = (zssa1 * zsr3) * (1.0f - zasy1) * 0.5f;
         g3 = nma2(zasy1 * zsr3, f2(cz), f2(1.0f)) * 0.5f;
-        gm = cw1 * zsr3;
+        gm = cw1 * (zsr3 * F2_DOWN);
         gp = nma2(zssa1, zasy1, f2(1.0f)) * zsr3;
     }
     const F2 g4 = 1.0f - g3;
     const F2 zrk = sqrt2(gm * gp);
     const F2 zrp = zrk * cz;
     const F2 zrpp0 = (1.0f - zrp) * (zrp + 1.0f);
-    const F2 zbd = ztau1 * snt, zb1 = min2(zrk * ztau1, 500.0f), zb2 = min2(zbd, 500.0f), zb4 = ASY ? t0 * snt : zbd;
+    const F2 zbd = ztau1 * snt, zb1 = min2(zrk * ztau1, 500.0f), zb2 = min2(zbd, 500.0f), zb4 = ASY ? sw4_cap(t0 * snt) : zbd;
     const SwPos2 p1 = sw4_pos(zb1), p2 = sw4_pos(zb2);
     F2 em1, em2, em;
     const F2 e1 = sw4_tblexp(zb1, p1, em1), e2 = sw4_tblexp(zb2, p2, em2);
