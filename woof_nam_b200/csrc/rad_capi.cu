@@ -305,10 +305,41 @@ void sw_lut(std::vector<R>& v)   // exp_tbl(0:10000) (phys_rrtm_sw_spcvrtc.py:60
 
 // The plain FP64 precision runs the first-design kernels (lw_column_kernel / sw_column_kernel<double>);
 // the mixed precision runs the production kernels (lw2_column_kernel<float> / sw2_column_kernel).
-template <class R>
-void* kernel_ptr_lw(bool mc) { return sizeof(R) == 4 ? (mc ? (void*)lw2_column_kernel<float, true> : (void*)lw2_column_kernel<float, false>) : (void*)lw_column_kernel<double>; }
-template <class R>
-void* kernel_ptr_sw() { return (void*)sw_column_kernel<R>; }
+// Dynamic shared memory of a CTA of sw4_sweep_kernel (the segment checkpoints).
+constexpr size_t sw4_sweep_smem() { return (size_t)(SW2_NSEG - 1) * 2 * SW4_SWEEP_THREADS * sizeof(float2); }
+// The solve kernels' dynamic shared-memory limits, each the largest any launch of the kernel asks for.  A limit belongs to
+// the kernel on the device, not to a handle or a call: set per launch to that launch's size, a solve without aerosol lowered
+// it between another thread's call and its larger launch.  Set once, with the device's tables.
+cudaError_t set_smem_limits()
+{
+    const struct {
+        const void* kernel;
+        size_t bytes;
+    } lim[] = {{(const void*)lw3_optics_kernel, sizeof(LwSetupK<float>)},
+               {(const void*)lw3_sweep_kernel<LW_OVR_MAXRAN>, lw3_sweep_smem()},
+               {(const void*)lw3_sweep_kernel<LW_OVR_MAXRAN, true>, lw3_sweep_smem()},
+               {(const void*)lw3_sweep_kernel<LW_OVR_RANDOM>, lw3_sweep_smem()},
+               {(const void*)lw3_sweep_kernel<LW_OVR_RANDOM, true>, lw3_sweep_smem()},
+               {(const void*)lw3_sweep_kernel<LW_OVR_MCICA>, lw3_sweep_smem()},
+               {(const void*)lw3_sweep_kernel<LW_OVR_MCICA, true>, lw3_sweep_smem()},
+               {(const void*)lw3_fp64_kernel, sizeof(LwShared<double>)},
+               {(const void*)lw2_column_kernel<float, false>, sizeof(LwShared<float>)},
+               {(const void*)lw2_column_kernel<float, true>, sizeof(LwShared<float>)},
+               {(const void*)lw_column_kernel<double>, sizeof(LwShared<double>)},
+               {(const void*)sw4_gas_kernel, sw4_gas_smem(true)},
+               {(const void*)sw4_rt_kernel, sw4_rt_smem(true)},
+               {(const void*)sw4_fix_kernel, sw4_rt_smem(true)},
+               {(const void*)sw4_sweep_kernel<false>, sw4_sweep_smem()},
+               {(const void*)sw4_sweep_kernel<true>, sw4_sweep_smem()},
+               {(const void*)sw2_column_kernel<false>, sw2_smem_bytes(true)},
+               {(const void*)sw2_column_kernel<true>, sw2_smem_bytes(true)},
+               {(const void*)sw_column_kernel<double>, sizeof(SwShared<double>)}};
+    for (const auto& l : lim) {
+        const cudaError_t e = cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.bytes);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
 
 template <class T>
 int upload(RadHandle* h, T** dptr, const std::vector<T>& host)
@@ -593,20 +624,18 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
             LwLut<double> dl;
             dl.ex = h->d_lwd; dl.tfn = h->d_lwd + 10001; dl.tau = h->d_lwd + 2 * 10001;
             const size_t smem1 = sizeof(LwSetupK<float>), smemd = sizeof(LwShared<double>);
-            RAD_CUDA(h, cudaFuncSetAttribute((void*)lw3_optics_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-            RAD_CUDA(h, cudaFuncSetAttribute((void*)lw3_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemd));
             const int64_t lstep = diag_lw ? std::min(lwc, (int64_t)LW_DIAG_CHUNK) : lwc;
             for (int64_t c0 = 0; c0 < ntot; c0 += lstep) {
                 const int64_t nc = std::min(lstep, ntot - c0);
                 RAD_CUDA(h, cudaMemsetAsync(h->d_lw3list, 0, sizeof(int), st));
                 lw3_optics_kernel<<<(unsigned)nc, LW3_OPT_THREADS, smem1, st>>>(bt, c0, h->d_lw3, h->d_lw3list, h->d_err);
+                RAD_CUDA(h, cudaGetLastError());   // nothing reads a scratch that was not written
                 const unsigned g2 = (unsigned)std::min<int64_t>(nc, h->nsm);
                 float* pg = h->d_lwpg;
                 const auto sweep = mc ? (diag_lw ? lw3_sweep_kernel<LW_OVR_MCICA, true> : lw3_sweep_kernel<LW_OVR_MCICA>)
                                    : cfg.iovrlw == 0
                                        ? (diag_lw ? lw3_sweep_kernel<LW_OVR_RANDOM, true> : lw3_sweep_kernel<LW_OVR_RANDOM>)
                                        : (diag_lw ? lw3_sweep_kernel<LW_OVR_MAXRAN, true> : lw3_sweep_kernel<LW_OVR_MAXRAN>);
-                RAD_CUDA(h, cudaFuncSetAttribute((const void*)sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lw3_sweep_smem()));
                 sweep<<<g2, LW3_SWEEP_WARPS * 32, lw3_sweep_smem(), st>>>(bt, c0, nc, h->d_lw3, fl, pg);
                 h->launches += 2;
                 if (!mc) {
@@ -621,7 +650,6 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
             RAD_CUDA(h, cudaGetLastError());
         } else {
         const size_t smem = sizeof(LwShared<R>);
-        RAD_CUDA(h, cudaFuncSetAttribute(kernel_ptr_lw<R>(mc), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (sizeof(R) == 4 && mc) {
             lw2_column_kernel<R, true><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, nullptr);
             h->launches += 1;
@@ -631,7 +659,6 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
             LwLut<double> dl;
             dl.ex = h->d_lwd; dl.tfn = h->d_lwd + 10001; dl.tau = h->d_lwd + 2 * 10001;
             const size_t smemd = sizeof(LwShared<double>);
-            RAD_CUDA(h, cudaFuncSetAttribute((void*)lw3_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemd));
             RAD_CUDA(h, cudaMemsetAsync(sc.pos, 0, sizeof(int), st));
             lw2_column_kernel<R, false><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, sc.pos);
             lw3_fp64_kernel<<<(unsigned)h->nsm, LW3_FP64_THREADS, smemd, st>>>(bt, 0, sc.pos, dl, h->d_err);
@@ -696,7 +723,6 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
         if (sizeof(R) == 4) {
             const size_t smem = sw2_smem_bytes(any_aer);
             if (fixed) {   // no scratch: one CTA per sunlit column, R/T recomputed on the way down
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw2_column_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 sw2_column_kernel<false><<<(unsigned)ntot, SW2_THREADS, smem, st>>>(bt, any_aer ? 1 : 0, h->d_swf, h->d_swd,
                                                                                      h->d_err, nullptr);
             } else if (sw4_chunk(cfg) > 0) {
@@ -706,21 +732,18 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 const int64_t swc = sw4_chunk(cfg);
                 const size_t smem0 = sw4_gas_smem(any_aer);
                 const size_t smem1 = sw4_rt_smem(any_aer);    // the image without taug (read from the image)
-                const size_t smem2 = (size_t)(SW2_NSEG - 1) * 2 * SW4_SWEEP_THREADS * sizeof(float2);
+                const size_t smem2 = sw4_sweep_smem();
                 const size_t bb = sw4_block_bytes(nlay);
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_gas_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0));
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_rt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_sweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw4_sweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
                 Sw4Lists lists = sw4_lists(h->d_sw4list, nlay, h->sw4_cap);
                 if (std::min(swc, ntot) < SW4_EXACT_MIN) lists.cap = 0;
                 for (int64_t d0 = 0; d0 < ntot; d0 += swc) {
                     const int64_t nc = std::min(swc, ntot - d0);
                     sw4_gas_kernel<<<(unsigned)nc, SW4_GAS_THREADS, smem0, st>>>(bt, any_aer ? 1 : 0, h->d_err, (int)d0, h->d_sw4img,
                                                                                  lists);
+                    RAD_CUDA(h, cudaGetLastError());
                     sw4_rt_kernel<<<(unsigned)nc, SW4_RT_THREADS, smem1, st>>>(bt, any_aer ? 1 : 0, (int)d0, h->d_sw4img, h->d_sw4,
                                                                                bb, lists.head, lists.items);
+                    RAD_CUDA(h, cudaGetLastError());
                     sw4_fix_kernel<<<(unsigned)(SW4_FIX_MINB * h->nsm), SW4_FIX_THREADS, smem1, st>>>(
                         bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, lists);
                     if (lists.cap > 0)
@@ -737,7 +760,6 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 }
                 nlaunch = (4 + (lists.cap > 0) + (diag_sw ? 1 : 0)) * ((ntot + swc - 1) / swc);
             } else {       // SW2_CTAS_PER_SM CTAs per SM walk the day list, each with its R/T store
-                RAD_CUDA(h, cudaFuncSetAttribute((void*)sw2_column_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 sw2_column_kernel<true><<<(unsigned)(SW2_CTAS_PER_SM * h->nsm), SW2_THREADS, smem, st>>>(
                     bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, h->d_err, h->d_swrt);
             }
@@ -745,7 +767,6 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
             SwLut<R> lut;
             lut.ex = (const R*)h->d_swd;
             const size_t smem = sizeof(SwShared<R>);
-            RAD_CUDA(h, cudaFuncSetAttribute(kernel_ptr_sw<R>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             sw_column_kernel<R><<<(unsigned)ntot, SW_THREADS, smem, st>>>(bt, lut, h->d_swd, h->d_err);
         }
         h->launches += nlaunch;
@@ -927,6 +948,7 @@ int rad_load_tables(RadHandle* h, const void* blob, size_t nbytes)
         pw[0] = 1u;
         for (int i = 1; i < 624; ++i) pw[i] = 69069u * pw[i - 1];
         RAD_CUDA(h, cudaMemcpyToSymbol(c_mt_pow, pw, sizeof(pw)));
+        RAD_CUDA(h, set_smem_limits());
         RAD_CUDA(h, cudaDeviceSynchronize());
         dt.tf = tf;
         dt.td = td;

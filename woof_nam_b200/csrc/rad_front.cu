@@ -41,6 +41,7 @@
 #include "rad_front.h"
 
 #include <cmath>
+#include <mutex>
 
 namespace rad {
 namespace front {
@@ -706,15 +707,27 @@ __global__ void __launch_bounds__(256) k_setaer_volc(const __grid_constant__ Vol
 
 inline unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// Room for a launch of `smem` bytes of dynamic shared memory.  A kernel's limit is one for all threads of the process and
+// is only raised here, so that no call lowers it between another thread's call and its launch.
+template <class K>
+cudaError_t raise_smem(K kernel, size_t smem)
+{
+    if (smem <= 48 * 1024) return cudaSuccess;                     // every kernel's limit from the start
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+    if (e != cudaSuccess || (size_t)at.maxDynamicSharedSizeBytes >= smem) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
 }  // namespace
 
 cudaError_t dayparts(const DaypartsArgs& a, cudaStream_t st)
 {
     const size_t smem = 2 * sizeof(int) * (size_t)a.im;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_dayparts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = raise_smem(k_dayparts, smem);
+    if (e != cudaSuccess) return e;
     k_dayparts<<<(unsigned)a.jm, DP_THREADS, smem, st>>>(a);
     return cudaGetLastError();
 }
@@ -728,10 +741,8 @@ cudaError_t getgases(const GasArgs& a, cudaStream_t st)
 cudaError_t getozn(const OzoneArgs& a, cudaStream_t st)
 {
     const size_t smem = sizeof(float) * ((size_t)2 * a.loz * a.jmr + a.loz + (size_t)a.loz * OZ_THREADS);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_getozn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = raise_smem(k_getozn, smem);
+    if (e != cudaSuccess) return e;
     k_getozn<<<blocks(a.n, OZ_THREADS), OZ_THREADS, smem, st>>>(a);
     return cudaGetLastError();
 }
@@ -751,10 +762,8 @@ cudaError_t setemis(const EmisArgs& a, cudaStream_t st)
 cudaError_t progcld2(const CloudArgs& a, cudaStream_t st)
 {
     const size_t smem = sizeof(float) * (size_t)a.nlay * CLD_THREADS;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_progcld2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = raise_smem(k_progcld2, smem);
+    if (e != cudaSuccess) return e;
     k_progcld2<<<blocks(a.n, CLD_THREADS), CLD_THREADS, smem, st>>>(a);
     return cudaGetLastError();
 }
