@@ -528,6 +528,11 @@ typedef struct {
     double sw_ms;            /* device time of the SW column kernel */
 } RadProfile;
 
+/* Instrumentation: per SW band (16..29), how many of the last tile's layer reflectances the handle's last rad_solve gave to
+ * the float64 recompute lists, and how many each list holds (what is past it stays with the kernel that found it, with
+ * the same result).  *capacity = 0: the tile was too small for the lists, and so are all counts.  Waits for the device. */
+int rad_sw_recomputes(RadHandle* h, int32_t* counts, int32_t* capacity);
+
 int rad_profile_enable(RadHandle* h, int on);
 int rad_profile_read(RadHandle* h, RadProfile* p);
 

@@ -28,7 +28,7 @@ def _resonant(n, nlay, mode, seed):
     return Columns(**d, solcon=cols.solcon)
 
 
-@pytest.mark.parametrize("nlay,mode,tile", [(61, 2, 100), (61, 3, 0), (2, 2, 37), (16, 2, 64), (33, 3, 128)])
+@pytest.mark.parametrize("nlay,mode,tile", [(61, 2, 100), (61, 3, 90), (2, 2, 37), (16, 2, 64), (33, 3, 128)])
 def test_resonant_columns(nlay, mode, tile):
     import torch
     from woof_nam_b200.solver import RadSolver
@@ -48,8 +48,8 @@ def test_resonant_columns(nlay, mode, tile):
 
 def test_recompute_lists_and_their_overflow():
     """A tile of 4,096 columns or more hands its float64 recomputes to sw4_exact_kernel through per-band lists (here
-    with more resonant g-points than the lists hold, so some stay with sw4_fix_kernel); smaller tiles run them all in
-    sw4_fix_kernel.  Same bits either way, and within tolerance of the oracle."""
+    with more resonant g-points in some bands than a list holds, so that some stay with sw4_fix_kernel, and fewer in
+    others); smaller tiles run them all in sw4_fix_kernel.  Same bits either way, and within tolerance of the oracle."""
     import torch
     from woof_nam_b200.solver import RadSolver
     cols = _resonant(4600, 61, 2, 77)
@@ -59,6 +59,11 @@ def test_recompute_lists_and_their_overflow():
         out = s.solve(s.to_device(cols), cols.solcon)
         torch.cuda.synchronize()
         assert s.device_error() == 0
+        counts, cap = s.sw_recomputes()
+        if t == 0:                                   # one tile of all the columns
+            assert cap == 4600 and max(counts) > cap and any(0 < c <= cap for c in counts), counts
+        else:
+            assert cap == (t if t >= 4096 else 0)
         outs.append({k: v.cpu().numpy() for k, v in out.items()})
     for o in outs[1:]:
         for k in o:

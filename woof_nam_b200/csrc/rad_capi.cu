@@ -87,6 +87,7 @@ struct RadHandle {
     unsigned char* d_sw4 = nullptr;                // chunked SW: header and layer R/T of one chunk's columns
     void* d_sw4list = nullptr;                     // chunked SW: work lists of the float64 fix-up (Sw4Lists)
     int64_t sw4_cap = 0;                           // columns d_sw4 and d_sw4img hold
+    int sw4_list_cap = 0;                          // entries per band list of the last launch (0: no lists)
     float* d_aerf = nullptr;                       // aerosol band tables of the loaded month (AF_* offsets)
     int* d_aeri = nullptr;                         // their integer part (AI_* offsets)
     int nsm = 148;                                 // SMs of the device (grid of the float64 column kernel)
@@ -736,6 +737,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                 const size_t bb = sw4_block_bytes(nlay);
                 Sw4Lists lists = sw4_lists(h->d_sw4list, nlay, h->sw4_cap);
                 if (std::min(swc, ntot) < SW4_EXACT_MIN) lists.cap = 0;
+                h->sw4_list_cap = lists.cap;
                 for (int64_t d0 = 0; d0 < ntot; d0 += swc) {
                     const int64_t nc = std::min(swc, ntot - d0);
                     sw4_gas_kernel<<<(unsigned)nc, SW4_GAS_THREADS, smem0, st>>>(bt, any_aer ? 1 : 0, h->d_err, (int)d0, h->d_sw4img,
@@ -1610,6 +1612,18 @@ int rad_device_error(RadHandle* h, int32_t* code)
     RAD_CUDA(h, cudaMemcpy(&v, h->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     RAD_CUDA(h, cudaMemset(h->d_err, 0, sizeof(int)));
     *code = v;
+    return RAD_OK;
+}
+
+int rad_sw_recomputes(RadHandle* h, int32_t* counts, int32_t* capacity)
+{
+    if (!h || !counts || !capacity) return fail(h, RAD_E_INVALID, "rad_sw_recomputes: null argument");
+    for (int b = 0; b < 14; ++b) counts[b] = 0;
+    *capacity = h->d_sw4list ? h->sw4_list_cap : 0;
+    if (*capacity > 0) {
+        RAD_CUDA(h, cudaDeviceSynchronize());
+        RAD_CUDA(h, cudaMemcpy(counts, (const int*)h->d_sw4list + 1, 14 * sizeof(int), cudaMemcpyDeviceToHost));
+    }
     return RAD_OK;
 }
 

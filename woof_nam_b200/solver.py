@@ -304,6 +304,14 @@ class RadSolver:
         _lib.check(self.lib, self.handle, rc, "rad_device_error")
         return int(code.value)
 
+    def sw_recomputes(self) -> tuple[list, int]:
+        """Per SW band, the float64 recomputes the last solve's last tile put on the lists, and a list's capacity
+        (0: no lists); see rad_sw_recomputes."""
+        n, cap = (ctypes.c_int32 * 14)(), ctypes.c_int32()
+        rc = self.lib.rad_sw_recomputes(self.handle, n, ctypes.byref(cap))
+        _lib.check(self.lib, self.handle, rc, "rad_sw_recomputes")
+        return list(n), int(cap.value)
+
     def profile(self, on: bool = True) -> None:
         """Start (or stop) device-time accounting of the library's kernels on this handle."""
         _lib.check(self.lib, self.handle, self.lib.rad_profile_enable(self.handle, int(on)), "rad_profile_enable")
