@@ -650,25 +650,27 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
             }
             RAD_CUDA(h, cudaGetLastError());
         } else {
-        const size_t smem = sizeof(LwShared<R>);
-        if (sizeof(R) == 4 && mc) {
-            lw2_column_kernel<R, true><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, nullptr);
-            h->launches += 1;
-        } else if (sizeof(R) == 4) {
-            // NAM route: columns with a cloudy layer under 1 hPa go to the float64 column kernel through a list
-            // in the day-list scratch's pos array (ntot + 1 words; the SW part rewrites it afterwards)
-            LwLut<double> dl;
-            dl.ex = h->d_lwd; dl.tfn = h->d_lwd + 10001; dl.tau = h->d_lwd + 2 * 10001;
-            const size_t smemd = sizeof(LwShared<double>);
-            RAD_CUDA(h, cudaMemsetAsync(sc.pos, 0, sizeof(int), st));
-            lw2_column_kernel<R, false><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, sc.pos);
-            lw3_fp64_kernel<<<(unsigned)h->nsm, LW3_FP64_THREADS, smemd, st>>>(bt, 0, sc.pos, dl, h->d_err);
-            h->launches += 2;
-        } else {
-            lw_column_kernel<R><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err);
-            h->launches += 1;
-        }
-        RAD_CUDA(h, cudaGetLastError());
+            const size_t smem = sizeof(LwShared<R>);
+            if constexpr (sizeof(R) == 4) {
+                if (mc) {
+                    lw2_column_kernel<R, true><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, nullptr);
+                    h->launches += 1;
+                } else {
+                    // NAM route: columns with a cloudy layer under 1 hPa go to the float64 column kernel through a list
+                    // in the day-list scratch's pos array (ntot + 1 words; the SW part rewrites it afterwards)
+                    LwLut<double> dl;
+                    dl.ex = h->d_lwd; dl.tfn = h->d_lwd + 10001; dl.tau = h->d_lwd + 2 * 10001;
+                    const size_t smemd = sizeof(LwShared<double>);
+                    RAD_CUDA(h, cudaMemsetAsync(sc.pos, 0, sizeof(int), st));
+                    lw2_column_kernel<R, false><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err, sc.pos);
+                    lw3_fp64_kernel<<<(unsigned)h->nsm, LW3_FP64_THREADS, smemd, st>>>(bt, 0, sc.pos, dl, h->d_err);
+                    h->launches += 2;
+                }
+            } else {
+                lw_column_kernel<R><<<(unsigned)ntot, LW_THREADS, smem, st>>>(bt, lut, h->d_err);
+                h->launches += 1;
+            }
+            RAD_CUDA(h, cudaGetLastError());
         }
     }
     if ((mrc = mark_if(1))) return mrc;
@@ -684,14 +686,14 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                                                      sc.k8, sc.kw);
         h->launches += 1;
     } else {
-    k_dayflags<<<gb, T, 0, st>>>(db, ntot, sc.flag);
-    size_t tb = sc.cub_bytes;
-    RAD_CUDA(h, cub::DeviceScan::ExclusiveSum(sc.cub, tb, sc.flag, sc.pos, (int)(ntot + 1), st));
-    k_scatter<<<gb, T, 0, st>>>(sc.flag, sc.pos, ntot, sc.daycol, sc.nday);
-    k_fill_int<<<(unsigned)((ncmin + T - 1) / T), T, 0, st>>>(sc.cmin, ncmin, std::numeric_limits<int>::max());
-    k_laytrop<<<gb, T, 0, st>>>(db, nlay, sc.daycol, sc.nday, sc.lt, sc.cmin, chunk, sc.pos);
-    k_groups<<<gb, T, 0, st>>>(db, sc.daycol, sc.nday, sc.lt, sc.cmin, chunk, sc.pos, sc.k8, sc.kw);
-    h->launches += 7;   // day flags, scan (2 kernels), scatter, fill, laytrop, groups
+        k_dayflags<<<gb, T, 0, st>>>(db, ntot, sc.flag);
+        size_t tb = sc.cub_bytes;
+        RAD_CUDA(h, cub::DeviceScan::ExclusiveSum(sc.cub, tb, sc.flag, sc.pos, (int)(ntot + 1), st));
+        k_scatter<<<gb, T, 0, st>>>(sc.flag, sc.pos, ntot, sc.daycol, sc.nday);
+        k_fill_int<<<(unsigned)((ncmin + T - 1) / T), T, 0, st>>>(sc.cmin, ncmin, std::numeric_limits<int>::max());
+        k_laytrop<<<gb, T, 0, st>>>(db, nlay, sc.daycol, sc.nday, sc.lt, sc.cmin, chunk, sc.pos);
+        k_groups<<<gb, T, 0, st>>>(db, sc.daycol, sc.nday, sc.lt, sc.cmin, chunk, sc.pos, sc.k8, sc.kw);
+        h->launches += 7;   // day flags, scan (2 kernels), scatter, fill, laytrop, groups
     }
     RAD_CUDA(h, cudaGetLastError());
     // ---- SW over the day columns; zeros first (night columns keep them, as swrad does)
@@ -721,7 +723,7 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
         }
         if ((mrc = mark_if(2))) return mrc;
         int64_t nlaunch = 1;
-        if (sizeof(R) == 4) {
+        if constexpr (sizeof(R) == 4) {
             const size_t smem = sw2_smem_bytes(any_aer);
             if (fixed) {   // no scratch: one CTA per sunlit column, R/T recomputed on the way down
                 sw2_column_kernel<false><<<(unsigned)ntot, SW2_THREADS, smem, st>>>(bt, any_aer ? 1 : 0, h->d_swf, h->d_swd,
@@ -752,11 +754,11 @@ int launch_batch(RadHandle* h, int nreq, const RadColumns* ins, const RadOutputs
                         sw4_exact_kernel<<<(unsigned)(SW4_EXACT_MINB * h->nsm), SW4_EXACT_THREADS, 0, st>>>(
                         bt, any_aer ? 1 : 0, h->d_swf, h->d_swd, (int)d0, h->d_sw4img, h->d_sw4, bb, lists);
                     if (diag_sw) {
-                        sw4_sweep_kernel<true><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
+                        sw4_sweep_kernel<true><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, (int)d0, (int)nc,
                                                                                         h->d_sw4, bb, h->d_swpg);
                         k_sw_diag<<<(unsigned)nc, SW4_DIAG_WARPS * 32, 0, st>>>(bt, (int)d0, h->d_sw4, bb, h->d_swpg, dout);
                     } else {
-                        sw4_sweep_kernel<false><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, h->d_err, (int)d0, (int)nc,
+                        sw4_sweep_kernel<false><<<(unsigned)nc, SW4_SWEEP_THREADS, smem2, st>>>(bt, (int)d0, (int)nc,
                                                                                          h->d_sw4, bb);
                     }
                 }

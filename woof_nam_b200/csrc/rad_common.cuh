@@ -212,6 +212,6 @@ struct ReqBatch {
 };
 
 // Error word written by kernels on bad input (host reads it after a synchronising call).
-enum : int { RAD_DEV_OK = 0, RAD_DEV_NLAY = 1, RAD_DEV_INDEX = 2, RAD_DEV_TIMEOUT = 3 };
+enum : int { RAD_DEV_OK = 0, RAD_DEV_NLAY = 1 };
 
 }  // namespace rad

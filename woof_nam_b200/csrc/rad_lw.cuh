@@ -1132,137 +1132,135 @@ __device__ __forceinline__ void lw_column_body(const LwBatch& bt, const LwLut<R>
     }
     lw_setup<R, NT>(s, a, col, tid);
     if (tid < LW_THREADS) {                          // the sweeps take the first LW_WARPS warps
-    const R eps = (R)1.0e-6f;
-    const bool rnd = a.rnd != 0;
-    // ---- phase C: rtrnmr (or rtrn) sweeps, one g-point per lane
-    const int warp = tid >> 5, lane = tid & 31;
-    const int g = tid;
-    const bool act = g < LW_NGPT;
-    int band = 0;
-    if (act)
-        while (g >= c_lw_ns[band + 1]) ++band;
-    const R bpade = (R)1.0f / (R)0.278f, tblint = (R)10000, rec_6 = (R)0.166667f, c06 = (R)0.06f;
-    R trngas[NLAY_MAX + 1], gassrcu[NLAY_MAX + 1], trntot[NLAY_MAX + 1], totsrcu[NLAY_MAX + 1], dn[NLAY_MAX + 1];
-    R radtotd = 0, radclrd = 0, totradd = 0, clrradd = 0, rad = 0;
-    if (act) {
-        const R sdif = s.secdiff[band];
-        for (int k = nlay; k >= 1; --k) {
-            R odepth = fmaxR((R)0, sdif * s.taug[g][k - 1]);
-            R atrgas, trng, gasfac;
-            if (odepth <= c06) {
-                atrgas = odepth - (R)0.5f * odepth * odepth;
-                trng = (R)1 - atrgas;
-                gasfac = rec_6 * odepth;
-            } else {
-                const R tblind = odepth / (bpade + odepth);
-                const int it = (int)(tblint * tblind + (R)0.5f);
-                trng = ldt(lut.ex + it); atrgas = (R)1 - trng; gasfac = ldt(lut.tfn + it); odepth = ldt(lut.tau + it);
-            }
-            const R plfrac = s.fracs[g][k - 1];
-            const R blay = s.pklay[k][band];
-            const R dplnku = s.pklev[k][band] - blay;
-            const R dplnkd = s.pklev[k - 1][band] - blay;
-            const R gassrcd = plfrac * (blay + dplnkd * gasfac) * atrgas;
-            gassrcu[k] = plfrac * (blay + dplnku * gasfac) * atrgas;
-            trngas[k] = trng;
-            const R clfr = s.cldfrc[k];
-            if (s.lstd[k] && !rnd) { totradd = clfr * radtotd; clrradd = radtotd - totradd; rad = 0; }
-            if (clfr >= eps) {
-                const R odcld = sdif * s.taucld[band][k - 1];
-                const R odtot = odepth + odcld;
-                R totfac, atrtot, trnt;
-                if (odtot < c06) {
-                    totfac = rec_6 * odtot; atrtot = odtot - (R)0.5f * odtot * odtot; trnt = (R)1 - atrtot;
-                } else {
-                    const R tblind = odtot / (bpade + odtot);
-                    const int it = (int)(tblint * tblind + (R)0.5f);
-                    totfac = ldt(lut.tfn + it); trnt = ldt(lut.ex + it); atrtot = (R)1 - trnt;
-                }
-                const R totsrcd = plfrac * (blay + dplnkd * totfac) * atrtot;
-                totsrcu[k] = plfrac * (blay + dplnku * totfac) * atrtot;
-                if (rnd) {
-                    // rtrn (phys_rrtm_lw_rtrn.cu:141-142, 232-233): the cloud fraction blends the cloudy and gas
-                    // sources; trntot holds the effective clear fraction for the upward sweep
-                    const R efclrfr = (R)1 - ((R)1 - rexp(-odcld)) * clfr;
-                    trntot[k] = efclrfr;
-                    radtotd = radtotd * trng * efclrfr + gassrcd + clfr * (totsrcd - gassrcd);
-                    radclrd = radclrd * trng + gassrcd;
-                    dn[k - 1] = radtotd;
-                    continue;
-                }
-                trntot[k] = trnt;
-                totradd = totradd * trnt + clfr * totsrcd;
-                clrradd = clrradd * trng + ((R)1 - clfr) * gassrcd;
-                radtotd = totradd + clrradd;
-                radclrd = radclrd * trng + gassrcd;
-                const R radmod = rad * (s.facclr1d[k - 1] * trng + s.faccld1d[k - 1] * trnt) -
-                                 s.faccmb1d[k - 1] * gassrcd + s.faccmb2d[k - 1] * totsrcd;
-                rad = -radmod + s.facclr2d[k - 1] * (clrradd + radmod) - s.faccld2d[k - 1] * (totradd - radmod);
-                totradd = totradd + rad;
-                clrradd = clrradd - rad;
-            } else {
-                radtotd = radtotd * trng + gassrcd;
-                radclrd = radclrd * trng + gassrcd;
-            }
-            dn[k - 1] = radtotd;
-        }
-    }
-    // surface: emission and reflection; clear-sky surface values
-    R radtotu = 0, radclru = 0, totradu = 0, clrradu = 0;
-    const R semi = act ? s.semiss[band] : (R)0;
-    if (act) {
-        const R reflct = (R)1 - semi;
-        const R rad0 = semi * s.fracs[g][0] * s.pklay[0][band];
-        radtotu = rad0 + reflct * radtotd;
-        radclru = rad0 + reflct * radclrd;
-    }
-    // scalar partials: sfc up/down total and clear
-    {
-        double v0 = act ? (double)radtotu : 0.0, v1 = act ? (double)radclru : 0.0;
-        double v2 = act ? (double)radtotd : 0.0, v3 = act ? (double)radclrd : 0.0;
-        v0 = warp_sum(v0); v1 = warp_sum(v1); v2 = warp_sum(v2); v3 = warp_sum(v3);
-        if (lane == 0) { s.scal[warp][2] = v0; s.scal[warp][3] = v1; s.scal[warp][4] = v2; s.scal[warp][5] = v3; }
-        double f0 = act ? (double)radtotu - (double)radtotd : 0.0;
-        f0 = warp_sum(f0);
-        if (lane == 0) s.fnet[warp][0] = f0;
-    }
-    for (int k = 1; k <= nlay; ++k) {
+        const R eps = (R)1.0e-6f;
+        const bool rnd = a.rnd != 0;
+        // ---- phase C: rtrnmr (or rtrn) sweeps, one g-point per lane
+        const int warp = tid >> 5, lane = tid & 31;
+        const int g = tid;
+        const bool act = g < LW_NGPT;
+        int band = 0;
+        if (act)
+            while (g >= c_lw_ns[band + 1]) ++band;
+        const R bpade = (R)1.0f / (R)0.278f, tblint = (R)10000, rec_6 = (R)0.166667f, c06 = (R)0.06f;
+        R trngas[NLAY_MAX + 1], gassrcu[NLAY_MAX + 1], trntot[NLAY_MAX + 1], totsrcu[NLAY_MAX + 1], dn[NLAY_MAX + 1];
+        R radtotd = 0, radclrd = 0, totradd = 0, clrradd = 0, rad = 0;
         if (act) {
-            const R clfr = s.cldfrc[k], trng = trngas[k], gasu = gassrcu[k];
-            if (s.lstu[k] && !rnd) { totradu = clfr * radtotu; clrradu = radtotu - totradu; rad = 0; }
-            if (rnd && clfr >= eps) {
-                radtotu = radtotu * trng * trntot[k] + gasu + clfr * (totsrcu[k] - gasu);
-                radclru = radclru * trng + gasu;
-            } else if (clfr >= eps) {
-                const R trnt = trntot[k], totu = totsrcu[k];
-                totradu = totradu * trnt + clfr * totu;
-                clrradu = clrradu * trng + ((R)1 - clfr) * gasu;
-                radtotu = totradu + clrradu;
-                radclru = radclru * trng + gasu;
-                const R radmod = rad * (s.facclr1u[k + 1] * trng + s.faccld1u[k + 1] * trnt) -
-                                 s.faccmb1u[k + 1] * gasu + s.faccmb2u[k + 1] * totu;
-                rad = -radmod + s.facclr2u[k + 1] * (clrradu + radmod) - s.faccld2u[k + 1] * (totradu - radmod);
-                totradu = totradu + rad;
-                clrradu = clrradu - rad;
-            } else {
-                radtotu = radtotu * trng + gasu;
-                radclru = radclru * trng + gasu;
+            const R sdif = s.secdiff[band];
+            for (int k = nlay; k >= 1; --k) {
+                R odepth = fmaxR((R)0, sdif * s.taug[g][k - 1]);
+                R atrgas, trng, gasfac;
+                if (odepth <= c06) {
+                    atrgas = odepth - (R)0.5f * odepth * odepth;
+                    trng = (R)1 - atrgas;
+                    gasfac = rec_6 * odepth;
+                } else {
+                    const R tblind = odepth / (bpade + odepth);
+                    const int it = (int)(tblint * tblind + (R)0.5f);
+                    trng = ldt(lut.ex + it); atrgas = (R)1 - trng; gasfac = ldt(lut.tfn + it); odepth = ldt(lut.tau + it);
+                }
+                const R plfrac = s.fracs[g][k - 1];
+                const R blay = s.pklay[k][band];
+                const R dplnku = s.pklev[k][band] - blay;
+                const R dplnkd = s.pklev[k - 1][band] - blay;
+                const R gassrcd = plfrac * (blay + dplnkd * gasfac) * atrgas;
+                gassrcu[k] = plfrac * (blay + dplnku * gasfac) * atrgas;
+                trngas[k] = trng;
+                const R clfr = s.cldfrc[k];
+                if (s.lstd[k] && !rnd) { totradd = clfr * radtotd; clrradd = radtotd - totradd; rad = 0; }
+                if (clfr >= eps) {
+                    const R odcld = sdif * s.taucld[band][k - 1];
+                    const R odtot = odepth + odcld;
+                    R totfac, atrtot, trnt;
+                    if (odtot < c06) {
+                        totfac = rec_6 * odtot; atrtot = odtot - (R)0.5f * odtot * odtot; trnt = (R)1 - atrtot;
+                    } else {
+                        const R tblind = odtot / (bpade + odtot);
+                        const int it = (int)(tblint * tblind + (R)0.5f);
+                        totfac = ldt(lut.tfn + it); trnt = ldt(lut.ex + it); atrtot = (R)1 - trnt;
+                    }
+                    const R totsrcd = plfrac * (blay + dplnkd * totfac) * atrtot;
+                    totsrcu[k] = plfrac * (blay + dplnku * totfac) * atrtot;
+                    if (rnd) {
+                        // rtrn (phys_rrtm_lw_rtrn.cu:141-142, 232-233): the cloud fraction blends the cloudy and gas
+                        // sources; trntot holds the effective clear fraction for the upward sweep
+                        const R efclrfr = (R)1 - ((R)1 - rexp(-odcld)) * clfr;
+                        trntot[k] = efclrfr;
+                        radtotd = radtotd * trng * efclrfr + gassrcd + clfr * (totsrcd - gassrcd);
+                        radclrd = radclrd * trng + gassrcd;
+                        dn[k - 1] = radtotd;
+                        continue;
+                    }
+                    trntot[k] = trnt;
+                    totradd = totradd * trnt + clfr * totsrcd;
+                    clrradd = clrradd * trng + ((R)1 - clfr) * gassrcd;
+                    radtotd = totradd + clrradd;
+                    radclrd = radclrd * trng + gassrcd;
+                    const R radmod = rad * (s.facclr1d[k - 1] * trng + s.faccld1d[k - 1] * trnt) -
+                                     s.faccmb1d[k - 1] * gassrcd + s.faccmb2d[k - 1] * totsrcd;
+                    rad = -radmod + s.facclr2d[k - 1] * (clrradd + radmod) - s.faccld2d[k - 1] * (totradd - radmod);
+                    totradd = totradd + rad;
+                    clrradd = clrradd - rad;
+                } else {
+                    radtotd = radtotd * trng + gassrcd;
+                    radclrd = radclrd * trng + gassrcd;
+                }
+                dn[k - 1] = radtotd;
             }
         }
-        double f = act ? (double)radtotu - (double)(k < nlay ? dn[k] : (R)0) : 0.0;
-        f = warp_sum(f);
-        if (lane == 0) s.fnet[warp][k] = f;
-    }
-    {
-        double v0 = act ? (double)radtotu : 0.0, v1 = act ? (double)radclru : 0.0;
-        v0 = warp_sum(v0); v1 = warp_sum(v1);
-        if (lane == 0) { s.scal[warp][0] = v0; s.scal[warp][1] = v1; }
-    }
+        // surface: emission and reflection; clear-sky surface values
+        R radtotu = 0, radclru = 0, totradu = 0, clrradu = 0;
+        const R semi = act ? s.semiss[band] : (R)0;
+        if (act) {
+            const R reflct = (R)1 - semi;
+            const R rad0 = semi * s.fracs[g][0] * s.pklay[0][band];
+            radtotu = rad0 + reflct * radtotd;
+            radclru = rad0 + reflct * radclrd;
+        }
+        // scalar partials: sfc up/down total and clear
+        {
+            double v0 = act ? (double)radtotu : 0.0, v1 = act ? (double)radclru : 0.0;
+            double v2 = act ? (double)radtotd : 0.0, v3 = act ? (double)radclrd : 0.0;
+            v0 = warp_sum(v0); v1 = warp_sum(v1); v2 = warp_sum(v2); v3 = warp_sum(v3);
+            if (lane == 0) { s.scal[warp][2] = v0; s.scal[warp][3] = v1; s.scal[warp][4] = v2; s.scal[warp][5] = v3; }
+            double f0 = act ? (double)radtotu - (double)radtotd : 0.0;
+            f0 = warp_sum(f0);
+            if (lane == 0) s.fnet[warp][0] = f0;
+        }
+        for (int k = 1; k <= nlay; ++k) {
+            if (act) {
+                const R clfr = s.cldfrc[k], trng = trngas[k], gasu = gassrcu[k];
+                if (s.lstu[k] && !rnd) { totradu = clfr * radtotu; clrradu = radtotu - totradu; rad = 0; }
+                if (rnd && clfr >= eps) {
+                    radtotu = radtotu * trng * trntot[k] + gasu + clfr * (totsrcu[k] - gasu);
+                    radclru = radclru * trng + gasu;
+                } else if (clfr >= eps) {
+                    const R trnt = trntot[k], totu = totsrcu[k];
+                    totradu = totradu * trnt + clfr * totu;
+                    clrradu = clrradu * trng + ((R)1 - clfr) * gasu;
+                    radtotu = totradu + clrradu;
+                    radclru = radclru * trng + gasu;
+                    const R radmod = rad * (s.facclr1u[k + 1] * trng + s.faccld1u[k + 1] * trnt) -
+                                     s.faccmb1u[k + 1] * gasu + s.faccmb2u[k + 1] * totu;
+                    rad = -radmod + s.facclr2u[k + 1] * (clrradu + radmod) - s.faccld2u[k + 1] * (totradu - radmod);
+                    totradu = totradu + rad;
+                    clrradu = clrradu - rad;
+                } else {
+                    radtotu = radtotu * trng + gasu;
+                    radclru = radclru * trng + gasu;
+                }
+            }
+            double f = act ? (double)radtotu - (double)(k < nlay ? dn[k] : (R)0) : 0.0;
+            f = warp_sum(f);
+            if (lane == 0) s.fnet[warp][k] = f;
+        }
+        {
+            double v0 = act ? (double)radtotu : 0.0, v1 = act ? (double)radclru : 0.0;
+            v0 = warp_sum(v0); v1 = warp_sum(v1);
+            if (lane == 0) { s.scal[warp][0] = v0; s.scal[warp][1] = v1; }
+        }
     }
     __syncthreads();
     // ---- outputs: fluxes x flxfac, heating rates from float64 net-flux differences
-    const double fluxfac = sizeof(R) == 4 ? (double)(float)(2.0 * 3.14159265358979323846 / 2.0 * 2.0) * 0.0 : 0.0;
-    (void)fluxfac;
     const double pi = 3.14159265358979323846;
     const double flxfac = 0.5 * (sizeof(R) == 4 ? (double)(float)((double)(float)pi * 2.0e4) : pi * 2.0e4);
     const double heatfac = sizeof(R) == 4 ? (double)(9.80665f * 1.0e-2f / 1.0046e3f) : 9.80665 * 1.0e-2 / 1.0046e3;

@@ -25,8 +25,6 @@ constexpr int LW_OVR_RANDOM = 2;   // rtrn: NAM route, iovrlw = 0
 template <class R>
 struct LwTerms {
     R trng, gassrcd, gassrcu, trnt, totsrcd, totsrcu;
-    R atrg;        // gas absorptance 1 - trng as computed (directly from the depth for thin layers)
-    R atrt;        // cloudy: total absorptance 1 - trnt, likewise
 };
 
 // A depth that has the last entry of the tables; above it the product with the diffusivity may be infinite, whose
@@ -56,8 +54,7 @@ __device__ __forceinline__ LwTerms<R> lw2_terms(const LwShared<R>& s, const LwLu
     const R dplnkd = s.pklev[k - 1][band] - blay;
     t.gassrcd = plfrac * (blay + dplnkd * gasfac) * atrgas;
     t.gassrcu = plfrac * (blay + dplnku * gasfac) * atrgas;
-    t.atrg = atrgas;
-    t.trnt = 1; t.totsrcd = 0; t.totsrcu = 0; t.atrt = 0;
+    t.trnt = 1; t.totsrcd = 0; t.totsrcu = 0;
     if (cloudy) {
         const R odtot = fminR((R)LW_OD_MAX, odepth + sdif * s.taucld[band][k - 1]);
         R totfac, atrtot;
@@ -70,7 +67,6 @@ __device__ __forceinline__ LwTerms<R> lw2_terms(const LwShared<R>& s, const LwLu
         }
         t.totsrcd = plfrac * (blay + dplnkd * totfac) * atrtot;
         t.totsrcu = plfrac * (blay + dplnku * totfac) * atrtot;
-        t.atrt = atrtot;
     }
     return t;
 }

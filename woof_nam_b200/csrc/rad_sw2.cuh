@@ -42,10 +42,7 @@
 namespace rad {
 
 constexpr int SW2_WARPS = 4, SW2_THREADS = 128;
-#ifndef RAD_SW2_SEG
-#define RAD_SW2_SEG 4
-#endif
-constexpr int SW2_SEG = RAD_SW2_SEG;                              // layers per checkpoint segment
+constexpr int SW2_SEG = 4;                                        // layers per checkpoint segment
 constexpr int SW2_NSEG = (NLAY_MAX + SW2_SEG - 1) / SW2_SEG;
 constexpr float SW2_RESONANCE = 1.0e-2f;                          // float64 R/T where |1-(k mu0)^2| < this
 constexpr double SW2_TBL_MARGIN = 0.01;                           // table-index rounding margin (see sw2_tbl_sure)

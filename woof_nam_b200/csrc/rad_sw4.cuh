@@ -445,8 +445,8 @@ sw4_rt_kernel(const __grid_constant__ SwBatch bt, int any_aer, int d0, const int
                 if (q1) enqueue(k0, g + 1, q1);
             }
         };
-        if (!clr5) clear(std::true_type{});
-        else clear(std::false_type{});
+        if (MODE == 1 || !clr5) clear(std::true_type{});
+        else if constexpr (MODE != 1) clear(std::false_type{});
         __syncthreads();
         // cloudy pass: the layers with a slot, mixture R/T blended with the clear R/T (or, McICA, taken
         // unblended where the g-point's sub-column bit is set)
@@ -663,7 +663,7 @@ __device__ __forceinline__ double warp_sum4(const double* v, int lane)
 // summed together.
 template <bool DIAG = false>
 __global__ void __launch_bounds__(SW4_SWEEP_THREADS, SW4_SWEEP_MINB)
-sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int* err, int d0, int nc, const unsigned char* scr,
+sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int d0, int nc, const unsigned char* scr,
                  size_t blk_bytes, float* __restrict__ pg = nullptr)
 {
     extern __shared__ __align__(16) float2 ckpt[];                 // [(nseg - 1) x 2][SW4_SWEEP_THREADS]
@@ -849,7 +849,6 @@ sw4_sweep_kernel(const __grid_constant__ SwBatch bt, int* err, int d0, int nc, c
             a.fdncmp[5 * N + col] = (float)tot(c[7], t[7]);
         }
     }
-    (void)err;
 }
 
 // swrad's optional outputs of a chunk from the DIAG sweeps' profiles (swrad_post's lhsw0 / lhswb / lflxprf blocks): one
