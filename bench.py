@@ -551,10 +551,11 @@ def main():
     lw_ms, sw_ms = prof["lw_ms"] / max(prof["solves"], 1), prof["sw_ms"] / max(prof["solves"], 1)
     lw_tf = ops["lw_flops_per_col"] * n / (lw_ms * 1e-3) / 1e12
     sw_tf = ops["sw_flops_per_daycol"] * nday / (sw_ms * 1e-3) / 1e12
-    # the mixed precision runs the two-kernel LW (gas optics, then sweeps, per chunk) and the two-kernel SW
+    # the mixed precision runs the two-kernel LW (gas optics, then sweeps, per chunk) and the chunked SW
     # (set-up, optics and layer R/T into the chunk scratch, then the adding sweeps, per chunk of day columns)
     lw_name = "lw3_optics_kernel+lw3_sweep_kernel"
-    sw_name = "sw2_column_kernel" if mcfg.sw_sweep_chunk < 0 else "sw4_optics_kernel+sw4_sweep_kernel"
+    sw_name = "sw2_column_kernel" if mcfg.sw_sweep_chunk < 0 else \
+        "sw4_gas_kernel+sw4_rt_kernel+sw4_fix_kernel+sw4_exact_kernel+sw4_sweep_kernel"
     dom = sw_name if sw_ms >= lw_ms else lw_name
     achieved = sw_tf if dom == sw_name else lw_tf
     traffic = None

@@ -69,7 +69,7 @@ typedef struct {
                                 ~88 KB per column of scratch, then the sweeps); 0 = 32768; negative = the
                                 single-kernel LW (gas optics in shared memory, no scratch) */
     int32_t sw_sweep_chunk;  /* mixed precision: day columns per chunk of the two-kernel SW (set-up, optics and
-                                the layer reflectances / transmittances through ~345 KB per column of scratch, then
+                                the layer reflectances / transmittances through ~407 KB per column of scratch, then
                                 the adding sweeps); 0 = 16384; negative = the single-kernel SW (no scratch besides
                                 the R/T stores) */
 } RadConfig;

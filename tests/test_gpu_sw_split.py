@@ -1,5 +1,5 @@
-"""The two-kernel SW (sw4_optics_kernel + sw4_sweep_kernel: set-up, optics and the layer R/T of a chunk of day
-columns into the chunk scratch, then the adding sweeps from it) against the single-kernel SW (sw_sweep_chunk
+"""The chunked SW (the sw4_* kernels: set-up, optics and the layer R/T of a chunk of day columns
+into the chunk scratch, then the adding sweeps from it) against the single-kernel SW (sw_sweep_chunk
 < 0) through the C-ABI, with chunks smaller than the day count (several chunks, a ragged last one, chunks past
 the day count that exit at once), with aerosol optics, on the McICA route, and against the float64 oracle
 within the mixed-precision tolerances (0.05 W/m^2, 0.01 K/day).  Both forms run the same statements and make

@@ -1,7 +1,8 @@
 // rad_f32x2.cuh -- two floats side by side in one 64-bit register pair: the packed single-precision operations of
 // sm_100 (add / sub / mul / fma .f32x2).  Each acts on both halves with the rounding of its scalar form, so a pair
-// of independent g-points costs one issue slot per operation instead of two; the column kernels issue on 55-62 % of
-// their cycles with the FMA pipe at 18-28 %, so issue slots, not FMA lanes, are what they run out of.
+// of independent g-points costs one issue slot per operation instead of two: with one g-point per lane the column kernels
+// issued on 55-62 % of their cycles with the FMA pipe at 18-28 %, so issue slots, not FMA lanes, were what they ran out of
+// (in pairs: 52-68 % and 14-31 % at half the time or less in the R/T and the LW sweeps).
 #pragma once
 #include <cuda_runtime.h>
 

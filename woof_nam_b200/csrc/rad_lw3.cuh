@@ -58,7 +58,7 @@ __host__ __device__ constexpr int64_t lw3_block_floats(int nlay) { return (LW3_H
 
 // Optics CTA: 8 warps, 3 CTAs per SM (24 warps, 80 registers a thread, no spills).  The CTAs per SM set how many
 // columns share an SM's L1 for the table gathers, and more than 3 cost more than they gain; more warps per CTA share a
-// column's tasks and hide the gathers' latency, until the registers run out.  Bound: the L1 data pipe (67 % of its peak
+// column's tasks and hide the gathers' latency, until the registers run out.  Bound: the L1 data pipe (68 % of its peak
 // wavefronts: every task's gathers touch a line per layer of the warp) and phase A's barriers.  Measured per 131,072
 // columns of 61 layers: one g-point per task 17.4 ms; pairs 13.2 (288 x 3: 13.3, 224 x 4: 14.9, 320 x 3: 14.4, 384 x 2
 // 14.1, 448 x 2: 14.1); phase A and the records spread out 12.6; packed layer words 12.35 (288 x 3: 12.5, 192 x 4: 13.5);

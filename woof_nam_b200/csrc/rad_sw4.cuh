@@ -1,11 +1,12 @@
 // rad_sw4.cuh -- the chunked SW of rad_solve (mixed precision): set-up and gas optics, the layer reflectances
-// and transmittances, their float64 fix-ups, and the adding sweeps in four kernels per chunk of sunlit columns.
+// and transmittances, their float64 fix-ups and recomputes, and the adding sweeps in five kernels per chunk of sunlit
+// columns.
 //
 // Same statements as sw2_column (rad_sw2.cuh), split where the work changes shape, and each kernel small enough
 // that the CTAs resident on an SM run out of the instruction cache (one kernel with all three phases spent most
 // of its stalls waiting for instructions):
 //  * sw4_gas_kernel, one CTA (128 threads) per sunlit column, six per SM: set-up and cloud optics
-//    (sw2_setup), gas and Rayleigh optical depths per (g-point, layer); writes the column image (the part of the
+//    (sw2_setup), gas and Rayleigh optical depths per (g-point pair, layer); writes the column image (the part of the
 //    shared-memory layout the later phases read, taug included).
 //  * sw4_rt_kernel, one CTA per column: loads the image, then the layer R/T of the clear pass and, in the
 //    layers with cloud, of the cloudy pass (spcvrtc.cu:112-173, 330-460) in float without branches, a task a pair
@@ -13,14 +14,17 @@
 //    tasks so that a warp shares the cloudy branch.  A g-point whose R/T needs a float64 step (the resonance, or an
 //    exp-table argument near an entry bound whose neighbouring entry matters) is queued.  Output per column: a
 //    header (solar source per g-point, albedos, overlap fractions, heating factors, the cloudy-pass slot of each
-//    layer), the R/T as [layer][field][g-point] (a warp of the sweep kernel reads 32 consecutive g-points of one
-//    field and layer: one 128-byte line) and the queue.
-//  * sw4_fix_kernel, over the tile's queues: sw2_layer (the sweep kernels' own function) for the queued g-points.
-//    Bound: issue slots.  Measured per 131,072 columns (65,536 sunlit, 61 layers): 12.76 ms as one kernel with one
-//    g-point per thread and the queue formed by the same CTA; 9.48 ms with pairs; 4.30 + 3.35 ms as two kernels --
-//    the queue's float64 code no longer sets the registers (128, 4 CTAs per SM; now 80, 6 CTAs) nor keeps a CTA's
-//    other warps waiting, and the columns at a resonance (thousands of entries; up to 2,000,000 cycles in one CTA
-//    when a fixed queue of 527 overflowed) spread over the grid.
+//    layer), the R/T as [layer][field][g-point] (a warp of the sweep kernel reads 28 consecutive pairs of g-points of
+//    one field and layer, 224 contiguous bytes: half a row) and the queue.
+//  * sw4_fix_kernel, over the tile's queues: sw2_layer (the single-kernel SW's own function) for the queued g-points,
+//    cut into items.  Taking the queue out of the R/T kernel left that 80 registers and 6 CTAs per SM instead of 128 and
+//    4, no CTA waits for its slowest float64 lane any more, and the columns at a resonance (thousands of entries; up to
+//    2,000,000 cycles in one CTA when a fixed queue of 527 overflowed) spread over the grid.
+//  * sw4_exact_kernel (tiles of SW4_EXACT_MIN columns or more), over per-band lists: the g-points whose R/T are
+//    recomputed in float64 from the column's inputs.
+//    Measured per 131,072 columns (65,536 sunlit, 61 layers): 12.76 ms for the R/T as one kernel with one g-point per
+//    thread and the queue formed by the same CTA; 9.48 with pairs; 4.30 + 3.35 as R/T and fix-up; 4.30 + 1.70 + 0.23 with
+//    the recomputes apart.
 //  * sw4_sweep_kernel, one CTA per column: the adding method alone (swflux, spcvrtc.cu:178-215) -- the upward
 //    sweep with segment checkpoints, the downward sweep re-reading each segment's R/T, float64 level sums and
 //    the swrad epilogue.
@@ -34,7 +38,7 @@ namespace rad {
 
 constexpr int SW4_FIELDS = 6;                       // rb, rd, tb, td, e3 (delta-scaled beam), e4 (unscaled beam)
 constexpr int SW4_LAYER = SW4_FIELDS * SW_NGPT;     // floats per layer and pass, [field][g]
-// CTA shapes of the three kernels, swept on the B200 (same bits): the gas-optics kernel at 128 threads x 6 CTAs
+// CTA shapes of the kernels, swept on the B200 (same bits): the gas-optics kernel at 128 threads x 6 CTAs
 // per SM against 160 x 5, 192 x 4, 256 x 3, 320 x 2, 384 x 2 (SW +0.2 to +9.8 %).
 constexpr int SW4_RT_THREADS = 128;                 // threads of an R/T CTA
 constexpr int SW4_OPT_MINB = 6;                     // CTAs per SM the R/T kernel is compiled for (4: 4.62, 5: 4.41, 6: 4.30 ms)
@@ -657,7 +661,7 @@ __device__ __forceinline__ double warp_sum4(const double* v, int lane)
 // The adding method of one sunlit column from its block (sw2_column phase C with the R/T read instead of formed).  Four
 // warps per column: warps 0 and 1 run the clear pass, warps 2 and 3 the cloudy one (idle in a cloudless column), a lane
 // per pair of g-points (28 lanes each), so a pass's chain of layers is not lengthened by the other's.  Bound: the latency
-// of a segment's rows and of the recurrence (2.8 TB/s of R/T rows read).  Measured per 131,072 columns (65,536 sunlit):
+// of a segment's rows and of the recurrence (3.6 TB/s of R/T rows read, 44 % of the DRAM peak).  Measured per 131,072 columns (65,536 sunlit):
 // 6.47 ms with both passes and one g-point per lane at 80 registers; the same with pairs and both passes in two warps
 // (168 registers, 6 CTAs per SM: latency); 5.06 ms with the passes in warps of their own and the four levels of a segment
 // summed together.

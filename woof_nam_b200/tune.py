@@ -4,7 +4,7 @@ fastest per (device, layers, route, column-count bucket).
 * lw_chunk: the column tile of the LW gas-optics / sweep kernel pair -- how many columns share one scratch
   pass (88 KB per column) before the sweeps read it back.
 * sw_sweep_chunk: the tile of sunlit columns of the SW's kernels (gas optics into the image, layer R/T into the
-  blocks, float64 fix-ups, adding sweeps; ~345 KB per column).
+  blocks, float64 fix-ups, adding sweeps; ~407 KB per column: blocks, images and lists).
 
 Small tiles keep more of the scratch in L2 but launch more often and leave the GPU idle at each tile's tail;
 large tiles do the opposite and hold more HBM.  Every candidate gives the same bits (each column's arithmetic
